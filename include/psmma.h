@@ -60,7 +60,9 @@ extern "C" {
 #define PSMMA_ESCRATCH      -117  /* request exceeds the fixed scratch of psmma_cauchy_split_noalloc */
 
 /* ---- options ------------------------------------------------------------------------ */
-#define PSMMA_PREC_FP64   0   /* plain path: FP64 tensor-core MMA, H tile generated in smem  */
+#define PSMMA_PREC_FP64   0   /* FP64 results: real kinds by the exact modular product rounded once
+                                 (or FP64 tensor-core MMA where the operands span too many
+                                 bits, the caller brings a workspace, or the call is captured)  */
 #define PSMMA_PREC_SPLIT  1   /* split path: exact modular slices on BF16 tensor cores (tcgen05),
                                  FP64 scaling and recombination (all four kinds)              */
 
@@ -438,7 +440,10 @@ int psmma_server_destroy(psmma_server* s);
 /* Bytes of device workspace a call with these sizes and options needs.  The FP64 path needs
  * none, except for products with too few 128 x 128 output tiles to fill the SMs, which it
  * splits along K into partial sums when workspace is available (0 otherwise).  Pass a buffer
- * at least this large in opts->work to avoid library allocation. */
+ * at least this large in opts->work to avoid library allocation.  An FP64 call with opts->work
+ * runs the FP64 tensor-core kernel; one without it takes the exact modular product, whose
+ * planes (up to 40 GiB: n = k = 4096 2.9 GB) come from the stream's pool, or the kernel where
+ * that allocation fails. */
 size_t psmma_workspace_size(int kind, int n, int k, const psmma_opts* opts);
 
 /* Frees the library-owned workspace pools of the current device. */

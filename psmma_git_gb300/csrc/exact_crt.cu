@@ -1,0 +1,636 @@
+// The FP64 precision's fast route: the structured product Q = alpha*A*H + beta*Q with A*H formed
+// EXACTLY on the BF16 tensor cores and rounded once.
+//
+// GB300 issues about two FP64 multiply-adds per SM per cycle, on the scalar and on the tensor
+// form alike (0.6e12 a second), so a product of 2 n^3 FP64 flops is bound by that pipe.  The
+// modular GEMM of split_crt.cu runs BF16 at 1700 times that rate, and unlike the split precision,
+// which rounds A and H to the bits its moduli cover, this route takes as many moduli as the
+// operands need:
+//   1. a_max, the lowest set bit and the 2-norm of every row of A; the same of every column of H,
+//      generated in FP64 by the entry formulas of the DMMA kernel (fp64_structured.cu).
+//   2. Row i times 2^-lsb_i and column j times 2^-lsb_j are integers without any rounding.  A bound
+//      of |Z_ij| = |(A'H')_ij| from the norms gives the number of moduli whose product exceeds
+//      2 |Z| (8 to 32 in steps of 4, up to 241 bits), on the device.
+//   3. One BF16 GEMM per modulus, the Chinese remainder theorem in 28-bit limbs, and one rounding
+//      of Z 2^(lsb_i + lsb_j) to FP64; then alpha and beta.
+// The rounded sum of exact products is at least as accurate as any order of FP64 additions.  Where
+// a row or column spans more than 112 bits, the bound exceeds the moduli, an entry is not finite or
+// a device wait gave up, the flag `nmod` is 0 and the DMMA kernel, enqueued behind this route and
+// gated on that flag, computes the product as it would alone.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <cmath>
+
+#include "psmma_internal.h"
+#include "split_passes.cuh"
+#include "tcgen05_util.cuh"
+
+namespace psmma {
+
+int launch_modular_gemm(__nv_bfloat16* RA, __nv_bfloat16* RH, int8_t* R, int M, int N, int kp, int kr, int planes,
+                        const int* moduli, const int* nmod_dev, unsigned* status, int sms, cudaStream_t stream);
+
+namespace {
+
+// ------------------------------------------------------------------------------------------
+// Moduli and CRT constants (compile time)
+// ------------------------------------------------------------------------------------------
+// Pairwise coprime, at most 256: 2^8, 3*5*17, 11*23, 13*19, 7*31 and primes.
+constexpr int EX_MAX = 32, EX_GROUPS = EX_MAX / 4, EX_LIMBS = 9, EX_CHUNKS = 8;
+constexpr int kExModuli[EX_MAX] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193, 191,
+                                   217, 181, 179, 173, 167, 163, 157, 151, 149, 139, 137, 131, 127, 113, 109, 107};
+
+// The CRT for the first 4 G moduli.  The four moduli of a group g (product P_g < 2^32) are first
+// combined in 32-bit arithmetic: with u_i = residue + 128 in [0, 255],
+//   X_g = b_g + sum_i u_i c_i (mod P_g),  X_g = Z W_g^-1 mod P_g,  W_g = M / P_g,
+// and Z = sum_g X_g W_g - q M with q the nearest integer to sum_g X_g / P_g.
+struct ExCrt {
+  unsigned c[EX_MAX], f[EX_MAX];      // c_i, floor(2^20 c_i / P_g)
+  unsigned b[EX_GROUPS], fb[EX_GROUPS], P[EX_GROUPS], G[EX_GROUPS];  // ..., P_g, floor(2^52 / P_g)
+  unsigned W[EX_GROUPS][EX_LIMBS];    // W_g in 28-bit limbs
+  unsigned M[EX_LIMBS];
+};
+struct ExTables {
+  ExCrt crt[EX_GROUPS + 1];           // by group count (2..8)
+  float g[EX_MAX][EX_CHUNKS];         // 2^(14 t) mod m, symmetric; [0] = 1 / m
+  float m[EX_MAX];
+};
+
+constexpr unsigned long long ex_inv(unsigned long long a, unsigned long long m) {
+  for (unsigned long long x = 1; x < m; ++x)
+    if (a * x % m == 1) return x;
+  return 0;
+}
+
+constexpr ExTables make_tables() {
+  ExTables T{};
+  for (int l = 0; l < EX_MAX; ++l) {
+    const int m = kExModuli[l];
+    T.m[l] = (float)m;
+    long long p = 1;
+    for (int t = 0; t < EX_CHUNKS; ++t) {
+      const long long s = p > m / 2 ? p - m : p;
+      T.g[l][t] = t == 0 ? 1.0f / (float)m : (float)s;
+      p = p * (1 << 14) % m;
+    }
+  }
+  for (int G = 2; G <= EX_GROUPS; ++G) {
+    ExCrt& C = T.crt[G];
+    for (int g = 0; g < G; ++g) {
+      unsigned long long P = 1;
+      for (int i = 0; i < 4; ++i) P *= (unsigned long long)kExModuli[4 * g + i];
+      C.P[g] = (unsigned)P;
+      C.G[g] = (unsigned)((1ull << 52) / P);
+      C.W[g][0] = 1;
+      for (int l = 0; l < 4 * G; ++l) {
+        if (l / 4 == g) continue;
+        unsigned long long carry = 0;
+        for (int t = 0; t < EX_LIMBS; ++t) {
+          const unsigned long long v = (unsigned long long)C.W[g][t] * kExModuli[l] + carry;
+          C.W[g][t] = (unsigned)(v & 0xFFFFFFFull);
+          carry = v >> 28;
+        }
+      }
+      unsigned long long bias = 0;
+      for (int i = 0; i < 4; ++i) {
+        const unsigned long long m = kExModuli[4 * g + i], Q = P / m;
+        unsigned long long w = 0;  // W_g mod m
+        for (int t = EX_LIMBS - 1; t >= 0; --t) w = (w * (1ull << 28) + C.W[g][t]) % m;
+        const unsigned long long y = ex_inv(w, m) * ex_inv(Q % m, m) % m;
+        C.c[4 * g + i] = (unsigned)(Q * y);
+        C.f[4 * g + i] = (unsigned)((Q * y << 20) / P);
+        bias = (bias + 128 * (Q * y)) % P;
+      }
+      const unsigned long long b = bias ? P - bias : 0;
+      C.b[g] = (unsigned)b;
+      C.fb[g] = (unsigned)((b << 20) / P);
+    }
+    C.M[0] = 1;
+    for (int l = 0; l < 4 * G; ++l) {
+      unsigned long long carry = 0;
+      for (int t = 0; t < EX_LIMBS; ++t) {
+        const unsigned long long v = (unsigned long long)C.M[t] * kExModuli[l] + carry;
+        C.M[t] = (unsigned)(v & 0xFFFFFFFull);
+        carry = v >> 28;
+      }
+    }
+  }
+  return T;
+}
+
+__constant__ ExTables kEx = make_tables();
+
+struct ExLog2 {
+  float v[EX_GROUPS + 1];  // log2 of the product of the first 4 G moduli, rounded down
+};
+
+// ------------------------------------------------------------------------------------------
+// Device parameters and workspace
+// ------------------------------------------------------------------------------------------
+struct ExParams {
+  unsigned status;
+  int nmod;      // moduli of this call; 0: the DMMA route
+  int ncA, ncH;  // 14-bit chunks of A' and H'
+  unsigned run_dmma;
+};
+
+size_t al1k(size_t x) { return (x + 1023) & ~(size_t)1023; }
+
+struct ExLayout {
+  int kp, kr;
+  size_t off_amax, off_asq, off_alsb, off_hmax, off_hsum, off_hsq, off_hlsb, off_ht, off_ra, off_rh, off_r, total;
+};
+
+ExLayout ex_layout(int M, int N, int K, int planes) {
+  ExLayout L;
+  L.kp = (K + 63) / 64 * 64;
+  L.kr = (N + 255) / 256 * 256;
+  size_t o = 1024;
+  L.off_amax = o; o += al1k((size_t)M * 8);
+  L.off_asq = o;  o += al1k((size_t)M * 8);
+  L.off_alsb = o; o += al1k((size_t)M * 4);
+  L.off_hmax = o; o += al1k((size_t)N * 8);
+  L.off_hsum = o; o += al1k((size_t)N * 8);
+  L.off_hsq = o;  o += al1k((size_t)N * 8);
+  L.off_hlsb = o; o += al1k((size_t)N * 4);
+  L.off_ht = o;   o += al1k((size_t)N * L.kp * 8);
+  L.off_ra = o;   o += al1k((size_t)planes * M * L.kp * 2);
+  L.off_rh = o;   o += al1k((size_t)planes * N * L.kp * 2);
+  L.off_r = o;    o += al1k((size_t)planes * M * L.kr);
+  L.total = o;
+  return L;
+}
+
+// ------------------------------------------------------------------------------------------
+// Passes
+// ------------------------------------------------------------------------------------------
+__global__ void k_ex_init(ExParams* prm, unsigned long long* amax, double* asq, int* alsb, int M) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *prm = ExParams{0u, 0, 0, 0, 1u};
+  if (i < M) {
+    amax[i] = 0ull;
+    asq[i] = 0.0;
+    alsb[i] = NO_LSB;
+  }
+}
+
+__global__ void k_ex_row_stats(const double* __restrict__ A, long lda, int n, int k, int kchunk,
+                               unsigned long long* __restrict__ amax, double* __restrict__ asq,
+                               int* __restrict__ alsb) {
+  row_absmax_blk<true>(A, lda, nullptr, 0, k, n, k, kchunk, amax, asq, blockIdx.x, blockIdx.y, alsb);
+}
+
+template <int KIND>
+__global__ void k_ex_h(GenSpec gs, int K, int kp, double* __restrict__ Ht, unsigned long long* __restrict__ hmax,
+                       double* __restrict__ hsum, double* __restrict__ hsq, int* __restrict__ hlsb) {
+  h_pass1_blk<KIND, true>(gs, K, kp, Ht, hmax, hsum, hsq, nullptr, blockIdx.x, nullptr, hlsb);
+}
+
+// An upper bound of log2 of the mantissa (in [1, 2)) of the normal double with bits b.
+__device__ __forceinline__ float log2_mant_up(unsigned long long b) {
+  const float f = __uint_as_float(0x3F800000u | ((unsigned)(b >> 29) & 0x7FFFFFu));
+  return log2f(f) + 1e-5f;
+}
+
+// Number of moduli and chunk counts from the statistics.  With a'_i = row i of A' = A 2^-alsb_i and
+// h'_j likewise, |Z_ij| <= max|a'| max sum|h'| and <= max ||a'||_2 max ||h'||_2; the CRT needs
+// |Z| < 0.497 M.  Norms whose squares leave the range of FP64 count max * sqrt(k).
+__global__ void __launch_bounds__(1024) k_ex_params(ExParams* prm, ExLog2 lg, int max_groups, int M, int N, int K,
+                                                    const unsigned long long* __restrict__ amax,
+                                                    const double* __restrict__ asq, const int* __restrict__ alsb,
+                                                    const unsigned long long* __restrict__ hmax,
+                                                    const double* __restrict__ hsum, const double* __restrict__ hsq,
+                                                    const int* __restrict__ hlsb) {
+  float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // bits A, log2 max A, log2 ||A||, bits H, log2 sum H, log2 ||H||
+  int bad = 0;
+  const float lk = log2f((float)K) + 1e-3f;
+  for (int r = threadIdx.x; r < M + N; r += blockDim.x) {
+    const bool h = r >= M;
+    const int i = h ? r - M : r;
+    const unsigned long long b = h ? hmax[i] : amax[i];
+    if (b == 0) continue;
+    if (b >= INF_BITS) { bad = 1; continue; }
+    const int lsb = h ? hlsb[i] : alsb[i], top = ilogb_bits(b);
+    const float bits = (float)(top + 1 - lsb);
+    const bool safe = top > -450 && top < 450;
+    const unsigned long long q = (unsigned long long)__double_as_longlong(h ? hsq[i] : asq[i]);
+    const int eq = (int)(q >> 52) - 1023;
+    const float two = safe && q < INF_BITS && eq > -1000 && q != 0
+                          ? 0.5f * ((float)(eq - 2 * lsb) + log2_mant_up(q)) + 0.01f
+                          : bits + 0.5f * lk;
+    float one = bits;
+    if (h) {
+      const unsigned long long sb = (unsigned long long)__double_as_longlong(hsum[i]);
+      const int es = (int)(sb >> 52) - 1023;
+      one = safe && sb < INF_BITS && sb != 0 ? (float)(es - lsb) + log2_mant_up(sb) + 0.01f : bits + lk;
+    }
+    const int o = h ? 3 : 0;
+    v[o] = fmaxf(v[o], bits);
+    v[o + 1] = fmaxf(v[o + 1], one);
+    v[o + 2] = fmaxf(v[o + 2], two);
+  }
+  __shared__ float sv[32][6];
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int t = 0; t < 6; ++t) v[t] = fmaxf(v[t], __shfl_xor_sync(0xffffffffu, v[t], o));
+  if ((threadIdx.x & 31) == 0)
+    for (int t = 0; t < 6; ++t) sv[threadIdx.x >> 5][t] = v[t];
+  bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)blockDim.x / 32; ++w)
+      for (int t = 0; t < 6; ++t) v[t] = fmaxf(v[t], sv[w][t]);
+    const float need = fminf(v[1] + v[4], v[2] + v[5]) + 1.05f;
+    int g = 2;
+    while (g <= max_groups && lg.v[g] < need) ++g;
+    const bool fits = !bad && g <= max_groups && v[0] <= 14.f * EX_CHUNKS && v[3] <= 14.f * EX_CHUNKS;
+    prm->ncA = ((int)v[0] + 13) / 14;
+    prm->ncH = ((int)v[3] + 13) / 14;
+    prm->nmod = fits ? 4 * g : 0;
+    prm->run_dmma = fits ? 0u : 1u;
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+// Residues.  x * 2^-lsb is cut into NC 14-bit chunks (exact floats, signed); with
+// g_t = 2^(14 t) mod m symmetric, sum_t g_t c_t is congruent to it and below 2^14 (1 + 7 * 128) <
+// 2^24, so the FMAs are exact; quotient and remainder as in split_crt.cu's residue_f (|r| <= 128).
+// ------------------------------------------------------------------------------------------
+template <int NC>
+struct ExChunks {
+  float c[NC];
+};
+
+template <int NC>
+__device__ __forceinline__ ExChunks<NC> ex_chunks(double x, int lsb) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int ex = (int)((b >> 52) & 0x7FF);
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (ex ? 1ull << 52 : 0ull);
+  int sh = (ex ? ex : 1) - 1075 - lsb;  // >= -52: the bits shifted out are zero
+  unsigned long long lo, hi = 0;
+  if (sh <= 0) {
+    lo = m == 0 ? 0 : m >> min(63, -sh);
+  } else if (sh < 64) {
+    lo = m << sh;
+    hi = m >> (64 - sh);
+  } else {
+    lo = 0;
+    hi = m << min(63, sh - 64);
+  }
+  const bool neg = (b >> 63) != 0;
+  const float s = neg ? -1.0f : 1.0f, o = neg ? 8388608.0f : -8388608.0f;
+  ExChunks<NC> r;
+#pragma unroll
+  for (int t = 0; t < NC; ++t) {
+    const unsigned long long w = t < 4 ? lo >> (14 * t) : (t == 4 ? (lo >> 56) | (hi << 8) : hi >> (14 * t - 64));
+    r.c[t] = fmaf(__uint_as_float(0x4B000000u | ((unsigned)w & 0x3FFFu)), s, o);
+  }
+  return r;
+}
+
+// Four neighbouring integers: one 8-byte store per plane.
+template <int NC>
+__device__ __forceinline__ void ex_write_quad(const double (&x)[4], int lsb, bool ok, int nmod, uint2* dst,
+                                              size_t plane_u2) {
+  ExChunks<NC> c[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) c[q] = ex_chunks<NC>(ok ? x[q] : 0.0, lsb);
+#pragma unroll 4
+  for (int l = 0; l < nmod; ++l) {
+    const float inv = kEx.g[l][0], mf = kEx.m[l];
+    unsigned f[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float t = c[q].c[0];
+#pragma unroll
+      for (int e = 1; e < NC; ++e) t = fmaf(c[q].c[e], kEx.g[l][e], t);
+      const float qq = fmaf(t, inv, 12582912.0f) - 12582912.0f;
+      f[q] = __float_as_uint(fmaf(-qq, mf, t));
+    }
+    *dst = make_uint2(__byte_perm(f[0], f[1], 0x7632), __byte_perm(f[2], f[3], 0x7632));
+    dst += plane_u2;
+  }
+}
+
+__device__ __forceinline__ void ex_write_quad_nc(int nc, const double (&x)[4], int lsb, bool ok, int nmod, uint2* dst,
+                                                 size_t plane_u2) {
+  if (nc <= 4)
+    ex_write_quad<4>(x, lsb, ok, nmod, dst, plane_u2);
+  else if (nc <= 6)
+    ex_write_quad<6>(x, lsb, ok, nmod, dst, plane_u2);
+  else
+    ex_write_quad<8>(x, lsb, ok, nmod, dst, plane_u2);
+}
+
+// RA[l][i][kk], rows i, K-major: 64 x 64 tiles of A transposed through shared memory (element
+// (k, r) at column (r + k/4) mod 64 of row k: conflict-free both ways).
+__global__ void __launch_bounds__(256) k_ex_residues_A(const double* __restrict__ A, long lda, int n, int k, int kp,
+                                                       const int* __restrict__ alsb, const ExParams* prm,
+                                                       __nv_bfloat16* __restrict__ RA) {
+  __shared__ double tile[64][64];
+  const int nmod = prm->nmod;
+  if (nmod == 0) return;
+  const int nc = prm->ncA;
+  const int i0 = blockIdx.x * 64, k0 = blockIdx.y * 64;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int kk = ty; kk < 64; kk += 8) {
+    const int gk = k0 + kk;
+#pragma unroll
+    for (int rr = tx; rr < 64; rr += 32) {
+      const int gi = i0 + rr;
+      tile[kk][(rr + (kk >> 2)) & 63] = (gi < n && gk < k) ? __ldg(A + gi + (long)gk * lda) : 0.0;
+    }
+  }
+  __syncthreads();
+  const size_t plane = (size_t)n * kp;
+  const int tq = threadIdx.x & 15, tr = threadIdx.x >> 4;
+  for (int r = tr; r < 64; r += 16) {
+    const int gi = i0 + r;
+    if (gi >= n) continue;
+    const int lsb = alsb[gi], kk = 4 * tq;
+    double x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = tile[kk + q][(r + tq) & 63];
+    ex_write_quad_nc(nc, x, lsb, lsb != NO_LSB, nmod, (uint2*)(RA + (size_t)gi * kp + k0 + kk), plane / 4);
+  }
+}
+
+__global__ void __launch_bounds__(128) k_ex_residues_H(const double* __restrict__ Ht, int ncols, int kp,
+                                                       const int* __restrict__ hlsb, const ExParams* prm,
+                                                       __nv_bfloat16* __restrict__ RH) {
+  const int nmod = prm->nmod;
+  if (nmod == 0) return;
+  const int j = blockIdx.x, kk = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
+  if (kk >= kp) return;  // kp is a multiple of 64
+  const int lsb = hlsb[j];
+  const double2 h01 = *(const double2*)(Ht + (size_t)j * kp + kk);
+  const double2 h23 = *(const double2*)(Ht + (size_t)j * kp + kk + 2);
+  const double x[4] = {h01.x, h01.y, h23.x, h23.y};
+  const size_t plane = (size_t)ncols * kp;
+  ex_write_quad_nc(prm->ncH, x, lsb, lsb != NO_LSB, nmod, (uint2*)(RH + (size_t)j * kp + kk), plane / 4);
+}
+
+// ------------------------------------------------------------------------------------------
+// CRT
+// ------------------------------------------------------------------------------------------
+__device__ __noinline__ double ex_outside_normal(unsigned long long m, int x, bool neg) {
+  const double v = ldexp((double)m, x);
+  return neg ? -v : v;
+}
+
+// The magnitude in four 64-bit words times 2^e as a double, rounded to nearest even.
+__device__ __forceinline__ double ex_round(const unsigned long long (&w)[4], bool neg, int e) {
+  unsigned long long h, l, rest;
+  int p;
+  if (w[3]) {
+    h = w[3]; l = w[2]; rest = w[1] | w[0]; p = 255;
+  } else if (w[2]) {
+    h = w[2]; l = w[1]; rest = w[0]; p = 191;
+  } else if (w[1]) {
+    h = w[1]; l = w[0]; rest = 0; p = 127;
+  } else {
+    h = w[0]; l = 0; rest = 0; p = 63;
+  }
+  if (h == 0) return 0.0;
+  const int s = __clzll((long long)h);
+  p -= s;
+  const unsigned long long top = s ? (h << s) | (l >> (64 - s)) : h;
+  rest |= s ? l << s : l;
+  unsigned long long m = top >> 11;
+  const bool sticky = (top & 0x3FFull) != 0 || rest != 0;
+  const unsigned long long up = (top & 0x400ull) && (sticky || (m & 1));
+  const int field = p + e + 1023;
+  if (field >= 1 && field <= 2045) {  // adding the carry to the bits moves the exponent with it
+    unsigned long long bits = (((unsigned long long)field << 52) | (m & 0xFFFFFFFFFFFFFull)) + up;
+    if (neg) bits |= 1ull << 63;
+    return __longlong_as_double((long long)bits);
+  }
+  // subnormal or overflowing results: one rounding at their own precision, from 63 bits and a
+  // sticky bit (ldexp rounds a double exactly scaled; the 53-bit m would be rounded twice)
+  if (field > 2045) return ex_outside_normal(m + up, p - 52 + e, neg);
+  const int drop = 1 - field + 11;  // bits of `top` below the subnormal's last place
+  if (drop > 64) return neg ? -0.0 : 0.0;
+  const unsigned long long keep = drop < 64 ? top >> drop : 0;
+  const unsigned long long half = 1ull << (drop - 1);
+  const bool st2 = (top & (half - 1)) != 0 || rest != 0;
+  unsigned long long bits = keep + (((top & half) && (st2 || (keep & 1))) ? 1 : 0);
+  if (neg) bits |= 1ull << 63;
+  return __longlong_as_double((long long)bits);
+}
+
+// Column c's element from its 4 G residues, offset by 128 (word l holds modulus l's for four
+// columns), times 2^e.
+template <int G>
+__device__ __forceinline__ double ex_crt(const unsigned (&w)[EX_MAX], int c, int e) {
+  constexpr int NL = G + 1;  // 28-bit limbs: log2 M = 63.7, 95, 125, 156, 185, 214, 241 for G = 2..8
+  const ExCrt& C = kEx.crt[G];
+  unsigned long long acc[NL];
+#pragma unroll
+  for (int t = 0; t < NL; ++t) acc[t] = 0;
+  unsigned qs = 0;
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    unsigned t = C.b[g], f = C.fb[g];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const unsigned u = __byte_perm(w[4 * g + i], 0u, 0x4440u + c);
+      t += u * C.c[4 * g + i];
+      f += u * C.f[4 * g + i];
+    }
+    const unsigned X = t - (f >> 20) * C.P[g];  // in [0, 1.002 P_g), below 2^32
+    qs += __umulhi(X, C.G[g]);                  // 2^20 X / P_g
+#pragma unroll
+    for (int s = 0; s < NL; ++s) acc[s] += (unsigned long long)X * C.W[g][s];
+  }
+  const unsigned q = (qs + (1u << 19)) >> 20;
+  long long carry = 0;
+  unsigned long long word[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int s = 0; s < NL; ++s) {
+    const long long z = (long long)acc[s] - (long long)((unsigned long long)q * C.M[s]) + carry;
+    const int off = (28 * s) & 63, wi = (28 * s) >> 6;
+    if (s < NL - 1) {
+      const unsigned long long d = (unsigned long long)z & 0xFFFFFFFull;
+      carry = z >> 28;
+      word[wi] |= d << off;
+      if (off > 36) word[wi + 1] |= d >> (64 - off);
+    } else {  // the top limb carries the sign
+      word[wi] |= (unsigned long long)z << off;
+#pragma unroll
+      for (int v = wi + 1; v < 4; ++v)
+        word[v] = (unsigned long long)(v == wi + 1 && off ? z >> (64 - off) : z >> 63);
+    }
+  }
+  const bool neg = (long long)word[3] < 0;
+  if (neg) {
+    unsigned long long cy = 1;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      word[v] = ~word[v] + cy;
+      cy = cy && word[v] == 0;
+    }
+  }
+  return ex_round(word, neg, e);
+}
+
+// TI rows x 128 columns a block (32 x 8 threads), four neighbouring columns of a row per thread,
+// transposed through shared memory as in crt_combine_blk.  TI = 32 writes whole 256-byte runs of
+// Q's columns; small outputs take TI = 8, four times the blocks, each with a quarter of the serial
+// recombinations (n = 256: 16 blocks are a tenth of the SMs).
+template <int G, int TI>
+__device__ __forceinline__ void ex_combine(const int8_t* __restrict__ R, int n, int k, int kr,
+                                           const int* __restrict__ alsb, const int* __restrict__ hlsb, double alpha,
+                                           double beta, double* __restrict__ Q, long ldq, double (&tile)[128][TI]) {
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int i0 = blockIdx.y * TI, j0 = blockIdx.x * 128, jb = j0 + 4 * tx;
+  const size_t plane = (size_t)n * kr;
+  for (int a = 0; a < TI / 8; ++a) {
+    const int il = ty + 8 * a, i = i0 + il;
+    double val[4] = {0.0, 0.0, 0.0, 0.0};
+    if (i < n && jb < k) {
+      unsigned w[EX_MAX];
+      const int8_t* rp = R + (size_t)i * kr + jb;
+#pragma unroll
+      for (int l = 0; l < 4 * G; ++l) w[l] = __ldg((const unsigned*)(rp + (size_t)l * plane)) ^ 0x80808080u;
+      const int ea = alsb[i];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int eh = jb + c < k ? hlsb[jb + c] : NO_LSB;
+        if (ea != NO_LSB && eh != NO_LSB) val[c] = ex_crt<G>(w, c, ea + eh);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) tile[4 * tx + c][(il + tx) & (TI - 1)] = val[c];
+  }
+  __syncthreads();
+  const bool scale = alpha != 1.0, accumulate = beta != 0.0;
+  const int t = ty * 32 + tx, ir = t % TI, i = i0 + ir;
+  for (int jl = t / TI; jl < 128; jl += 256 / TI) {
+    const int jj = j0 + jl;
+    if (i < n && jj < k) {
+      double* qp = Q + i + (long)jj * ldq;
+      double v = tile[jl][(ir + (jl >> 2)) & (TI - 1)];
+      if (scale || accumulate) {
+        v *= alpha;
+        if (accumulate) v = fma(beta, *qp, v);
+      }
+      *qp = v;
+    }
+  }
+}
+
+template <int TI>
+__global__ void __launch_bounds__(256, 2) k_ex_combine(const int8_t* __restrict__ R, int n, int k, int kr, ExParams* prm,
+                                                    const int* __restrict__ alsb, const int* __restrict__ hlsb,
+                                                    double alpha, double beta, double* __restrict__ Q, long ldq) {
+  __shared__ double tile[128][TI];
+  const int nmod = prm->nmod;
+  if (nmod == 0) return;
+  if (prm->status != 0) {  // a wait of the GEMM gave up: the DMMA kernel computes the product
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) prm->run_dmma = 1u;
+    return;
+  }
+  switch (nmod / 4) {
+    case 2: ex_combine<2, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
+    case 3: ex_combine<3, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
+    case 4: ex_combine<4, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
+    case 5: ex_combine<5, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
+    case 6: ex_combine<6, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
+    case 7: ex_combine<7, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
+    default: ex_combine<8, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
+  }
+}
+
+ExLog2 ex_log2() {
+  ExLog2 r;
+  double l = 0.0;
+  r.v[0] = r.v[1] = 0.0f;
+  for (int i = 0; i < EX_MAX; ++i) {
+    l += std::log2((double)kExModuli[i]);
+    if (i % 4 == 3) r.v[(i + 1) / 4] = (float)(l - 1e-3);
+  }
+  return r;
+}
+
+constexpr size_t EX_WORK_CAP = (size_t)40 << 30;
+
+// Planes the workspace cap allows (a multiple of 4, at most 32).
+int ex_planes(int M, int N, int K) {
+  int planes = EX_MAX;
+  while (planes > 0 && ex_layout(M, N, K, planes).total > EX_WORK_CAP) planes -= 4;
+  return planes;
+}
+
+}  // namespace
+
+size_t exact_workspace(int M, int N, int K) {
+  const int planes = ex_planes(M, N, K);
+  return planes >= 16 ? ex_layout(M, N, K, planes).total : 0;
+}
+
+// Every size the passes' grids cover: the DMMA kernel's time is that of whole 128 x 128 x 16 tile
+// steps, about 75 us each (2 FP64 FMAs per SM and cycle), so that it is slower from one step on
+// (n = 32: 166 us against 61-68; n = 256: 609 / 92; n = 2048: 16.4 ms / 0.75; n = 4096: 129 / 3.0).
+bool exact_route(int M, int N, int K) { return K < (1 << 21) && M <= 8 * 65535 && N <= 8 * 65535; }
+
+// Enqueues the exact route of Q (M x N) = alpha A (M x K) H (K x N) + beta Q; *gate receives the
+// device word that tells the DMMA kernel behind it to run.
+int launch_exact(int M, int N, int K, double alpha, const double* A, long lda, const GenSpec& gs, double beta,
+                 double* Q, long ldq, void* work, size_t lwork, cudaStream_t stream, const unsigned** gate) {
+  const int planes = ex_planes(M, N, K);
+  const ExLayout L = ex_layout(M, N, K, planes);
+  if (planes < 16 || !work || lwork < L.total) return PSMMA_EWORKSPACE;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return PSMMA_EDEVICE;
+  static const ExLog2 lg = ex_log2();
+  char* w = (char*)work;
+  ExParams* prm = (ExParams*)w;
+  auto* amax = (unsigned long long*)(w + L.off_amax);
+  auto* hmax = (unsigned long long*)(w + L.off_hmax);
+  double *asq = (double*)(w + L.off_asq), *hsum = (double*)(w + L.off_hsum), *hsq = (double*)(w + L.off_hsq);
+  int *alsb = (int*)(w + L.off_alsb), *hlsb = (int*)(w + L.off_hlsb);
+  double* Ht = (double*)(w + L.off_ht);
+  auto* RA = (__nv_bfloat16*)(w + L.off_ra);
+  auto* RH = (__nv_bfloat16*)(w + L.off_rh);
+  int8_t* R = (int8_t*)(w + L.off_r);
+  *gate = &prm->run_dmma;
+
+  prof_begin(stream);
+  k_ex_init<<<(M + 255) / 256, 256, 0, stream>>>(prm, amax, asq, alsb, M);
+  // enough blocks for some eight waves, so that the loads of a chunk (eight in flight a thread) are
+  // not a serial chain: n = 2048 at 1024-column chunks 208 us, n = 256 at 128 27 us
+  int kchunk = 1024;
+  while (kchunk > 16 && (long)((M + 127) / 128) * ((K + kchunk - 1) / kchunk) < 8L * sms) kchunk >>= 1;
+  k_ex_row_stats<<<dim3((M + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, stream>>>(A, lda, M, K, kchunk, amax, asq,
+                                                                                     alsb);
+  prof_mark(stream, "row_scale");
+  switch (gs.kind) {
+    case KIND_CAUCHY: k_ex_h<KIND_CAUCHY><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
+    case KIND_TOEPLITZ: k_ex_h<KIND_TOEPLITZ><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
+    case KIND_HANKEL: k_ex_h<KIND_HANKEL><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
+    case KIND_CAUCHY_EIG: k_ex_h<KIND_CAUCHY_EIG><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
+    default: return PSMMA_EUNSUPPORTED;
+  }
+  prof_mark(stream, "h_generate");
+  k_ex_params<<<1, 1024, 0, stream>>>(prm, lg, planes / 4, M, N, K, amax, asq, alsb, hmax, hsum, hsq, hlsb);
+  prof_mark(stream, "params");
+  k_ex_residues_A<<<dim3((M + 63) / 64, L.kp / 64), 256, 0, stream>>>(A, lda, M, K, L.kp, alsb, prm, RA);
+  prof_mark(stream, "residues_A");
+  k_ex_residues_H<<<dim3(N, (L.kp / 4 + 127) / 128), 128, 0, stream>>>(Ht, N, L.kp, hlsb, prm, RH);
+  prof_mark(stream, "residues_H");
+  const int st = launch_modular_gemm(RA, RH, R, M, N, L.kp, L.kr, planes, kExModuli, &prm->nmod, &prm->status, sms, stream);
+  if (st) return st;
+  prof_mark(stream, "modular_gemm");
+  const int cols = (N + 127) / 128;
+  if ((long)cols * ((M + 31) / 32) >= 4L * sms)
+    k_ex_combine<32><<<dim3(cols, (M + 31) / 32), dim3(32, 8), 0, stream>>>(R, M, N, L.kr, prm, alsb, hlsb, alpha, beta,
+                                                                            Q, ldq);
+  else
+    k_ex_combine<8><<<dim3(cols, (M + 7) / 8), dim3(32, 8), 0, stream>>>(R, M, N, L.kr, prm, alsb, hlsb, alpha, beta, Q,
+                                                                         ldq);
+  prof_mark(stream, "crt_combine");
+  return cudaGetLastError() == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
+}
+
+}  // namespace psmma

@@ -51,6 +51,11 @@ void* pool_get(size_t bytes, cudaStream_t stream, int* status, int slot) {
   return pl.ptr;
 }
 
+bool stream_capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone;
+}
+
 // ------------------------------------------------------------------------------------
 // Per-(device, stream) status words: the split path's asynchronous calls OR their device
 // status (DEV_ERR_TIMEOUT when a bounded wait gave up) into the word of their stream;
@@ -93,10 +98,7 @@ bool g_prof_created = false;
 bool prof_enabled() { return g_prof_on; }
 
 // Phases inside a stream capture are not traced (their events would belong to the graph).
-static bool capturing(cudaStream_t stream) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone;
-}
+static bool capturing(cudaStream_t stream) { return stream_capturing(stream); }
 
 void prof_begin(cudaStream_t stream) {
   if (!g_prof_on || capturing(stream)) return;
@@ -193,6 +195,29 @@ void* f64_work(int M, int N, int K, const psmma_opts* o, cudaStream_t s, size_t*
   return w;
 }
 
+// A real product on the FP64 precision: the exact modular route where it is the faster one, with
+// the DMMA kernel enqueued behind it for the operands it does not take (decided on the device);
+// else the DMMA kernel alone.  The route needs a workspace of its own, which a caller that brings
+// opts->work has not sized, and which a graph must not keep by its address: both keep the kernel.
+int run_f64(int n, int k, double alpha, const double* A, int lda, const GenSpec& gs, double beta, double* Q, int ldq,
+            const psmma_opts* o, cudaStream_t s) {
+  int st = PSMMA_OK;
+  size_t wb = 0;
+  void* w = f64_work(n, k, k, o, s, &wb, &st);
+  if (st) return st;
+  const unsigned* gate = nullptr;
+  if (alpha != 0.0 && !o->work && exact_route(n, k, k) && !stream_capturing(s)) {
+    const size_t need = exact_workspace(n, k, k);
+    int pst = PSMMA_OK;
+    void* xw = need ? pool_get(need, s, &pst) : nullptr;
+    if (xw) {
+      st = launch_exact(n, k, k, alpha, A, lda, gs, beta, Q, ldq, xw, need, s, &gate);
+      if (st) return st;
+    }
+  }
+  return launch_struct_f64_ws(n, k, k, alpha, A, lda, gs, beta, Q, ldq, w, wb, s, gate);
+}
+
 int run_real(int kind, int n, int k, double alpha, const double* A, int lda, const double* gen,
              int ldgen, double beta, double* Q, int ldq, const psmma_opts* opts, void* stream) {
   const psmma_opts* o = opts ? opts : &kDefaultOpts;
@@ -214,10 +239,7 @@ int run_real(int kind, int n, int k, double alpha, const double* A, int lda, con
     return launch_split(kind, n, k, alpha, A, lda, gen, ldgen, beta, Q, ldq, o->n_moduli, work,
                         need, s, false, o->block_levels);
   }
-  size_t wb = 0;
-  void* w = f64_work(n, k, k, o, s, &wb, &st);
-  if (st) return st;
-  return launch_struct_f64_ws(n, k, k, alpha, A, lda, reference_gens(kind, gen, ldgen, k), beta, Q, ldq, w, wb, s);
+  return run_f64(n, k, alpha, A, lda, reference_gens(kind, gen, ldgen, k), beta, Q, ldq, o, s);
 }
 
 int run_dft(int n, int k, double alpha, const psmma_complex* B, int ldb, double beta,
@@ -438,10 +460,7 @@ int run_eig(int n, int k, double alpha, const double* A, int lda, const double* 
     return launch_split_general(n, k, k, alpha, A, lda, gs, beta, Q, ldq, o->n_moduli, work, need, s, dstat,
                                 o->block_levels);
   }
-  size_t wb = 0;
-  void* w = f64_work(n, k, k, o, s, &wb, &st);
-  if (st) return st;
-  return launch_struct_f64_ws(n, k, k, alpha, A, lda, gs, beta, Q, ldq, w, wb, s);
+  return run_f64(n, k, alpha, A, lda, gs, beta, Q, ldq, o, s);
 }
 
 int host_eig(int n, int k, double alpha, const double* A, int lda, const double* F, const double* U,

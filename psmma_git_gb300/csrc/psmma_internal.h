@@ -111,7 +111,15 @@ int launch_struct_f64(int M, int N, int K, double alpha, const double* X, long l
 // The same with a workspace for split K (used when the output has too few tiles to fill the
 // SMs and lwork >= f64_splitk_bytes); work may be NULL.
 int launch_struct_f64_ws(int M, int N, int K, double alpha, const double* X, long ldx, const GenSpec& gs,
-                         double beta, double* C, long ldc, void* work, size_t lwork, cudaStream_t stream);
+                         double beta, double* C, long ldc, void* work, size_t lwork, cudaStream_t stream,
+                         const unsigned* gate = nullptr);
+// The FP64 precision's exact modular route (exact_crt.cu): whether it is the faster one for a
+// product of these sizes, the bytes it needs (0: none fits its workspace cap), and its launches.
+// *gate receives the device word that makes the DMMA kernel enqueued behind it run.
+bool exact_route(int M, int N, int K);
+size_t exact_workspace(int M, int N, int K);
+int launch_exact(int M, int N, int K, double alpha, const double* A, long lda, const GenSpec& gs, double beta,
+                 double* Q, long ldq, void* work, size_t lwork, cudaStream_t stream, const unsigned** gate);
 size_t f64_splitk_bytes(int M, int N, int K, int sms);
 int launch_dft_table(double2* w, int n, cudaStream_t stream);
 // C (n x k complex, ldc) = alpha F_n B + beta C on the FP64 path (plain embedding, or the
@@ -230,6 +238,8 @@ int f64_group_enqueue(const F64Group& g, cudaStream_t stream);
 // Library-owned device workspace (psmma_capi.cu): grow-only, one pool per (device, stream,
 // slot); a call that needs two independent regions takes them from two slots.
 void* pool_get(size_t bytes, cudaStream_t stream, int* status, int slot = 0);
+// Whether work enqueued on `stream` is being captured into a graph.
+bool stream_capturing(cudaStream_t stream);
 
 // Per-phase tracing (psmma_capi.cu): when enabled, launchers record a CUDA event on the
 // launch stream after each phase; psmma_profile_read turns them into milliseconds.

@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "psmma_internal.h"
+#include "split_passes.cuh"
 #include "tcgen05_util.cuh"
 
 namespace psmma {
@@ -57,18 +58,6 @@ struct CrtConsts {
   unsigned long long biasl[4];         // sum_l 128 * climb[l][t], per limb, unreduced
   unsigned Mlimb[4];                   // M as four 32-bit limbs
   int top32;                           // sum_l 255 * climb[l][3] < 2^32: top limb summed in 32 bits
-};
-
-// Device-side parameters of one call (in the workspace).
-constexpr int PARAMS_BLOCKS = 32;  // blocks of the single-product parameter pass
-
-struct SplitDevParams {
-  unsigned status;
-  int PA, PH;                   // bits of the integer-scaled A (per row) and H (per column)
-  unsigned long long rho_bits;  // max_j sum_k |H_kj| / max_k |H_kj| (bits of a positive double)
-  unsigned done;                // parameter-pass blocks finished
-  unsigned hbad;                // block-recursive products: some column of H is not finite
-  double part[PARAMS_BLOCKS][6];  // their partial ratio maxima and sums, combined in block order
 };
 
 // ------------------------------------------------------------------------------------------
@@ -272,217 +261,9 @@ size_t split_workspace_general(int M, int N, int K, int n_moduli, int block_req)
 // ------------------------------------------------------------------------------------------
 // Pass kernels
 // ------------------------------------------------------------------------------------------
-constexpr unsigned long long ABS_MASK = 0x7FFFFFFFFFFFFFFFull;
-constexpr unsigned long long INF_BITS = 0x7FF0000000000000ull;
-constexpr int NO_SCALE = -100000;
-
-// The bound sums (row sums of squares of A, column sums of |H| and of H^2) are accumulated in
-// FP32 on a per-thread power-of-two scale, because GB300 issues FP64 at about one operation
-// per SM per cycle.  abs_scaled_up gives |x| * 2^-e as a float that is never below the true
-// value (top 23 mantissa bits, rounded up; magnitudes under 2^-126 become 2^-126), from the
-// bits of x on the integer pipe, and sets *big when |x| * 2^-e >= 2^56 (then the caller sums
-// that thread's values in FP64 instead).  With round-up FP32 adds the sums stay upper bounds.
-__device__ __forceinline__ float abs_scaled_up(unsigned long long ab, int e, bool* big) {
-  const int fe = (int)(ab >> 52) - 1023 - e + 127;
-  *big |= fe >= 127 + 56;
-  const int fc = max(1, min(fe, 254));
-  unsigned fb = ((unsigned)fc << 23) | ((unsigned)(ab >> 29) & 0x7FFFFFu);
-  fb += (fe < 1 || (ab & 0x1FFFFFFFull) != 0ull) ? 1u : 0u;
-  return ab ? __uint_as_float(fb) : 0.0f;
-}
-
-// Row max of |A| as the bits of a non-negative double (NaN/Inf compare above all finite) and
-// row sums of squares (for the Cauchy-Schwarz bound of the integer product).
-// Columns kk >= ka of A come from A2 (ld lda2) at kk - ka (ka = k: A alone).
-__device__ __forceinline__ const double* acol(const double* A, long lda, const double* A2, long lda2, int ka,
-                                              int kk) {
-  return kk < ka ? A + (long)kk * lda : A2 + (long)(kk - ka) * lda2;
-}
-
-__device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, long lda, const double* A2, long lda2,
-                                               int ka, int n, int k, int kchunk,
-                                               unsigned long long* __restrict__ amax_bits,
-                                               double* __restrict__ asq, int bx, int by) {
-  int i = bx * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int k0 = by * kchunk, k1 = min(k, k0 + kchunk);
-  unsigned long long mb = 0;
-  float sq32 = 0.0f;
-  int e = NO_SCALE;  // set by the first group with a nonzero entry
-  bool big = false;
-  int kk = k0;
-  // eight independent loads in flight per thread (a warp reads 32 consecutive rows)
-  for (; kk + 8 <= k1; kk += 8) {
-    unsigned long long b[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      b[u] = (unsigned long long)__double_as_longlong(__ldg(acol(A, lda, A2, lda2, ka, kk + u) + i)) & ABS_MASK;
-    unsigned long long gm = 0;
-#pragma unroll
-    for (int u = 0; u < 8; ++u) gm = b[u] > gm ? b[u] : gm;
-    mb = gm > mb ? gm : mb;
-    if (e == NO_SCALE && gm) e = (int)(gm >> 52) - 1023;
-    if (e != NO_SCALE) {
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const float f = abs_scaled_up(b[u], e, &big);
-        sq32 = __fmaf_ru(f, f, sq32);
-      }
-    }
-  }
-  for (; kk < k1; ++kk) {
-    const unsigned long long b =
-        (unsigned long long)__double_as_longlong(__ldg(acol(A, lda, A2, lda2, ka, kk) + i)) & ABS_MASK;
-    mb = b > mb ? b : mb;
-    if (e == NO_SCALE && b) e = (int)(b >> 52) - 1023;
-    if (e != NO_SCALE) {
-      const float f = abs_scaled_up(b, e, &big);
-      sq32 = __fmaf_ru(f, f, sq32);
-    }
-  }
-  double sq = 0.0;
-  if (big) {  // entries 2^56 times the thread's first ones (or Inf/NaN): FP64 sum
-    for (kk = k0; kk < k1; ++kk) {
-      const double a = __ldg(acol(A, lda, A2, lda2, ka, kk) + i);
-      sq = fma(a, a, sq);
-    }
-  } else if (e != NO_SCALE) {
-    sq = ldexp((double)sq32, 2 * e);
-  }
-  if (mb) atomicMax(amax_bits + i, mb);
-  if (sq != 0.0) atomicAdd(asq + i, sq);
-}
-
 __global__ void k_row_absmax(const double* __restrict__ A, long lda, int n, int k, int kchunk,
                              unsigned long long* __restrict__ amax_bits, double* __restrict__ asq) {
   row_absmax_blk(A, lda, nullptr, 0, k, n, k, kchunk, amax_bits, asq, blockIdx.x, blockIdx.y);
-}
-
-// H pass 1: Ht[j][kk] = H(kk, j) in FP64, column max |H| and column sum |H|, and the global
-// ratio rho = max_j sum/max over finite columns.  One block per column j.
-template <int KIND>
-// hmax_all != nullptr receives the column maximum over every generated row (with gs.srows the
-// statistics cover the first srows rows only).
-__device__ __forceinline__ void h_pass1_blk(const GenSpec& gs, int K, int kp, double* __restrict__ Ht,
-                                            unsigned long long* __restrict__ hmax_bits, double* __restrict__ hsum,
-                                            double* __restrict__ hsq, SplitDevParams* prm, int j,
-                                            unsigned long long* __restrict__ hmax_all = nullptr) {
-  double w = 0.0, v = 0.0, w1 = 0.0, dlj = 0.0, drj = 0.0;
-  VSplit vs;
-  vs.ok = false;
-  if (KIND == KIND_CAUCHY || KIND == KIND_CAUCHY_EIG) {
-    w = __ldg(gs.Fc + j);   // F(j)
-    v = __ldg(gs.Vc + j);   // V(j)
-    vs = v_split(v);
-  }
-  if (KIND == KIND_CAUCHY_EIG) {
-    dlj = __ldg(gs.dl + j);  // DIFL(j)
-    if (j < gs.fc1_len) {
-      w1 = __ldg(gs.Fc1 + j);  // F(j+1)
-      drj = __ldg(gs.dr + j);  // DIFR(j)
-    }
-  }
-  unsigned long long mb = 0, mb_all = 0;
-  float s32 = 0.0f, s2_32 = 0.0f;
-  int e = NO_SCALE;  // set by the thread's first nonzero entry
-  bool big = false;
-  const long srows = gs.srows > 0 ? gs.srows : (long)kp;
-  double* row = Ht + (long)j * kp;
-  for (int kk = threadIdx.x; kk < kp; kk += blockDim.x) {
-    double h = 0.0;
-    if (kk < K) {
-      if (KIND == KIND_CAUCHY) {
-        if (gs.k1 > 0 && kk >= gs.k1) {
-          const int t = kk - gs.k1;  // tail rows: dense, or Cauchy with the second row generators
-          h = gs.B ? __ldg(gs.B + t + (long)j * gs.ldb) : cauchy_entry(__ldg(gs.Ur2 + t), v, vs, __ldg(gs.Dr2 + t) - w);
-        } else {
-          double d = __ldg(gs.Dr + kk), u = __ldg(gs.Ur + kk);
-          h = cauchy_entry(u, v, vs, d - w);  // U(i)*V(j) / (D(i)-F(j))
-        }
-      } else if (KIND == KIND_CAUCHY_EIG) {
-        if (gs.k1 > 0 && kk >= gs.k1) {
-          // tail rows of merged products: dense, or CauchyEig rows in permuted order
-          const int t = kk - gs.k1;
-          h = gs.B ? __ldg(gs.B + t + (long)j * gs.ldb)
-                   : cauchy_entry(__ldg(gs.Ur2 + t), v, vs,
-                                  eig_den(__ldg(gs.Dr2 + t), w, w1, dlj, drj, __ldg(gs.rglob2 + t) - 1 <= gs.cg0 + j));
-        } else {
-          const double fi = __ldg(gs.Dr + kk), u = __ldg(gs.Ur + kk);
-          const bool upper = gs.rglob ? (__ldg(gs.rglob + kk) - 1 <= gs.cg0 + j) : (kk - j <= gs.diag_off);
-          h = cauchy_entry(u, v, vs, eig_den(fi, w, w1, dlj, drj, upper));
-        }
-      } else if (KIND == KIND_TOEPLITZ || KIND == KIND_HANKEL) {
-        if (gs.k1 > 0 && kk >= gs.k1) {  // dense tail rows (the R P^T factor of a merged product)
-          h = __ldg(gs.B + (kk - gs.k1) + (long)j * gs.ldb);
-        } else {
-          const long idx = KIND == KIND_TOEPLITZ ? (gs.order - 1) + j - kk : (long)kk + j;
-          h = (gs.glen <= 0 || (idx >= 0 && idx < gs.glen)) ? __ldg(gs.g + idx) : 0.0;
-        }
-      } else {  // KIND_DENSE (the split DFT generates F in k_h_pass1_dft3)
-        h = __ldg(gs.B + kk + (long)j * gs.ldb);
-      }
-    }
-    row[kk] = h;
-    unsigned long long b = (unsigned long long)__double_as_longlong(h) & ABS_MASK;
-    mb_all = b > mb_all ? b : mb_all;
-    if (kk >= srows) continue;
-    mb = b > mb ? b : mb;
-    if (e == NO_SCALE && b) e = (int)(b >> 52) - 1023;
-    if (e != NO_SCALE) {
-      const float f = abs_scaled_up(b, e, &big);
-      s32 = __fadd_ru(s32, f);
-      s2_32 = __fmaf_ru(f, f, s2_32);
-    }
-  }
-  double s = 0.0, s2 = 0.0;
-  if (big) {  // entries 2^56 times the thread's first one (or Inf/NaN): FP64 sums
-    for (int kk = threadIdx.x; kk < srows; kk += blockDim.x) {
-      const double h = row[kk];
-      s += fabs(h);
-      s2 = fma(h, h, s2);
-    }
-  } else if (e != NO_SCALE) {
-    s = ldexp((double)s32, e);
-    s2 = ldexp((double)s2_32, 2 * e);
-  }
-  __shared__ unsigned long long smax[32], smax_all[32];
-  __shared__ double ssum[32], ssq[32];
-  for (int o = 16; o > 0; o >>= 1) {
-    unsigned long long ob = __shfl_xor_sync(0xffffffffu, mb, o);
-    mb = ob > mb ? ob : mb;
-    ob = __shfl_xor_sync(0xffffffffu, mb_all, o);
-    mb_all = ob > mb_all ? ob : mb_all;
-    s += __shfl_xor_sync(0xffffffffu, s, o);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-  }
-  int wid = threadIdx.x >> 5, ln = threadIdx.x & 31;
-  if (ln == 0) { smax[wid] = mb; smax_all[wid] = mb_all; ssum[wid] = s; ssq[wid] = s2; }
-  __syncthreads();
-  if (wid == 0) {
-    int nw = blockDim.x >> 5;
-    mb = ln < nw ? smax[ln] : 0ull;
-    mb_all = ln < nw ? smax_all[ln] : 0ull;
-    s = ln < nw ? ssum[ln] : 0.0;
-    s2 = ln < nw ? ssq[ln] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) {
-      unsigned long long ob = __shfl_xor_sync(0xffffffffu, mb, o);
-      mb = ob > mb ? ob : mb;
-      ob = __shfl_xor_sync(0xffffffffu, mb_all, o);
-      mb_all = ob > mb_all ? ob : mb_all;
-      s += __shfl_xor_sync(0xffffffffu, s, o);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-    }
-    if (ln == 0) {
-      if (hmax_all) hmax_all[j] = mb_all;
-      hmax_bits[j] = mb;
-      hsum[j] = s;
-      hsq[j] = s2;
-      if (mb > 0 && mb < INF_BITS && isfinite(s)) {
-        double rho = s / __longlong_as_double((long long)mb);
-        atomicMax(&prm->rho_bits, (unsigned long long)__double_as_longlong(rho));
-      }
-    }
-  }
 }
 
 template <int KIND>
@@ -618,13 +399,6 @@ __global__ void k_split_params(SplitDevParams* prm, double log2M, int n, int nco
       params_finish(prm, log2M, k, tot);
     }
   }
-}
-
-// floor(log2 x) from the bits of a positive finite double, on the integer pipe (GB300's FP64
-// pipe is narrow, and the library ilogb goes through it).
-__device__ __forceinline__ int ilogb_bits(unsigned long long b) {
-  const int ex = (int)(b >> 52);
-  return ex ? ex - 1023 : 63 - __clzll((long long)b) - 1074;  // subnormal: b is the mantissa
 }
 
 // Exponent s such that |x * 2^s| < 2^P for all |x| <= amax (amax finite, > 0).
@@ -1437,6 +1211,7 @@ constexpr int G_STAGES = 4;
 constexpr int G_CHUNK_KB = 16;
 // Chunk sums are added as int32 and reduced modulo m every 16 chunks: |sum| <= 2^28 + 128.
 constexpr int G_RED_CHUNKS = 16;
+constexpr int GEMM_MAX_MODULI = 32;  // a launch's moduli (exact_crt.cu runs up to 32)
 constexpr int G_EPI_WARPS = 8;
 constexpr int G_THREADS = (G_EPI_WARPS + 2) * 32;
 constexpr uint32_t G_A_BYTES = G_BM * G_BK * 2;
@@ -1459,8 +1234,10 @@ struct GemmArgs {
   int gate_set;
   int8_t* R;
   unsigned* status;
-  int m[SPL_MAX_MODULI];
-  float inv_m[SPL_MAX_MODULI];
+  // planes of moduli to run, decided on the device (nullptr: nmod); at most nmod
+  const int* nmod_dev;
+  int m[GEMM_MAX_MODULI];
+  float inv_m[GEMM_MAX_MODULI];
 };
 
 // Tile t of the launch -> (modulus, row tile, column tile).  Moduli are outermost; inside a
@@ -1493,7 +1270,9 @@ struct OneGemm {
   static constexpr bool kGlobalMaps = false;
   static constexpr int kSub = 1;
   static constexpr int kEpiWarps = G_EPI_WARPS;
-  __device__ int total() const { return g.tiles_m * g.tiles_n * g.nmod; }
+  __device__ int total() const {
+    return g.tiles_m * g.tiles_n * (g.nmod_dev ? min(max(*g.nmod_dev, 0), g.nmod) : g.nmod);
+  }
   __device__ TileInfo tile(int t) const {
     TileInfo ti;
     raster_tile(g.tiles_m, g.tiles_n, g.group_m, t, ti.l, ti.tm, ti.tn);
@@ -2606,6 +2385,45 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
   if (cudaGetLastError() != cudaSuccess) return PSMMA_EDEVICE;
 
   return split_status(b.prm, stream, status_dev_out);
+}
+
+// The modular products of exact_crt.cu: R[l] (M x kr bytes) = RA[l] (M x kp) RH[l]^T (N x kp) mod
+// moduli[l] for the first *nmod_dev (at most planes) moduli.  256-column tiles, or 128 where
+// those leave SMs without a tile (small products are one tile deep per modulus).
+template <int BN>
+static int modular_gemm_launch(const OneGemm& og, int tiles, int sms, cudaStream_t stream) {
+  using Shape = GemmShape<BN>;
+  if (set_smem_attr(k_crt_gemm<BN, OneGemm>, (int)Shape::SMEM) != cudaSuccess) return PSMMA_EDEVICE;
+  k_crt_gemm<BN, OneGemm><<<std::min(sms, tiles), G_THREADS, Shape::SMEM, stream>>>(og);
+  return PSMMA_OK;
+}
+
+int launch_modular_gemm(__nv_bfloat16* RA, __nv_bfloat16* RH, int8_t* R, int M, int N, int kp, int kr, int planes,
+                        const int* moduli, const int* nmod_dev, unsigned* status, int sms, cudaStream_t stream) {
+  if (planes > GEMM_MAX_MODULI) return PSMMA_EUNSUPPORTED;
+  const int tiles_m = (M + G_BM - 1) / G_BM;
+  const bool wide = (long)tiles_m * ((N + 255) / 256) * planes >= 2L * sms;
+  const int bn = wide ? 256 : 128;
+  OneGemm og;
+  memset(&og, 0, sizeof(og));
+  if (!make_tmap(&og.ta, RA, kp, M, planes, G_BM) || !make_tmap(&og.tb, RH, kp, N, planes, bn)) return PSMMA_EDEVICE;
+  GemmArgs& ga = og.g;
+  ga.n = M;
+  ga.kr = kr;
+  ga.nkb = kp / G_BK;
+  ga.tiles_m = tiles_m;
+  ga.tiles_n = (N + bn - 1) / bn;
+  ga.group_m = 16;
+  ga.R = R;
+  ga.status = status;
+  ga.nmod = planes;
+  ga.nmod_dev = nmod_dev;
+  for (int l = 0; l < planes; ++l) {
+    ga.m[l] = moduli[l];
+    ga.inv_m[l] = 1.0f / (float)moduli[l];
+  }
+  const int tiles = ga.tiles_m * ga.tiles_n * planes;
+  return wide ? modular_gemm_launch<256>(og, tiles, sms, stream) : modular_gemm_launch<128>(og, tiles, sms, stream);
 }
 
 // ---- Block-recursive Toeplitz / Hankel products --------------------------------------------
