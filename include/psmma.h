@@ -136,13 +136,14 @@ int pzmdftl(int n, int k, double alpha, const psmma_complex* B, int ldb,
             double beta, psmma_complex* C, int ldc, const psmma_opts* opts, void* stream);
 
 /* Replaces PZMDFTL1 (pzmdftL1.f90:1-2), the RRQR variant of PZMDFTL.  Both reference
- * routines compute the same product up to their 1e-13 truncation; on the GPU the DFT
- * tile is generated exactly, so this is the same computation as pzmdftl. */
+ * routines compute the same product up to their 1e-13 truncation; on the GPU the transform
+ * is exact up to the rounding of its result, so this is the same computation as pzmdftl. */
 int pzmdftl1(int n, int k, double alpha, const psmma_complex* B, int ldb,
              double beta, psmma_complex* C, int ldc, const psmma_opts* opts, void* stream);
 
-/* No counterpart in the reference.  The radix R (1, 2, 4 or 8) of the split path's first DFT
- * step for size n: with R > 1, pzmdftl / pzmdftl1 on the split path multiply F_(n/R) by the R k
+/* No counterpart in the reference.  The radix R (1, 2, 4 or 8) of the first step of the dense DFT
+ * products (the sizes the fixed-point transform does not cover: primes above 7200 and the like)
+ * for size n: with R > 1, pzmdftl / pzmdftl1 on the split path multiply F_(n/R) by the R k
  * columns B(r::R, :) (n^2 k / R complex multiply-adds on the tensor cores) and combine the R
  * partial transforms with the twiddles w^(j r) and R-point butterflies in FP64; R is the
  * largest of 8, 4, 2 that divides n with n / R >= 1024, else 1.  0 for n <= 0. */

@@ -466,8 +466,10 @@ size_t dft_f64_workspace(int n, int k) {
 int launch_dft_f64(int n, int k, double alpha, const double* B, long ldb, double beta, double* C, long ldc,
                    void* work, size_t lwork, cudaStream_t stream) {
   if (n <= 0 || k <= 0) return PSMMA_OK;
-  if (lwork < dft_f64_workspace(n, k) || !work) return PSMMA_EWORKSPACE;
   const int R = dft_radix_for(n);
+  const size_t fft = (long)R * k > 65535L * F64_BN ? 0 : fft_workspace(n, k);
+  if (fft && work && lwork >= fft) return launch_fft(n, k, alpha, B, ldb, beta, C, ldc, true, work, lwork, stream);
+  if (lwork < dft_f64_workspace(n, k) || !work) return PSMMA_EWORKSPACE;
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
   char* w = (char*)work;
   GenSpec gs;

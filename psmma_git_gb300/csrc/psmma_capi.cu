@@ -256,7 +256,9 @@ int run_dft(int n, int k, double alpha, const psmma_complex* B, int ldb, double 
     void* work = o->work;
     if (work) {
       if (o->lwork < need) return PSMMA_EWORKSPACE;
+      need = o->lwork;
     } else {
+      need = dft_pool_bytes(o->precision, n, k, o->n_moduli);
       work = pool_get(need, s, &st);
       if (st) return st;
     }
@@ -268,11 +270,13 @@ int run_dft(int n, int k, double alpha, const psmma_complex* B, int ldb, double 
     gs.kind = KIND_DFT;
     return launch_struct_f64(2 * n, k, 2 * n, 0.0, nullptr, 2L * ldb, gs, beta, (double*)C, 2L * ldc, s);
   }
-  const size_t need = dft_f64_workspace(n, k);
+  size_t need = dft_f64_workspace(n, k);
   void* work = o->work;
   if (work) {
     if (o->lwork < need) return PSMMA_EWORKSPACE;
+    need = o->lwork;
   } else {
+    need = dft_pool_bytes(o->precision, n, k, o->n_moduli);
     work = pool_get(need, s, &st);
     if (st) return st;
   }
@@ -659,8 +663,10 @@ size_t psmma_workspace_size(int kind, int n, int k, const psmma_opts* opts) {
   if (kind == KIND_CAUCHY_EIG)
     return o->precision == PSMMA_PREC_SPLIT ? split_workspace_general(n, k, k, o->n_moduli, o->block_levels)
                                             : f64_splitk_bytes(n, k, k, std::max(1, device_sms()));
+  if (kind == KIND_DFT)  // room for the dense product and for the transform, whose tables need a little more at small n
+    return std::max(fft_workspace(n, k), o->precision == PSMMA_PREC_SPLIT ? split_workspace_bytes(kind, n, k, o->n_moduli)
+                                                                         : dft_f64_workspace(n, k));
   if (o->precision == PSMMA_PREC_SPLIT) return split_workspace_bytes(kind, n, k, o->n_moduli, o->block_levels);
-  if (kind == KIND_DFT) return dft_f64_workspace(n, k);
   return f64_splitk_bytes(n, k, k, std::max(1, device_sms()));
 }
 

@@ -127,6 +127,15 @@ int launch_dft_table(double2* w, int n, cudaStream_t stream);
 size_t dft_f64_workspace(int n, int k);
 int launch_dft_f64(int n, int k, double alpha, const double* B, long ldb, double beta, double* C, long ldc,
                    void* work, size_t lwork, cudaStream_t stream);
+// The DFT as a fixed-point fast Fourier transform (fft_dft.cu), for either precision: bytes of its
+// workspace (0: n is not covered) and its launches.  ieee: a column that is not finite gives the
+// FP64 sums' infinities and NaN, else NaN throughout (the split precision's rule).
+size_t fft_workspace(int n, int k);
+int launch_fft(int n, int k, double alpha, const double* B, long ldb, double beta, double* C, long ldc, bool ieee,
+               void* work, size_t lwork, cudaStream_t stream);
+// Bytes a DFT call needs from the library's own pool or a server's arena: the transform's where it
+// covers n, else the dense product's.
+size_t dft_pool_bytes(int precision, int n, int k, int n_moduli);
 // The DFT's radix step (split_crt.cu): the radix for size n (1, 2, 4 or 8); B' (n/R x R k
 // complex) = [B(0::R,:) | ... | B(R-1::R,:)]; C(j + (n/R) s, c) = sum_r w_R^(s r) w_n^(j r)
 // P(j, r k + c) + beta C.

@@ -130,7 +130,7 @@ size_t request_workspace(const psmma_request& r) {
   if (r.kind == KIND_CAUCHY_EIG)
     return r.precision == PSMMA_PREC_SPLIT ? split_workspace_general(r.n, r.k, r.k, r.n_moduli) : 0;
   if (r.precision == PSMMA_PREC_SPLIT) return split_workspace_bytes(r.kind, r.n, r.k, r.n_moduli);
-  if (r.kind == KIND_DFT) return dft_f64_workspace(r.n, r.k);
+  if (r.kind == KIND_DFT) return std::max(dft_f64_workspace(r.n, r.k), fft_workspace(r.n, r.k));
   return 0;
 }
 

@@ -250,6 +250,12 @@ extern "C" int psmma_split_dft_radix(int n) { return n > 0 ? dft_radix(n) : 0; }
 
 int dft_radix_for(int n) { return n > 0 ? dft_radix(n) : 1; }
 
+size_t dft_pool_bytes(int precision, int n, int k, int n_moduli) {
+  const size_t fft = fft_workspace(n, k);
+  const size_t dense = precision == PSMMA_PREC_SPLIT ? split_workspace_bytes(KIND_DFT, n, k, n_moduli) : dft_f64_workspace(n, k);
+  return fft && (long)k * dft_radix(n) <= kSplitMaxRows ? fft : dense;
+}
+
 size_t split_workspace_general(int M, int N, int K, int n_moduli, int block_req) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const size_t plain = split_layout(M, K, N, resolve_nmod(n_moduli)).total;
@@ -3551,6 +3557,15 @@ static int split_core_dft3(int k, int n, double alpha, const double* B, long ldb
   const int R = dft_radix(n);
   SplitDevParams* prm = nullptr;
   int st;
+  const bool covered = nmod >= 8 && nmod <= SPL_MAX_MODULI && (long)k * R <= kSplitMaxRows;
+  const size_t fft = covered ? fft_workspace(n, k) : 0;
+  if (fft && work && lwork >= fft) {
+    // the fixed-point transform: no waits on the device, so no status to report
+    st = launch_fft(n, k, alpha, B, ldb, beta, C, ldc, false, work, lwork, stream);
+    if (st || !status_dev_out) return st;
+    if (status_dev_out == kStatusWait) return cudaStreamSynchronize(stream) == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
+    return cudaMemsetAsync(status_dev_out, 0, sizeof(unsigned), stream) == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
+  }
   if (R == 1) {
     st = dft3_enqueue(k, n, alpha, B, ldb, beta, C, ldc, nmod, work, lwork, stream, &prm);
   } else {
