@@ -127,6 +127,21 @@ int launch_dft_table(double2* w, int n, cudaStream_t stream);
 size_t dft_f64_workspace(int n, int k);
 int launch_dft_f64(int n, int k, double alpha, const double* B, long ldb, double beta, double* C, long ldc,
                    void* work, size_t lwork, cudaStream_t stream);
+// Toeplitz / Hankel multiplies of the split precision by number-theoretic transforms (ntt_th.cu): log2
+// of the transform length for order k (0: not covered), the bytes of its buffers, and its launches on
+// the buffers of the single product, which is enqueued behind it gated on *gate.
+struct SplitDevParams;
+int ntt_log(int k);
+size_t ntt_bytes(int n, int k);
+int launch_ntt(bool hankel, int n, int k, double alpha, const double* A, long lda, const double* g, double beta, double* Q,
+               long ldq, double log2M, SplitDevParams* prm, unsigned long long* amax, double* asq,
+               unsigned long long* hmax, double* hsq, void* flag_mem, void* buf, cudaStream_t stream,
+               const unsigned** gate);
+// Passes of split_crt.cu it shares: A's row maxima and squared norms, and the bits PA and PH.
+int launch_row_stats(const double* A, long lda, int M, int K, unsigned long long* amax, double* asq, int sms,
+                     cudaStream_t stream, const unsigned* gate = nullptr);
+int launch_split_params(SplitDevParams* prm, double log2M, int M, int N, int K, const unsigned long long* amax,
+                        const double* asq, const unsigned long long* hmax, const double* hsq, cudaStream_t stream);
 // The DFT as a fixed-point fast Fourier transform (fft_dft.cu), for either precision: bytes of its
 // workspace (0: n is not covered) and its launches.  ieee: a column that is not finite gives the
 // FP64 sums' infinities and NaN, else NaN throughout (the split precision's rule).

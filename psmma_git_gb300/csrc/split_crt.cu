@@ -267,15 +267,22 @@ size_t split_workspace_general(int M, int N, int K, int n_moduli, int block_req)
 // ------------------------------------------------------------------------------------------
 // Pass kernels
 // ------------------------------------------------------------------------------------------
+// A kernel with a gate (here and below) runs only when the gate is NULL or *gate != 0: the single
+// product enqueued behind the transform route of ntt_th.cu, for the generators that route leaves.
+__device__ __forceinline__ bool gated_off(const unsigned* gate) { return gate != nullptr && *gate == 0u; }
+
 __global__ void k_row_absmax(const double* __restrict__ A, long lda, int n, int k, int kchunk,
-                             unsigned long long* __restrict__ amax_bits, double* __restrict__ asq) {
+                             unsigned long long* __restrict__ amax_bits, double* __restrict__ asq,
+                             const unsigned* gate = nullptr) {
+  if (gated_off(gate)) return;
   row_absmax_blk(A, lda, nullptr, 0, k, n, k, kchunk, amax_bits, asq, blockIdx.x, blockIdx.y);
 }
 
 template <int KIND>
 __global__ void k_h_pass1(GenSpec gs, int K, int kp, double* __restrict__ Ht,
                           unsigned long long* __restrict__ hmax_bits, double* __restrict__ hsum,
-                          double* __restrict__ hsq, SplitDevParams* prm) {
+                          double* __restrict__ hsq, SplitDevParams* prm, const unsigned* gate = nullptr) {
+  if (gated_off(gate)) return;
   h_pass1_blk<KIND>(gs, K, kp, Ht, hmax_bits, hsum, hsq, prm, blockIdx.x);
 }
 
@@ -301,64 +308,81 @@ __global__ void k_h_pass1_all(GenSpec gs, int K, int kp, double* __restrict__ Ht
 // errors, ~2^-PA * c_A and ~2^-PH * c_H with c_A ~ rms_i(max|A_i:|)/rms(A),
 // c_H ~ rms_j(max|H_:j|)/rms(H) (same constant factor): PH - PA = round(log2(c_H/c_A)).
 // Partial maxima of the row / column ratios ||.||_2 / max|.| and sums of max^2 and ||.||_2^2
-// over rows [i0, i1) of A and columns [j0, j1) of H; the block's totals land in thread 0's v.
-__device__ __forceinline__ void params_partial(int i0, int i1, int j0, int j1, double rk,
+// over rows [i0, i1) of A and columns [j0, j1) of H; the block's totals land in thread 0's v.  The
+// squared ratios are taken in FP32, rounded up, on the operands' mantissas (an FP64 square root and
+// division a row are some 80 instructions on the two-lane FP64 pipe: the pass took 34 us at any size).
+__device__ __forceinline__ float ratio2_up(unsigned long long mb, unsigned long long qb) {
+  const float m = __uint_as_float(0x3F800000u | ((unsigned)(mb >> 29) & 0x7FFFFFu));          // below
+  const float q = __uint_as_float((0x3F800000u | ((unsigned)(qb >> 29) & 0x7FFFFFu)) + 1u);    // above
+  const int e = (int)(qb >> 52) - 1023 - 2 * ((int)(mb >> 52) - 1023);  // -1 .. 2 + log2 k
+  return __fdiv_ru(q, __fmul_rd(m, m)) * __uint_as_float((unsigned)(127 + max(-2, min(e, 60))) << 23);
+}
+__device__ __forceinline__ void params_partial(int i0, int i1, int j0, int j1, float rk,
                                                const unsigned long long* __restrict__ amax_bits,
                                                const double* __restrict__ asq,
                                                const unsigned long long* __restrict__ hmax_bits,
                                                const double* __restrict__ hsq, double v[6]) {
-  double ra = 0.0, amx2 = 0.0, afro = 0.0, rh = 0.0, hmx2 = 0.0, hfro = 0.0;
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-    const unsigned long long b = amax_bits[i];
-    if (b == 0 || b >= INF_BITS) continue;
-    const double m = __longlong_as_double((long long)b), q = asq[i];
-    const bool safe = m > 1e-140 && m < 1e140 && isfinite(q) && q > 0.0;
-    ra = fmax(ra, safe ? sqrt(q) / m : rk);
-    if (safe) { amx2 += m * m; afro += q; }
-  }
-  for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-    const unsigned long long b = hmax_bits[j];
-    if (b == 0 || b >= INF_BITS) continue;
-    const double m = __longlong_as_double((long long)b), q = hsq[j];
-    const bool safe = m > 1e-140 && m < 1e140 && isfinite(q) && q > 0.0;
-    rh = fmax(rh, safe ? sqrt(q) / m : rk);
-    if (safe) { hmx2 += m * m; hfro += q; }
-  }
-  v[0] = ra; v[1] = amx2; v[2] = afro; v[3] = rh; v[4] = hmx2; v[5] = hfro;
-  // block reduction: max for ra/rh, sums otherwise
-  for (int o = 16; o > 0; o >>= 1)
-    for (int t = 0; t < 6; ++t) {
-      double w = __shfl_xor_sync(0xffffffffu, v[t], o);
-      v[t] = (t == 0 || t == 3) ? fmax(v[t], w) : v[t] + w;
+  float mx[2] = {0.0f, 0.0f};                // largest squared ratios of the rows, the columns
+  double sm[4] = {0.0, 0.0, 0.0, 0.0};       // sums of max^2 and ||.||_2^2 of the rows, the columns
+  auto add = [&](int t, unsigned long long b, double q) {
+    if (b == 0 || b >= INF_BITS) return;
+    const unsigned long long qb = (unsigned long long)__double_as_longlong(q);
+    const int e = (int)(b >> 52) - 1023;
+    const bool safe = e > -465 && e < 465 && qb != 0 && qb < INF_BITS;
+    mx[t] = fmaxf(mx[t], safe ? ratio2_up(b, qb) : rk);
+    if (safe) {
+      const double m = __longlong_as_double((long long)b);
+      sm[2 * t] = fma(m, m, sm[2 * t]);
+      sm[2 * t + 1] += q;
     }
-  __shared__ double sv[6][32];
-  const int wid = threadIdx.x >> 5, ln = threadIdx.x & 31;
-  if (ln == 0)
-    for (int t = 0; t < 6; ++t) sv[t][wid] = v[t];
+  };
+  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) add(0, amax_bits[i], asq[i]);
+  for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) add(1, hmax_bits[j], hsq[j]);
+  auto reduce = [&]() {
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t) mx[t] = fmaxf(mx[t], __shfl_xor_sync(0xffffffffu, mx[t], o));
+#pragma unroll
+      for (int t = 0; t < 4; ++t) sm[t] += __shfl_xor_sync(0xffffffffu, sm[t], o);
+    }
+  };
+  reduce();
+  __shared__ float smx[2][32];
+  __shared__ double ssm[4][32];
+  const int wid = threadIdx.x >> 5, ln = threadIdx.x & 31, nw = blockDim.x >> 5;
+  if (ln == 0) {
+    for (int t = 0; t < 2; ++t) smx[t][wid] = mx[t];
+    for (int t = 0; t < 4; ++t) ssm[t][wid] = sm[t];
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = blockDim.x >> 5;
-    for (int t = 0; t < 6; ++t) {
-      double acc = sv[t][0];
-      for (int w = 1; w < nw; ++w) acc = (t == 0 || t == 3) ? fmax(acc, sv[t][w]) : acc + sv[t][w];
-      v[t] = acc;
-    }
+  if (wid == 0) {
+    for (int t = 0; t < 2; ++t) mx[t] = ln < nw ? smx[t][ln] : 0.0f;
+    for (int t = 0; t < 4; ++t) sm[t] = ln < nw ? ssm[t][ln] : 0.0;
+    reduce();
   }
+  v[0] = mx[0]; v[1] = sm[0]; v[2] = sm[1]; v[3] = mx[1]; v[4] = sm[2]; v[5] = sm[3];
 }
 
-// PA and PH from the totals (thread 0).
+// log2 of a positive normal double, to 1e-5 (FP32 on the mantissa).
+__device__ __forceinline__ float log2_fast(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return (float)((int)(b >> 52) - 1023) + log2f(__uint_as_float(0x3F800000u | ((unsigned)(b >> 29) & 0x7FFFFFu)));
+}
+
+// PA and PH from the totals (thread 0): v[0], v[3] the largest squared ratios, the others sums.  The
+// logarithms are FP32, their error (below 1e-4) well inside the factors 1.01.
 __device__ __forceinline__ void params_finish(SplitDevParams* prm, double log2M, int k, const double v[6]) {
-  const double rk = sqrt((double)k);
-  double rho = __longlong_as_double((long long)prm->rho_bits);
-  if (!(rho >= 1.0)) rho = rk * rk;
-  const double l1 = log2(rho * 1.01 + (double)k / 512.0);
-  const double cs = log2((v[0] * 1.01 + rk / 512.0) * (v[3] * 1.01 + rk / 512.0));
-  const double bound = fmin(l1, (v[0] > 0.0 && v[3] > 0.0) ? cs : l1);
-  int budget = (int)floor(log2M - 1.01 - bound);
+  const float rk = sqrtf((float)k);
+  const double rho_d = __longlong_as_double((long long)prm->rho_bits);
+  const float rho = rho_d >= 1.0 && rho_d < 1e30 ? __double2float_ru(rho_d) : rk * rk;
+  const float l1 = log2f(rho * 1.01f + (float)k / 512.0f);
+  const float cs = log2f((sqrtf((float)v[0]) * 1.01f + rk / 512.0f) * (sqrtf((float)v[3]) * 1.01f + rk / 512.0f));
+  const float bound = fminf(l1, (v[0] > 0.0 && v[3] > 0.0) ? cs : l1);
+  int budget = (int)floorf((float)(log2M - 1.01) - bound);
   int d = 0;
   if (v[1] > 0.0 && v[2] > 0.0 && v[4] > 0.0 && v[5] > 0.0) {
-    const double cA = sqrt(v[1] / v[2]), cH = sqrt(v[4] / v[5]);
-    d = (int)lrint(log2(cH / cA));
+    // log2(c_H / c_A), c = sqrt(sum max^2 / sum ||.||^2)
+    d = (int)lrintf(0.5f * ((log2_fast(v[4]) - log2_fast(v[5])) - (log2_fast(v[1]) - log2_fast(v[2]))));
     d = max(-12, min(12, d));
   }
   int PA = (budget - d) >> 1, PH = budget - PA;
@@ -375,62 +399,48 @@ __device__ __forceinline__ void split_params_blk(SplitDevParams* prm, double log
                                                  const unsigned long long* __restrict__ hmax_bits,
                                                  const double* __restrict__ hsq) {
   double v[6];
-  params_partial(0, n, 0, ncols, sqrt((double)k), amax_bits, asq, hmax_bits, hsq, v);
+  params_partial(0, n, 0, ncols, (float)k, amax_bits, asq, hmax_bits, hsq, v);
   if (threadIdx.x == 0) params_finish(prm, log2M, k, v);
 }
 
-// PARAMS_BLOCKS blocks, each over a slice of the rows and columns (the square roots and
-// divisions are FP64); the last block to finish combines the partials in block order, so the
-// result does not depend on the finishing order.
+// One to PARAMS_BLOCKS blocks, each over a slice of the rows and columns; the last block to finish
+// combines the partials in a fixed order, so the result does not depend on the finishing order.
 __global__ void k_split_params(SplitDevParams* prm, double log2M, int n, int ncols, int k,
                                const unsigned long long* __restrict__ amax_bits, const double* __restrict__ asq,
-                               const unsigned long long* __restrict__ hmax_bits, const double* __restrict__ hsq) {
+                               const unsigned long long* __restrict__ hmax_bits, const double* __restrict__ hsq,
+                               const unsigned* gate = nullptr) {
+  if (gated_off(gate)) return;
   const int G = gridDim.x, b = blockIdx.x;
   const int i0 = (int)((long)n * b / G), i1 = (int)((long)n * (b + 1) / G);
   const int j0 = (int)((long)ncols * b / G), j1 = (int)((long)ncols * (b + 1) / G);
   double v[6];
-  params_partial(i0, i1, j0, j1, sqrt((double)k), amax_bits, asq, hmax_bits, hsq, v);
+  params_partial(i0, i1, j0, j1, (float)k, amax_bits, asq, hmax_bits, hsq, v);
+  if (G == 1) {
+    if (threadIdx.x == 0) params_finish(prm, log2M, k, v);
+    return;
+  }
+  __shared__ int last;
   if (threadIdx.x == 0) {
     for (int t = 0; t < 6; ++t) prm->part[b][t] = v[t];
     __threadfence();
-    if (atomicAdd(&prm->done, 1u) == (unsigned)G - 1) {
-      __threadfence();
-      double tot[6];
-      for (int t = 0; t < 6; ++t) tot[t] = __ldcg(&prm->part[0][t]);
-      for (int q = 1; q < G; ++q)
-        for (int t = 0; t < 6; ++t) {
-          const double x = __ldcg(&prm->part[q][t]);
-          tot[t] = (t == 0 || t == 3) ? fmax(tot[t], x) : tot[t] + x;
-        }
-      params_finish(prm, log2M, k, tot);
-    }
+    last = atomicAdd(&prm->done, 1u) == (unsigned)G - 1;
+  }
+  __syncthreads();
+  if (last && threadIdx.x < 32) {  // one lane a block, combined in a fixed tree
+    __threadfence();
+    double tot[6];
+    for (int t = 0; t < 6; ++t) tot[t] = (int)threadIdx.x < G ? __ldcg(&prm->part[threadIdx.x][t]) : 0.0;
+    for (int o = 16; o > 0; o >>= 1)
+      for (int t = 0; t < 6; ++t) {
+        const double x = __shfl_xor_sync(0xffffffffu, tot[t], o);
+        tot[t] = (t == 0 || t == 3) ? fmax(tot[t], x) : tot[t] + x;
+      }
+    if (threadIdx.x == 0) params_finish(prm, log2M, k, tot);
   }
 }
 
-// Exponent s such that |x * 2^s| < 2^P for all |x| <= amax (amax finite, > 0).
-__device__ __forceinline__ int scale_exp(unsigned long long amax_bits, int P) {
-  return P - 1 - ilogb_bits(amax_bits);
-}
-
-// rint(x * 2^e) (round half to even) for finite x with |x * 2^e| < 2^53, computed from the
-// bits of x with integer operations only; *neg receives the sign.
-__device__ __forceinline__ unsigned long long scaled_int(double x, int e, bool* neg) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  *neg = (b >> 63) != 0;
-  const int ex = (int)((b >> 52) & 0x7FF);
-  unsigned long long m = b & 0xFFFFFFFFFFFFFull;
-  int E = -1074;
-  if (ex != 0) {
-    m |= 1ull << 52;
-    E = ex - 1075;
-  }
-  const int sh = E + e;
-  if (sh >= 0) return m << sh;  // the caller's bound keeps the result below 2^53
-  const int k = -sh;
-  if (k > 63) return 0;  // below one half
-  // round half to even: m / 2^k + 1/2 - 2^-k, plus 2^-k when the last kept bit is odd
-  return (m + ((1ull << (k - 1)) - 1) + ((m >> k) & 1)) >> k;
-}
+// Blocks of the parameter pass: one per 2048 rows and columns.
+static int params_blocks(int M, int N) { return std::max(1, std::min(PARAMS_BLOCKS, (M + N + 2047) / 2048)); }
 
 // Residues of neighbouring integers for every modulus, on the FP32 pipe.  A scaled integer
 // x < 2^53 with sign s is cut into x0 = x mod 2^23, x1 = (x >> 23) mod 2^15 and x2 = x >> 38
@@ -572,7 +582,8 @@ __device__ __forceinline__ void residues_A_blk(const double* __restrict__ A, lon
 
 __global__ void k_residues_A(const double* __restrict__ A, long lda, int n, int k, int kp,
                              const unsigned long long* __restrict__ amax_bits, const SplitDevParams* prm,
-                             CrtConsts cc, __nv_bfloat16* __restrict__ RA) {
+                             CrtConsts cc, __nv_bfloat16* __restrict__ RA, const unsigned* gate = nullptr) {
+  if (gated_off(gate)) return;
   residues_A_blk<64>(A, lda, nullptr, 0, k, n, k, kp, amax_bits, prm, cc, RA, blockIdx.x, blockIdx.y);
 }
 
@@ -618,8 +629,11 @@ __device__ __forceinline__ void residues_H_blk(const double* __restrict__ Ht, in
 
 __global__ void k_residues_H(const double* __restrict__ Ht, int ncols, int kp,
                              const unsigned long long* __restrict__ hmax_bits, const SplitDevParams* prm,
-                             CrtConsts cc, __nv_bfloat16* __restrict__ RH) {
-  residues_H_blk(Ht, ncols, kp, hmax_bits, prm, cc, RH, blockIdx.y, blockIdx.x);  // x: column (any count)
+                             CrtConsts cc, __nv_bfloat16* __restrict__ RH, const unsigned* gate = nullptr) {
+  if (gated_off(gate)) return;
+  // x: column (any count; a gated launch, which mostly returns at once, has fewer blocks than columns)
+  for (int j = blockIdx.x; j < ncols; j += gridDim.x)
+    residues_H_blk(Ht, ncols, kp, hmax_bits, prm, cc, RH, blockIdx.y, j);
 }
 
 // Speculative H residues: with guess >= 0 and !redo, the planes for PH = guess (before the
@@ -1772,50 +1786,6 @@ __global__ void __launch_bounds__((TS::kEpiWarps + 2) * 32, 1) k_crt_gemm(const 
 // ------------------------------------------------------------------------------------------
 typedef unsigned __int128 u128;
 
-// m * 2^x with the sign, for results outside the normal range; out of line, so that its FP64
-// instructions are not issued (predicated off) for every element.
-static __device__ __noinline__ double scaled_outside_normal(unsigned long long m, int x, bool neg) {
-  const double v = ldexp((double)m, x);
-  return neg ? -v : v;
-}
-
-// (hi:lo) * 2^-e as a double, (hi:lo) a non-negative 128-bit integer in two words, rounded
-// to nearest even from the bits; results outside the normal range go through ldexp.
-__device__ __forceinline__ double u128w_scaled(unsigned long long hi, unsigned long long lo, bool neg, int e) {
-  if ((hi | lo) == 0) return 0.0;
-  // normalise so that the leading bit is bit 63 of `top`; `rest` keeps the bits below
-  int p;
-  unsigned long long top, rest;
-  if (hi) {
-    const int s = __clzll((long long)hi);
-    p = 127 - s;
-    top = s ? (hi << s) | (lo >> (64 - s)) : hi;
-    rest = s ? (lo << s) : lo;
-  } else {
-    const int s = __clzll((long long)lo);
-    p = 63 - s;
-    top = lo << s;
-    rest = 0;
-  }
-  unsigned long long m = top >> 11;  // 53 bits
-  const unsigned long long low11 = top & 0x7FFull;
-  const bool sticky = (low11 & 0x3FFull) != 0 || rest != 0;
-  if ((low11 & 0x400ull) && (sticky || (m & 1))) {
-    ++m;
-    if (m == (1ull << 53)) {
-      m >>= 1;
-      ++p;
-    }
-  }
-  const int field = p - e + 1023;
-  if (field >= 1 && field <= 2046) {
-    unsigned long long bits = ((unsigned long long)field << 52) | (m & 0xFFFFFFFFFFFFFull);
-    if (neg) bits |= 1ull << 63;
-    return __longlong_as_double((long long)bits);
-  }
-  return scaled_outside_normal(m, p - 52 - e, neg);
-}
-
 // One block: 32 rows x 128 columns (32 x 8 threads); a thread recombines 4 neighbouring
 // columns of one row per pass from 32-bit loads (4 residues) of each plane, so each warp
 // request moves 128 bytes.  Per modulus and element: four 32x32->64-bit multiply-adds for
@@ -1991,7 +1961,9 @@ __global__ void __launch_bounds__(256, 3) k_crt_combine(const int8_t* __restrict
                                                      CrtConsts cc, const unsigned long long* __restrict__ amax_bits,
                                                      const unsigned long long* __restrict__ hmax_bits,
                                                      const SplitDevParams* prm, double alpha, double beta,
-                                                     double* __restrict__ Q, long ldq, int by0) {
+                                                     double* __restrict__ Q, long ldq, int by0,
+                                                     const unsigned* gate = nullptr) {
+  if (gated_off(gate)) return;
   crt_combine_blk<DFT_OUT, TOP32>(R, n, k, kr, cc, amax_bits, hmax_bits, prm, alpha, beta, Q, ldq, blockIdx.x,
                                   by0 + blockIdx.y);
 }
@@ -2320,9 +2292,25 @@ static int split_status(SplitDevParams* prm, cudaStream_t stream, unsigned* stat
 
 // Core of the split path: Q (M x N) = alpha * A (M x K, column-major, lda) * H (K x N) + beta * Q
 // (column-major, ldq), H generated from gs (any kind but the DFT: split_core_dft3).
+// Row maxima and norms of A (cleared before): chunks of columns short enough for some eight waves of
+// blocks (a chunk is a chain of loads, eight in flight a thread: 1000 x 777 in one chunk 55 us).
+int launch_row_stats(const double* A, long lda, int M, int K, unsigned long long* amax, double* asq, int sms,
+                     cudaStream_t stream, const unsigned* gate) {
+  int kchunk = 1024;
+  while (kchunk > 32 && (long)((M + 127) / 128) * ((K + kchunk - 1) / kchunk) < 8L * sms) kchunk >>= 1;
+  k_row_absmax<<<dim3((M + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, stream>>>(A, lda, M, K, kchunk, amax, asq, gate);
+  return cudaGetLastError() == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
+}
+
+int launch_split_params(SplitDevParams* prm, double log2M, int M, int N, int K, const unsigned long long* amax,
+                        const double* asq, const unsigned long long* hmax, const double* hsq, cudaStream_t stream) {
+  k_split_params<<<params_blocks(M, N), 512, 0, stream>>>(prm, log2M, M, N, K, amax, asq, hmax, hsq);
+  return cudaGetLastError() == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
+}
+
 static int split_core(int M, int N, int K, double alpha, const double* A, long lda, const GenSpec& gs, double beta,
                       double* Q, long ldq, int nmod, void* work, size_t lwork, cudaStream_t stream,
-                      unsigned* status_dev_out) {
+                      unsigned* status_dev_out, const unsigned* gate = nullptr) {
   if (gs.kind == KIND_DFT) return PSMMA_EUNSUPPORTED;  // split_core_dft3
   if (nmod < 8 || nmod > SPL_MAX_MODULI) return PSMMA_EUNSUPPORTED;
   if (K >= (1 << 24) || M > kSplitMaxRows || N >= (1 << 30)) return PSMMA_EUNSUPPORTED;
@@ -2332,31 +2320,32 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
   const SplitBuffers b = split_buffers(w, L);
   const CrtConsts cc = get_consts(nmod);
 
-  prof_begin(stream);
+  if (!gate) prof_begin(stream);
   if (cudaMemsetAsync(w, 0, L.off_wtab, stream) != cudaSuccess) return PSMMA_EDEVICE;  // params, maxima, sums
 
   // ---- A side: row maxima and norms
-  {
-    const int kchunk = 1024;
-    dim3 g1((M + 127) / 128, (K + kchunk - 1) / kchunk);
-    k_row_absmax<<<g1, 128, 0, stream>>>(A, lda, M, K, kchunk, b.amax, b.asq);
-  }
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return PSMMA_EDEVICE;
+  int rst = launch_row_stats(A, lda, M, K, b.amax, b.asq, sms, stream, gate);
+  if (rst) return rst;
   prof_mark(stream, "row_scale");
   // ---- H side: generate, column maxima / sums / norms
   switch (gs.kind) {
-    case KIND_CAUCHY: k_h_pass1<KIND_CAUCHY><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm); break;
-    case KIND_TOEPLITZ: k_h_pass1<KIND_TOEPLITZ><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm); break;
-    case KIND_HANKEL: k_h_pass1<KIND_HANKEL><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm); break;
-    case KIND_DENSE: k_h_pass1<KIND_DENSE><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm); break;
-    case KIND_CAUCHY_EIG: k_h_pass1<KIND_CAUCHY_EIG><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm); break;
+    case KIND_CAUCHY: k_h_pass1<KIND_CAUCHY><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
+    case KIND_TOEPLITZ: k_h_pass1<KIND_TOEPLITZ><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
+    case KIND_HANKEL: k_h_pass1<KIND_HANKEL><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
+    case KIND_DENSE: k_h_pass1<KIND_DENSE><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
+    case KIND_CAUCHY_EIG: k_h_pass1<KIND_CAUCHY_EIG><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
     default: return PSMMA_EUNSUPPORTED;
   }
   prof_mark(stream, "h_generate");
-  k_split_params<<<PARAMS_BLOCKS, 512, 0, stream>>>(b.prm, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsq);
+  k_split_params<<<params_blocks(M, N), 512, 0, stream>>>(b.prm, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsq, gate);
   prof_mark(stream, "params");
-  k_residues_A<<<dim3(L.kp / 64, (M + 63) / 64), 256, 0, stream>>>(A, lda, M, K, L.kp, b.amax, b.prm, cc, b.RA);
+  k_residues_A<<<dim3(L.kp / 64, (M + 63) / 64), 256, 0, stream>>>(A, lda, M, K, L.kp, b.amax, b.prm, cc, b.RA, gate);
   prof_mark(stream, "residues_A");
-  k_residues_H<<<dim3(N, rh_blocks_x(L.kp)), 128, 0, stream>>>(b.Ht, N, L.kp, b.hmax, b.prm, cc, b.RH);
+  k_residues_H<<<dim3(gate ? std::min(N, 512) : N, rh_blocks_x(L.kp)), 128, 0, stream>>>(b.Ht, N, L.kp, b.hmax, b.prm, cc,
+                                                                                      b.RH, gate);
   prof_mark(stream, "residues_H");
 
   OneGemm og;
@@ -2376,17 +2365,16 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
   using Shape = GemmShape<G_BN>;
   if (set_smem_attr(k_crt_gemm<G_BN, OneGemm>, (int)Shape::SMEM) != cudaSuccess)
     return PSMMA_EDEVICE;
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return PSMMA_EDEVICE;
   ga.nmod = nmod;
+  ga.gate = gate;
+  ga.gate_set = 1;
   const int total_tiles = ga.tiles_m * ga.tiles_n * nmod;
   k_crt_gemm<G_BN, OneGemm><<<std::min(sms, total_tiles), G_THREADS, Shape::SMEM, stream>>>(og);
   prof_mark(stream, "modular_gemm");
 
   dim3 gc((N + CRT_TJ - 1) / CRT_TJ, (M + CRT_TI - 1) / CRT_TI);
   (cc.top32 ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, stream>>>(
-      b.R, M, N, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq, 0);
+      b.R, M, N, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq, 0, gate);
   prof_mark(stream, "crt_combine");
   if (cudaGetLastError() != cudaSuccess) return PSMMA_EDEVICE;
 
@@ -2797,7 +2785,7 @@ static int split_core_block(int M, int N, int Np, int L, double alpha, const dou
   prof_mark(stream, "row_scale");
   br.h_side(nullptr, stream);
   prof_mark(stream, "h_generate");
-  k_split_params<<<PARAMS_BLOCKS, 512, 0, stream>>>(b.prm, br.cc.log2M, M, Np, Np, b.amax, b.asq, b.hmax, b.hsq);
+  k_split_params<<<params_blocks(M, Np), 512, 0, stream>>>(b.prm, br.cc.log2M, M, Np, Np, b.amax, b.asq, b.hmax, b.hsq);
   prof_mark(stream, "params");
   br.a_residues(A, lda, 0, M, b.prm, stream);
   prof_mark(stream, "residues_A");
@@ -2992,7 +2980,7 @@ static int split_core_s2(int M, int N, int K, double alpha, const double* A, lon
     default: return PSMMA_EUNSUPPORTED;
   }
   prof_mark(stream, "h_generate");
-  k_split_params<<<PARAMS_BLOCKS, 512, 0, stream>>>(b.prm, st.cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsq);
+  k_split_params<<<params_blocks(M, N), 512, 0, stream>>>(b.prm, st.cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsq);
   prof_mark(stream, "params");
   s2_h_operands(st, b.Ht, b.hmax, b.prm, stream);
   prof_mark(stream, "residues_H");
@@ -3000,7 +2988,7 @@ static int split_core_s2(int M, int N, int K, double alpha, const double* A, lon
   if (rc != PSMMA_OK) return rc;
   dim3 gc((N + CRT_TJ - 1) / CRT_TJ, (M + CRT_TI - 1) / CRT_TI);
   (st.cc.top32 ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, stream>>>(
-      b.R, M, N, Lo.kr, st.cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq, 0);
+      b.R, M, N, Lo.kr, st.cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq, 0, nullptr);
   prof_mark(stream, "crt_combine");
   if (cudaGetLastError() != cudaSuccess) return PSMMA_EDEVICE;
   return split_status(b.prm, stream, status_dev_out);
@@ -3117,7 +3105,7 @@ static int split_core_host(int M, int N, int K, double alpha, const double* A_h,
     const int r0 = t0 * G_BM, r1 = std::min(M, t1 * G_BM);
     dim3 gc((N + CRT_TJ - 1) / CRT_TJ, (r1 - r0 + CRT_TI - 1) / CRT_TI);
     (cc.top32 ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, s>>>(
-        b.R, M, N, L.kr, cc, b.amax, b.hmax, pk, alpha, beta, dQ, M, r0 / CRT_TI);
+        b.R, M, N, L.kr, cc, b.amax, b.hmax, pk, alpha, beta, dQ, M, r0 / CRT_TI, nullptr);
     prof_mark(s, "panel_gemm_crt");
     ok &= cudaEventRecord(ev_panel[p], s) == cudaSuccess;
     ok &= cudaStreamWaitEvent(cs, ev_panel[p], 0) == cudaSuccess;
@@ -3167,7 +3155,7 @@ static int split_core_host(int M, int N, int K, double alpha, const double* A_h,
       prof_mark(s, "panel_rows");
       panel(p, b.prm_guess);
     }
-    k_split_params<<<PARAMS_BLOCKS, 512, 0, s>>>(b.prm, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsq);
+    k_split_params<<<params_blocks(M, N), 512, 0, s>>>(b.prm, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsq);
     finish();
     if (!ok) return PSMMA_EDEVICE;
     if (head.status & DEV_ERR_TIMEOUT) return PSMMA_ETIMEDOUT;
@@ -3206,7 +3194,7 @@ static int split_core_host(int M, int N, int K, double alpha, const double* A_h,
   }
   if (!ok) return PSMMA_EDEVICE;
   prof_mark(s, "a_upload_rows");
-  k_split_params<<<PARAMS_BLOCKS, 512, 0, s>>>(b.prm, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsq);
+  k_split_params<<<params_blocks(M, N), 512, 0, s>>>(b.prm, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsq);
   k_residues_A<<<dim3(L.kp / 64, (M + 63) / 64), 256, 0, s>>>(dA, M, M, K, L.kp, b.amax, b.prm, cc, b.RA);
   if (ph_guess >= 8)
     k_residues_H_spec<<<grh, 128, 0, s>>>(b.Ht, N, L.kp, b.hmax, b.prm, cc, b.RH, ph_guess, 1);
@@ -3314,7 +3302,7 @@ static int split_core_host_block(int M, int N, int Np, int L, double alpha, cons
       prof_mark(s, "panel_rows");
       panel(p, b.prm_guess);
     }
-    k_split_params<<<PARAMS_BLOCKS, 512, 0, s>>>(b.prm, br.cc.log2M, M, Np, Np, b.amax, b.asq, b.hmax, b.hsq);
+    k_split_params<<<params_blocks(M, Np), 512, 0, s>>>(b.prm, br.cc.log2M, M, Np, Np, b.amax, b.asq, b.hmax, b.hsq);
     finish();
     if (!ok) return PSMMA_EDEVICE;
     if (head.status & DEV_ERR_TIMEOUT) return PSMMA_ETIMEDOUT;
@@ -3353,7 +3341,7 @@ static int split_core_host_block(int M, int N, int Np, int L, double alpha, cons
   }
   if (!ok) return PSMMA_EDEVICE;
   prof_mark(s, "a_upload_rows");
-  k_split_params<<<PARAMS_BLOCKS, 512, 0, s>>>(b.prm, br.cc.log2M, M, Np, Np, b.amax, b.asq, b.hmax, b.hsq);
+  k_split_params<<<params_blocks(M, Np), 512, 0, s>>>(b.prm, br.cc.log2M, M, Np, Np, b.amax, b.asq, b.hmax, b.hsq);
   br.a_residues(dA, M, 0, M, b.prm, s);
   br.h_operands(b.prm, s);
   prof_mark(s, "params_residues");
@@ -3455,7 +3443,7 @@ static int dft3_enqueue(int M, int nn, double alpha, const double* B, long ldb, 
   k_h_pass1_dft3<<<nn, 256, 0, stream>>>(b.wtab, nn, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm);
   prof_mark(stream, "h_generate");
   // the bounds are those of the real embedding: n columns, inner dimension 2n
-  k_split_params<<<PARAMS_BLOCKS, 512, 0, stream>>>(b.prm, cc.log2M, M, nn, 2 * nn, b.amax, b.asq, b.hmax, b.hsq);
+  k_split_params<<<params_blocks(M, nn), 512, 0, stream>>>(b.prm, cc.log2M, M, nn, 2 * nn, b.amax, b.asq, b.hmax, b.hsq);
   prof_mark(stream, "params");
   k_residues_A_dft3<<<dim3(M, (L.kp / 2 + 127) / 128), 128, 0, stream>>>(B, 2 * ldb, nn, L.kp, b.amax, b.prm, cc,
                                                                          b.RA, M);
@@ -3539,7 +3527,7 @@ static int dft3_enqueue(int M, int nn, double alpha, const double* B, long ldb, 
   } else {
     dim3 gc(L.kr / CRT_TJ, (M + CRT_TI - 1) / CRT_TI);
     (cc.top32 ? k_crt_combine<true, true> : k_crt_combine<true, false>)<<<gc, dim3(32, 8), 0, stream>>>(
-        b.R, M, nn, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, C, 2 * ldc, 0);
+        b.R, M, nn, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, C, 2 * ldc, 0, nullptr);
     prof_mark(stream, "crt_combine");
   }
   if (cudaGetLastError() != cudaSuccess) return PSMMA_EDEVICE;
@@ -3587,6 +3575,24 @@ static int split_core_dft3(int k, int n, double alpha, const double* B, long ldb
   return split_status(prm, stream, status_dev_out);
 }
 
+// Whether the transforms of ntt_th.cu are the faster route for a Toeplitz / Hankel multiply: the sum of
+// the terms in which the two differ, in microseconds.  Transforms: 2 lg levels of L points per row and
+// prime at 2.16e-7 us (8192 x 8192: 3.25 ms), 1.3 times that at L = 2^15 (tables past L1), and 60 us of
+// launches.  GEMMs: 2 k^2 flops per row and modulus at 1.5e9 a microsecond, three quarters of them per level of
+// the block step, and H's generation and residues, 1.1e-5 us an entry.  Measured (transforms / GEMMs):
+// n = k = 2048 0.35 / 0.37 ms, 3003 0.87 / 0.85, 4096 1.24 / 1.62, 8192 4.3 / 8.7, 16384 19.6 / 51.
+// More than 15 moduli leave the primes no bits for unequal columns.
+static bool ntt_route(int kind, int n, int k, int nmod) {
+  const int lg = ntt_log(k);
+  if (!lg || nmod > 15) return false;
+  const int np = nmod <= 14 ? 4 : 5;
+  const double L = (double)(1 << lg), kk = (double)k * k;
+  const double ntt = 2.16e-7 * n * L * 2 * lg * np * (lg >= 15 ? 1.3 : 1.0) + 60.0;
+  double gemm = (double)n * nmod * 2.0 * kk / 1.5e9;
+  for (int l = block_choice(kind, k, k, 0).L; l > 0; --l) gemm *= 0.75;
+  return ntt < gemm + 1.1e-5 * kk;
+}
+
 // kind == DFT: C (n x k complex, ldq) = alpha * F (n x n) * B (n x k complex, lda) + beta * C,
 //   computed as C^T = B^T F in the 3M form (split_core_dft3).
 int launch_split_any(int kind, int n, int k, double alpha, const double* A, long lda, const double* gen,
@@ -3595,6 +3601,20 @@ int launch_split_any(int kind, int n, int k, double alpha, const double* A, long
   const int nmod = resolve_nmod(n_moduli);
   if (kind == KIND_DFT) return split_core_dft3(k, n, alpha, A, lda, beta, Q, ldq, nmod, work, lwork, stream, status_dev_out);
   const GenSpec gs = reference_gens(kind, gen, ldgen, k);
+  if ((kind == KIND_TOEPLITZ || kind == KIND_HANKEL) && block_req == 0 && ntt_route(kind, n, k, nmod)) {
+    const SplitLayout L = split_layout(n, k, k, nmod);
+    if (work && lwork >= L.total && L.total - L.off_ra >= ntt_bytes(n, k)) {
+      char* w = (char*)work;
+      const SplitBuffers b = split_buffers(w, L);
+      const CrtConsts cc = get_consts(nmod);
+      if (cudaMemsetAsync(w, 0, L.off_wtab, stream) != cudaSuccess) return PSMMA_EDEVICE;
+      const unsigned* gate = nullptr;
+      const int st = launch_ntt(kind == KIND_HANKEL, n, k, alpha, A, lda, gen, beta, Q, ldq, cc.log2M, b.prm, b.amax, b.asq,
+                                b.hmax, b.hsq, w + L.off_wtab, w + L.off_ra, stream, &gate);
+      if (st) return st;
+      return split_core(n, k, k, alpha, A, lda, gs, beta, Q, ldq, nmod, work, lwork, stream, status_dev_out, gate);
+    }
+  }
   const BlockChoice bc = block_choice(kind, k, k, block_req);
   if (bc.L > 0 && gs.k1 == 0)
     return split_core_block(n, k, bc.Np, bc.L, alpha, A, lda, gs, beta, Q, ldq, nmod, work, lwork, stream,

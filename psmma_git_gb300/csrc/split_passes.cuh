@@ -1,5 +1,5 @@
-// Device passes shared by the modular paths (split_crt.cu, exact_crt.cu): the statistics of A's
-// rows and the generation of H with its column statistics.
+// Device passes shared by the modular paths (split_crt.cu, exact_crt.cu, ntt_th.cu): the statistics of A's
+// rows, the generation of H with its column statistics, the integer scaling and the rounding back.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -128,6 +128,75 @@ __device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, lon
 __device__ __forceinline__ int ilogb_bits(unsigned long long b) {
   const int ex = (int)(b >> 52);
   return ex ? ex - 1023 : 63 - __clzll((long long)b) - 1074;  // subnormal: b is the mantissa
+}
+
+// Exponent s such that |x * 2^s| < 2^P for all |x| <= amax (amax finite, > 0).
+__device__ __forceinline__ int scale_exp(unsigned long long amax_bits, int P) {
+  return P - 1 - ilogb_bits(amax_bits);
+}
+
+// rint(x * 2^e) (round half to even) for finite x with |x * 2^e| < 2^53, computed from the
+// bits of x with integer operations only; *neg receives the sign.
+__device__ __forceinline__ unsigned long long scaled_int(double x, int e, bool* neg) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  *neg = (b >> 63) != 0;
+  const int ex = (int)((b >> 52) & 0x7FF);
+  unsigned long long m = b & 0xFFFFFFFFFFFFFull;
+  int E = -1074;
+  if (ex != 0) {
+    m |= 1ull << 52;
+    E = ex - 1075;
+  }
+  const int sh = E + e;
+  if (sh >= 0) return m << sh;  // the caller's bound keeps the result below 2^53
+  const int k = -sh;
+  if (k > 63) return 0;  // below one half
+  // round half to even: m / 2^k + 1/2 - 2^-k, plus 2^-k when the last kept bit is odd
+  return (m + ((1ull << (k - 1)) - 1) + ((m >> k) & 1)) >> k;
+}
+
+// m * 2^x with the sign, for results outside the normal range; out of line, so that its FP64
+// instructions are not issued (predicated off) for every element.
+static __device__ __noinline__ double scaled_outside_normal(unsigned long long m, int x, bool neg) {
+  const double v = ldexp((double)m, x);
+  return neg ? -v : v;
+}
+
+// (hi:lo) * 2^-e as a double, (hi:lo) a non-negative 128-bit integer in two words, rounded
+// to nearest even from the bits; results outside the normal range go through ldexp.
+__device__ __forceinline__ double u128w_scaled(unsigned long long hi, unsigned long long lo, bool neg, int e) {
+  if ((hi | lo) == 0) return 0.0;
+  // normalise so that the leading bit is bit 63 of `top`; `rest` keeps the bits below
+  int p;
+  unsigned long long top, rest;
+  if (hi) {
+    const int s = __clzll((long long)hi);
+    p = 127 - s;
+    top = s ? (hi << s) | (lo >> (64 - s)) : hi;
+    rest = s ? (lo << s) : lo;
+  } else {
+    const int s = __clzll((long long)lo);
+    p = 63 - s;
+    top = lo << s;
+    rest = 0;
+  }
+  unsigned long long m = top >> 11;  // 53 bits
+  const unsigned long long low11 = top & 0x7FFull;
+  const bool sticky = (low11 & 0x3FFull) != 0 || rest != 0;
+  if ((low11 & 0x400ull) && (sticky || (m & 1))) {
+    ++m;
+    if (m == (1ull << 53)) {
+      m >>= 1;
+      ++p;
+    }
+  }
+  const int field = p - e + 1023;
+  if (field >= 1 && field <= 2046) {
+    unsigned long long bits = ((unsigned long long)field << 52) | (m & 0xFFFFFFFFFFFFFull);
+    if (neg) bits |= 1ull << 63;
+    return __longlong_as_double((long long)bits);
+  }
+  return scaled_outside_normal(m, p - 52 - e, neg);
 }
 
 // H pass 1: Ht[j][kk] = H(kk, j) in FP64, column max |H| and column sum |H|, and the global
