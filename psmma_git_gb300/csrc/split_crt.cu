@@ -3031,7 +3031,11 @@ static int split_core_host(int M, int N, int K, double alpha, const double* A_h,
   char* w = (char*)work;
   const SplitBuffers b = split_buffers(w, L);
   const CrtConsts cc = get_consts(nmod);
-  const bool spec = pa_guess >= 8 && ph_guess >= 8 && beta == 0.0;
+  // Small operands are not worth a guess: their upload takes little longer than the H passes it
+  // hides behind, and a wrong guess repeats every product (n = 4096, new operands each call: 4.3 ms
+  // guessing, 2.5 ms not; 16384: the upload is 10.7 of 78 ms).
+  const bool small = (size_t)M * K * 8 <= ((size_t)256 << 20);
+  const bool spec = pa_guess >= 8 && ph_guess >= 8 && beta == 0.0 && !small;
   cudaEvent_t* ev_up = ev;               // NP: column chunks or row panels of A landed
   cudaEvent_t* ev_panel = ev + NP;       // NP: panels of Q ready
   cudaEvent_t ev_start = ev[2 * NP], ev_q = ev[2 * NP + 1], ev_done = ev[2 * NP + 2];
@@ -3078,16 +3082,19 @@ static int split_core_host(int M, int N, int K, double alpha, const double* A_h,
   const int tiles_m = (M + G_BM - 1) / G_BM;
   int pb[NP + 1], npanels = 0;  // panel p: row tiles [pb[p], pb[p + 1])
   {
-    const int tp = (tiles_m + 7) / 8;
+    // eighths, but no fewer row tiles than some 0.25 ms of products (a panel costs 60 us of launches and
+    // of a last wave that is partly idle)
+    const double tile_ms = 2.0 * nmod * G_BM * (double)N * K / 1.5e12;
+    const int tp = std::min(tiles_m, std::max((tiles_m + 7) / 8, (int)std::ceil(0.25 / tile_ms)));
     pb[0] = 0;
-    if (tp >= 4 && tiles_m > tp) {
+    if (spec && tp >= 4 && tiles_m > tp) {
       pb[1] = 2;
       pb[2] = tp;
       npanels = 2;
     }
     while (tiles_m - pb[npanels] > tp) { pb[npanels + 1] = pb[npanels] + tp; ++npanels; }
     for (int rest = tiles_m - pb[npanels], cut = 0; rest > 0; ++cut) {
-      const int t = cut < 3 ? (rest + 1) / 2 : rest;
+      const int t = cut < (spec || tp == (tiles_m + 7) / 8 ? 3 : 1) ? (rest + 1) / 2 : rest;
       pb[npanels + 1] = pb[npanels] + t;
       ++npanels;
       rest -= t;
@@ -3184,8 +3191,7 @@ static int split_core_host(int M, int N, int K, double alpha, const double* A_h,
     ok &= cudaEventRecord(ev_up[ch], cs) == cudaSuccess;
     prof_mark(cs, "a_chunk_up");
     ok &= cudaStreamWaitEvent(s, ev_up[ch], 0) == cudaSuccess;
-    dim3 g1((M + 127) / 128, (c1 - c0 + kchunk - 1) / kchunk);
-    k_row_absmax<<<g1, 128, 0, s>>>(dA + (size_t)c0 * M, M, M, c1 - c0, kchunk, b.amax, b.asq);
+    if (launch_row_stats(dA + (size_t)c0 * M, M, M, c1 - c0, b.amax, b.asq, sms, s)) return PSMMA_EDEVICE;
   }
   if (beta != 0.0) {
     ok &= cudaMemcpy2DAsync(dQ, (size_t)M * 8, Q_h, (size_t)ldq_h * 8, (size_t)M * 8, (size_t)N,
