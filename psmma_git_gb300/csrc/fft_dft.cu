@@ -20,10 +20,11 @@
 //               one of the two forms.
 // Sizes none of the three covers keep the dense products (split_crt.cu, fp64_structured.cu).
 //
-// Measured (n = k, against the dense products it replaces): split precision n = 4096 0.60 ms (2.64),
-// 8192 2.13 (7.17), 16384 10.9 (43.0); FP64 n = 4800 1.02 ms (209).  ncu at n = 8192: the integer and
-// the wide multiply-add pipes 45 % busy each, issue 49 %, DRAM 10 %: bound by the passes' instructions
-// (about 680 a point with the conversions) and by the latencies 16 warps leave uncovered.
+// Measured (n = k, against the dense products it replaces): split precision n = 4096 0.30 ms (2.64),
+// 8192 1.42 (7.17), 16384 8.9 (43.0); FP64 n = 4800 0.71 ms (209).  ncu at n = 8192, before the first pass
+// took its entries from registers (1.73 ms): 510 instructions a point with the conversions, the integer
+// pipe 51 % and the wide multiply-adds 37 % busy, issue 45 %, DRAM 12 %: bound by the passes' instructions
+// and by the latencies that 16 warps (128 registers each thread) leave uncovered.
 #include <algorithm>
 #include <cstring>
 
@@ -144,7 +145,17 @@ struct Cx {
 __device__ __forceinline__ Cx operator+(Cx a, Cx b) { return {a.r + b.r, a.i + b.i}; }
 __device__ __forceinline__ Cx operator-(Cx a, Cx b) { return {a.r - b.r, a.i - b.i}; }
 __device__ __forceinline__ Cx sar(Cx a, int s) { return {a.r >> s, a.i >> s}; }
-__device__ __forceinline__ i64 wmad(int a, int b, i64 c) { return (i64)a * b + c; }
+// a b + c as one instruction (left to itself the compiler forms the product and adds it in two more:
+// 680 instead of 510 instructions a point at n = 8192, 2.13 instead of 1.73 ms).
+__device__ __forceinline__ i64 wmad(int a, int b, i64 c) {
+#ifdef __CUDA_ARCH__
+  i64 d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+#else
+  return (i64)a * b + c;
+#endif
+}
 
 // (x w) 2^-64 rounded, w = c + i s in halves: with w in Q62 the product over 4.  The halves of x
 // are taken signed, the product of the low halves (below one unit) left out.  |x| <= 2.6 * 2^61:
@@ -153,7 +164,7 @@ __device__ __forceinline__ Cx cmul(Cx x, Tw t) {
   const int al = (int)x.r, ah = (int)((x.r + 0x80000000ll) >> 32);
   const int bl = (int)x.i, bh = (int)((x.i + 0x80000000ll) >> 32);
   const int nz = -t.z, nw = -t.w;
-  const i64 hr = wmad(bh, nz, (i64)ah * t.x), hi = wmad(bh, t.x, (i64)ah * t.z);
+  const i64 hr = wmad(bh, nz, wmad(ah, t.x, 0)), hi = wmad(bh, t.x, wmad(ah, t.z, 0));
   const i64 mr = wmad(bl, nz, wmad(bh, nw, wmad(al, t.x, wmad(ah, t.y, 0x80000000ll))));
   const i64 mi = wmad(bl, t.x, wmad(bh, t.y, wmad(al, t.z, wmad(ah, t.w, 0x80000000ll))));
   return {hr + (mr >> 32), hi + (mi >> 32)};
@@ -260,13 +271,16 @@ struct Plan {
   Pass p[FFT_MAX_PASSES];
 };
 
-const int kRadices[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
+// Radices of the passes.  Powers of two take 16; in the general passes, whose addresses are not an XOR
+// with a constant, 16 and 15 points and their addresses do not fit 128 registers (n = 4800 as
+// 2 * 10 * 15 * 16 0.81 ms, its spills gone with 5 * 8 * 10 * 12).
+const int kRadices[] = {16, 12, 10, 9, 8, 6, 5, 4, 3, 2};
 
-// Fewest passes first, then the least spread: searched depth first over the radices.
+// Depth first over the radices, the largest first, for exactly `left` passes.
 bool factor(int n, int left, int* r, int at, int from) {
   if (n == 1) return left == 0;
   if (left == 0) return false;
-  for (int i = from; i < 11; ++i)
+  for (int i = from; i < 10; ++i)
     if (n % kRadices[i] == 0) {
       r[at] = kRadices[i];
       if (factor(n / kRadices[i], left - 1, r, at + 1, i)) return true;
@@ -279,10 +293,12 @@ bool make_plan(int n, Plan* P) {
   P->n = n;
   int r[FFT_MAX_PASSES];
   for (int np = 1; np <= 8; ++np)
-    if (n == 1 || factor(n, np, r, 0, 0)) {
+    if (n == 1 || factor(n, np, r, 0, (n & (n - 1)) ? 1 : 0)) {
       P->np = n == 1 ? 0 : np;
       std::reverse(r, r + P->np);  // the largest radix last: the last pass of the direct form finds
                                    // each butterfly's place by np - 1 divisions
+      // powers of two also begin with a radix of 16 (the first pass then takes its entries from global memory)
+      if ((n & (n - 1)) == 0 && P->np > 2) std::swap(r[0], r[1]);
       int N = n;
       for (int i = 0; i < P->np; ++i) {
         P->p[i] = {r[i], N, N / r[i], P->entries};
@@ -512,17 +528,17 @@ __device__ __forceinline__ Range pass_r(longlong2* s, const Pass& P, int n, int 
   return range;
 }
 
-template <bool DIT>
+// P2: powers of two alone.
+template <bool DIT, bool P2>
 __device__ __forceinline__ Range pass(longlong2* s, const Pass& P, int n, int d, const Tw* tw) {
-  if ((n & (n - 1)) == 0) switch (P.R) {
+  if (P2 || (n & (n - 1)) == 0) switch (P.R) {
       case 16: return pass_r<16, DIT, true>(s, P, n, d, tw);
       case 8: return pass_r<8, DIT, true>(s, P, n, d, tw);
       case 4: return pass_r<4, DIT, true>(s, P, n, d, tw);
       default: return pass_r<2, DIT, true>(s, P, n, d, tw);
     }
+  if constexpr (P2) return Range{};
   switch (P.R) {
-    case 16: return pass_r<16, DIT, false>(s, P, n, d, tw);
-    case 15: return pass_r<15, DIT, false>(s, P, n, d, tw);
     case 12: return pass_r<12, DIT, false>(s, P, n, d, tw);
     case 10: return pass_r<10, DIT, false>(s, P, n, d, tw);
     case 9: return pass_r<9, DIT, false>(s, P, n, d, tw);
@@ -666,30 +682,33 @@ __device__ __forceinline__ void last_r(longlong2* s, const Plan& P, const FftArg
   }
 }
 
-// The transform of one column (Bluestein: of length L, forward, in place).  `e` is the exponent of
-// the entries, kept by every thread.
-__device__ __forceinline__ int forward(longlong2* s, const Plan& P, const Tw* tw, unsigned* words, int w0, int np, int& e) {
-  for (int p = 0; p < np; ++p) {
-    const int d = headroom(words[w0 + p], FFT_TOP);
-    publish(pass<false>(s, P.p[p], P.n, d, tw), &words[w0 + p + 1]);
+// Passes p0 .. np - 1 of one column's transform, in place; words[p] holds the magnitude before pass p, `e` the
+// exponent of the entries, kept by every thread.
+template <bool P2 = false>
+__device__ __forceinline__ int forward(longlong2* s, const Plan& P, const Tw* tw, unsigned* words, int p0, int np, int& e) {
+  for (int p = p0; p < np; ++p) {
+    const int d = headroom(words[p], FFT_TOP);
+    publish(pass<false, P2>(s, P.p[p], P.n, d, tw), &words[p + 1]);
     e += inner_shift(P.p[p].R) + (P.p[p].M > 1 ? outer_shift(P.p[p].R) : 0) - d;
     __syncthreads();
   }
-  return w0 + np;
+  return np;
 }
 
+// FIRST16: direct form, a power of two of at least 512 points, a thread per radix-16 butterfly.
+template <bool FIRST16>
 __global__ void __launch_bounds__(512, 1) k_fft(const __grid_constant__ Plan P, const __grid_constant__ FftArgs a) {
   extern __shared__ __align__(16) unsigned char fft_smem[];
   longlong2* s = (longlong2*)fft_smem;
   __shared__ unsigned words[2 * FFT_MAX_PASSES + 4];
   __shared__ unsigned hmax;
   const int col = blockIdx.x / a.R0, s0 = blockIdx.x - col * a.R0;
-  const bool blue = a.form == FORM_BLUESTEIN;
+  const bool blue = !FIRST16 && a.form == FORM_BLUESTEIN;
   if (threadIdx.x < 2 * FFT_MAX_PASSES + 4) words[threadIdx.x] = 0u;
   if (threadIdx.x == 0) hmax = 0u;
   __syncthreads();
-  int e;
-  if (a.R0 > 1) {
+  int e, p0 = 0;
+  if (!FIRST16 && a.R0 > 1) {
     e = a.ce[col];
     if (e == NO_EXP) {
       nonfinite_column(a, col, s0);
@@ -709,6 +728,46 @@ __global__ void __launch_bounds__(512, 1) k_fft(const __grid_constant__ Plan P, 
     }
     publish(m, &words[0]);
     if (blue) e += 2;
+  } else if (FIRST16) {
+    // a thread's sixteen entries stay in registers from global memory through the first pass
+    const double* src = a.B + 2 * (long)col * a.ldb;
+    const int M = P.n / 16, m0 = threadIdx.x;
+    double2 v[16];
+    unsigned hm = 0;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) v[r] = load_c(src + 2 * (m0 + M * r), a.b16);
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+      hm = max(hm, max((unsigned)__double2hiint(v[r].x) & 0x7FFFFFFFu, (unsigned)__double2hiint(v[r].y) & 0x7FFFFFFFu));
+    hm = __reduce_max_sync(0xffffffffu, hm);
+    if ((threadIdx.x & 31) == 0) atomicMax(&hmax, hm);
+    __syncthreads();
+    const unsigned hmx = hmax;
+    if (hmx >= 0x7FF00000u) {
+      nonfinite_column(a, col, 0);
+      return;
+    }
+    const int emax = col_exponent(hmx);
+    Cx x[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) x[r] = {fx_from(v[r].x, emax), fx_from(v[r].y, emax)};
+    bf<16>(x);
+    x[0] = sar(x[0], outer_shift(16));
+    const int4* t = (const int4*)(a.tw + P.p[0].tw) + m0;
+    const int b0 = sw(m0);
+    Range m;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      if (r > 0) {
+        const int4 w = __ldg(t + (r - 1) * M);
+        x[r] = cmul(x[r], Tw{w.x, w.y, w.z, w.w});
+      }
+      s[b0 ^ sw(M * r)] = make_longlong2(x[r].r, x[r].i);
+      m.add(x[r]);
+    }
+    publish(m, &words[1]);
+    e = emax - (FFT_TOP - 1) + inner_shift(16) + outer_shift(16);
+    p0 = 1;
   } else {
     const double* src = a.B + 2 * (long)col * a.ldb;
     unsigned hm = 0;
@@ -755,11 +814,11 @@ __global__ void __launch_bounds__(512, 1) k_fft(const __grid_constant__ Plan P, 
       if (threadIdx.x == 0) put(a, col, s0, ld(s, 0), e);
       return;
     }
-    const int w = forward(s, P, a.tw, words, 0, P.np - 1, e);
+    const int w = forward<FIRST16>(s, P, a.tw, words, p0, P.np - 1, e);
     const int d = headroom(words[w], FFT_TOP);
     e -= d;
     const int R = P.p[P.np - 1].R;
-    if ((P.n & (P.n - 1)) == 0) {
+    if (FIRST16 || (P.n & (P.n - 1)) == 0) {
       switch (R) {
         case 16: last_r<16, true>(s, P, a, col, s0, d, e); break;
         case 8: last_r<8, true>(s, P, a, col, s0, d, e); break;
@@ -769,8 +828,6 @@ __global__ void __launch_bounds__(512, 1) k_fft(const __grid_constant__ Plan P, 
       return;
     }
     switch (R) {
-      case 16: last_r<16, false>(s, P, a, col, s0, d, e); break;
-      case 15: last_r<15, false>(s, P, a, col, s0, d, e); break;
       case 12: last_r<12, false>(s, P, a, col, s0, d, e); break;
       case 10: last_r<10, false>(s, P, a, col, s0, d, e); break;
       case 9: last_r<9, false>(s, P, a, col, s0, d, e); break;
@@ -783,6 +840,7 @@ __global__ void __launch_bounds__(512, 1) k_fft(const __grid_constant__ Plan P, 
     }
     return;
   }
+  if constexpr (FIRST16) return;
 
   // ---- Bluestein: transform, product with the chirp's, inverse transform (of the swapped parts)
   int w = forward(s, P, a.tw, words, 0, P.np, e);
@@ -802,7 +860,7 @@ __global__ void __launch_bounds__(512, 1) k_fft(const __grid_constant__ Plan P, 
   }
   for (int p = P.np - 1; p >= 0; --p) {
     const int d = headroom(words[w], 61);
-    publish(pass<true>(s, P.p[p], P.n, d, a.tw), &words[++w]);
+    publish(pass<true, false>(s, P.p[p], P.n, d, a.tw), &words[++w]);
     e += inner_shift(P.p[p].R) + outer_shift(P.p[p].R) - d;
     __syncthreads();
   }
@@ -953,8 +1011,13 @@ int launch_fft(int n, int k, double alpha, const double* B, long ldb, double bet
   const size_t smem = (size_t)((N + 7) / 8 * 8) * 16;
   // 128 registers a thread: 512 threads fill an SM.  They are shared by the columns whose entries fit
   // its shared memory (8 at most), so that one column's loads and stores overlap another's passes.
-  const int cols = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)227 * 1024 / (smem + 2048)));
-  const int threads = std::max(64, 512 / cols / 32 * 32);
+  const bool first16 = r.R0 == 1 && !blue && (N & (N - 1)) == 0 && N >= 512 && N <= 8192 && r.plan.p[0].R == 16;
+  int cols = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)227 * 1024 / (smem + 2048)));
+  int threads = std::max(64, 512 / cols / 32 * 32);
+  if (first16) {
+    threads = N / 16;
+    cols = std::min(cols, 512 / threads);
+  }
 
   prof_begin(stream);
   const int entries = std::max(r.plan.entries, std::max(r.n1, r.R0 > 1 ? (r.R0 - 1) * r.n1 : 0));
@@ -971,12 +1034,13 @@ int launch_fft(int n, int k, double alpha, const double* B, long ldb, double bet
     prof_mark(stream, "dft_first_pass");
   }
   // the attribute is the kernel's, shared by every thread that launches it: one value for all
-  if (set_smem_attr(k_fft, FFT_MAX * 16) != cudaSuccess) return PSMMA_EDEVICE;
+  if (set_smem_attr(k_fft<true>, FFT_MAX * 16) != cudaSuccess || set_smem_attr(k_fft<false>, FFT_MAX * 16) != cudaSuccess)
+    return PSMMA_EDEVICE;
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return PSMMA_EDEVICE;
   a.ahead = sms * cols;
-  k_fft<<<k * r.R0, threads, smem, stream>>>(r.plan, a);
+  (first16 ? k_fft<true> : k_fft<false>)<<<k * r.R0, threads, smem, stream>>>(r.plan, a);
   prof_mark(stream, "dft_transform");
   return cudaGetLastError() == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
 }
