@@ -187,6 +187,21 @@ __global__ void k_ex_h(GenSpec gs, int K, int kp, double* __restrict__ Ht, unsig
   h_pass1_blk<KIND, true>(gs, K, kp, Ht, hmax, hsum, hsq, nullptr, blockIdx.x, nullptr, hlsb);
 }
 
+// Both, for small operands: the first blocks 32 rows of A each (the longest), then a column of H each.
+template <int KIND>
+__global__ void __launch_bounds__(256) k_ex_stats(GenSpec gs, int M, int N, int K, int kp, const double* __restrict__ A,
+                                                  long lda, unsigned long long* __restrict__ amax,
+                                                  double* __restrict__ asq, int* __restrict__ alsb,
+                                                  double* __restrict__ Ht, unsigned long long* __restrict__ hmax,
+                                                  double* __restrict__ hsum, double* __restrict__ hsq,
+                                                  int* __restrict__ hlsb) {
+  const int rb = (M + SMALL_RB - 1) / SMALL_RB, b = blockIdx.x;
+  if (b < rb)
+    small_rows_blk<true>(A, lda, M, K, b, amax, asq, alsb);
+  else
+    h_pass1_blk<KIND, true>(gs, K, kp, Ht, hmax, hsum, hsq, nullptr, b - rb, nullptr, hlsb);
+}
+
 // An upper bound of log2 of the mantissa (in [1, 2)) of the normal double with bits b.
 __device__ __forceinline__ float log2_mant_up(unsigned long long b) {
   const float f = __uint_as_float(0x3F800000u | ((unsigned)(b >> 29) & 0x7FFFFFu));
@@ -196,12 +211,20 @@ __device__ __forceinline__ float log2_mant_up(unsigned long long b) {
 // Number of moduli and chunk counts from the statistics.  With a'_i = row i of A' = A 2^-alsb_i and
 // h'_j likewise, |Z_ij| <= max|a'| max sum|h'| and <= max ||a'||_2 max ||h'||_2; the CRT needs
 // |Z| < 0.497 M.  Norms whose squares leave the range of FP64 count max * sqrt(k).
-__global__ void __launch_bounds__(1024) k_ex_params(ExParams* prm, ExLog2 lg, int max_groups, int M, int N, int K,
-                                                    const unsigned long long* __restrict__ amax,
-                                                    const double* __restrict__ asq, const int* __restrict__ alsb,
-                                                    const unsigned long long* __restrict__ hmax,
-                                                    const double* __restrict__ hsum, const double* __restrict__ hsq,
-                                                    const int* __restrict__ hlsb) {
+// One block; thread 0 returns them.
+struct ExStats {
+  const unsigned long long* amax;
+  const double* asq;
+  const int* alsb;
+  const unsigned long long* hmax;
+  const double *hsum, *hsq;
+  const int* hlsb;
+};
+__device__ __forceinline__ ExParams ex_params(const ExStats& st, const ExLog2& lg, int max_groups, int M, int N, int K) {
+  const unsigned long long *amax = st.amax, *hmax = st.hmax;
+  const double *asq = st.asq, *hsum = st.hsum, *hsq = st.hsq;
+  const int *alsb = st.alsb, *hlsb = st.hlsb;
+  ExParams prm{0u, 0, 0, 0, 1u};
   float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // bits A, log2 max A, log2 ||A||, bits H, log2 sum H, log2 ||H||
   int bad = 0;
   const float lk = log2f((float)K) + 1e-3f;
@@ -244,11 +267,18 @@ __global__ void __launch_bounds__(1024) k_ex_params(ExParams* prm, ExLog2 lg, in
     int g = 2;
     while (g <= max_groups && lg.v[g] < need) ++g;
     const bool fits = !bad && g <= max_groups && v[0] <= 14.f * EX_CHUNKS && v[3] <= 14.f * EX_CHUNKS;
-    prm->ncA = ((int)v[0] + 13) / 14;
-    prm->ncH = ((int)v[3] + 13) / 14;
-    prm->nmod = fits ? 4 * g : 0;
-    prm->run_dmma = fits ? 0u : 1u;
+    prm.ncA = ((int)v[0] + 13) / 14;
+    prm.ncH = ((int)v[3] + 13) / 14;
+    prm.nmod = fits ? 4 * g : 0;
+    prm.run_dmma = fits ? 0u : 1u;
   }
+  return prm;
+}
+
+__global__ void __launch_bounds__(1024) k_ex_params(ExParams* prm, ExLog2 lg, int max_groups, int M, int N, int K,
+                                                    ExStats st) {
+  const ExParams p = ex_params(st, lg, max_groups, M, N, K);
+  if (threadIdx.x == 0) *prm = p;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -324,14 +354,11 @@ __device__ __forceinline__ void ex_write_quad_nc(int nc, const double (&x)[4], i
 
 // RA[l][i][kk], rows i, K-major: 64 x 64 tiles of A transposed through shared memory (element
 // (k, r) at column (r + k/4) mod 64 of row k: conflict-free both ways).
-__global__ void __launch_bounds__(256) k_ex_residues_A(const double* __restrict__ A, long lda, int n, int k, int kp,
-                                                       const int* __restrict__ alsb, const ExParams* prm,
-                                                       __nv_bfloat16* __restrict__ RA) {
+__device__ __forceinline__ void ex_residues_A_blk(const double* __restrict__ A, long lda, int n, int k, int kp,
+                                                  const int* __restrict__ alsb, int nmod, int nc,
+                                                  __nv_bfloat16* __restrict__ RA, int bx, int by) {
   __shared__ double tile[64][64];
-  const int nmod = prm->nmod;
-  if (nmod == 0) return;
-  const int nc = prm->ncA;
-  const int i0 = blockIdx.x * 64, k0 = blockIdx.y * 64;
+  const int i0 = bx * 64, k0 = by * 64;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int kk = ty; kk < 64; kk += 8) {
     const int gk = k0 + kk;
@@ -355,6 +382,26 @@ __global__ void __launch_bounds__(256) k_ex_residues_A(const double* __restrict_
   }
 }
 
+__global__ void __launch_bounds__(256) k_ex_residues_A(const double* __restrict__ A, long lda, int n, int k, int kp,
+                                                       const int* __restrict__ alsb, const ExParams* prm,
+                                                       __nv_bfloat16* __restrict__ RA) {
+  const int nmod = prm->nmod;
+  if (nmod == 0) return;
+  ex_residues_A_blk(A, lda, n, k, kp, alsb, nmod, prm->ncA, RA, blockIdx.x, blockIdx.y);
+}
+
+// Entries kk .. kk + 3 of column j.
+__device__ __forceinline__ void ex_residues_H_quad(const double* __restrict__ Ht, int ncols, int kp,
+                                                   const int* __restrict__ hlsb, int nmod, int nc,
+                                                   __nv_bfloat16* __restrict__ RH, int j, int kk) {
+  const int lsb = hlsb[j];
+  const double2 h01 = *(const double2*)(Ht + (size_t)j * kp + kk);
+  const double2 h23 = *(const double2*)(Ht + (size_t)j * kp + kk + 2);
+  const double x[4] = {h01.x, h01.y, h23.x, h23.y};
+  const size_t plane = (size_t)ncols * kp;
+  ex_write_quad_nc(nc, x, lsb, lsb != NO_LSB, nmod, (uint2*)(RH + (size_t)j * kp + kk), plane / 4);
+}
+
 __global__ void __launch_bounds__(128) k_ex_residues_H(const double* __restrict__ Ht, int ncols, int kp,
                                                        const int* __restrict__ hlsb, const ExParams* prm,
                                                        __nv_bfloat16* __restrict__ RH) {
@@ -362,12 +409,36 @@ __global__ void __launch_bounds__(128) k_ex_residues_H(const double* __restrict_
   if (nmod == 0) return;
   const int j = blockIdx.x, kk = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
   if (kk >= kp) return;  // kp is a multiple of 64
-  const int lsb = hlsb[j];
-  const double2 h01 = *(const double2*)(Ht + (size_t)j * kp + kk);
-  const double2 h23 = *(const double2*)(Ht + (size_t)j * kp + kk + 2);
-  const double x[4] = {h01.x, h01.y, h23.x, h23.y};
-  const size_t plane = (size_t)ncols * kp;
-  ex_write_quad_nc(prm->ncH, x, lsb, lsb != NO_LSB, nmod, (uint2*)(RH + (size_t)j * kp + kk), plane / 4);
+  ex_residues_H_quad(Ht, ncols, kp, hlsb, nmod, prm->ncH, RH, j, kk);
+}
+
+// Both, for small operands: blocks 0 .. a_blocks - 1 are the 64 x 64 tiles of A, the others 256 quads of H each.
+// INLINE: every block evaluates the parameters, block 0 publishes them.
+template <bool INLINE>
+__global__ void __launch_bounds__(256) k_ex_residues(const double* __restrict__ A, long lda, int M, int N, int K, int kp,
+                                                     ExStats st, ExLog2 lg, int max_groups, int a_blocks,
+                                                     const double* __restrict__ Ht, __nv_bfloat16* __restrict__ RA,
+                                                     __nv_bfloat16* __restrict__ RH, ExParams* prm) {
+  __shared__ ExParams sp;
+  if (INLINE) {
+    const ExParams p = ex_params(st, lg, max_groups, M, N, K);
+    if (threadIdx.x == 0) {
+      sp = p;
+      if (blockIdx.x == 0) *prm = p;
+    }
+  } else if (threadIdx.x == 0) {
+    sp = *prm;
+  }
+  __syncthreads();
+  if (sp.nmod == 0) return;
+  const int b = blockIdx.x;
+  if (b < a_blocks) {
+    const int tm = (M + 63) / 64;
+    ex_residues_A_blk(A, lda, M, K, kp, st.alsb, sp.nmod, sp.ncA, RA, b % tm, b / tm);
+  } else {
+    const int q = (b - a_blocks) * 256 + threadIdx.x, per = kp / 4, j = q / per;
+    if (j < N) ex_residues_H_quad(Ht, N, kp, st.hlsb, sp.nmod, sp.ncH, RH, j, 4 * (q - j * per));
+  }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -596,29 +667,55 @@ int launch_exact(int M, int N, int K, double alpha, const double* A, long lda, c
   int8_t* R = (int8_t*)(w + L.off_r);
   *gate = &prm->run_dmma;
 
+  const ExStats xs{amax, asq, alsb, hmax, hsum, hsq, hlsb};
   prof_begin(stream);
-  k_ex_init<<<(M + 255) / 256, 256, 0, stream>>>(prm, amax, asq, alsb, M);
-  // enough blocks for some eight waves, so that the loads of a chunk (eight in flight a thread) are
-  // not a serial chain: n = 2048 at 1024-column chunks 208 us, n = 256 at 128 27 us
-  int kchunk = 1024;
-  while (kchunk > 16 && (long)((M + 127) / 128) * ((K + kchunk - 1) / kchunk) < 8L * sms) kchunk >>= 1;
-  k_ex_row_stats<<<dim3((M + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, stream>>>(A, lda, M, K, kchunk, amax, asq,
-                                                                                     alsb);
-  prof_mark(stream, "row_scale");
-  switch (gs.kind) {
-    case KIND_CAUCHY: k_ex_h<KIND_CAUCHY><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
-    case KIND_TOEPLITZ: k_ex_h<KIND_TOEPLITZ><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
-    case KIND_HANKEL: k_ex_h<KIND_HANKEL><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
-    case KIND_CAUCHY_EIG: k_ex_h<KIND_CAUCHY_EIG><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
-    default: return PSMMA_EUNSUPPORTED;
+  if (small_operands(M, N, K)) {
+    const int blocks = N + (M + SMALL_RB - 1) / SMALL_RB;
+    switch (gs.kind) {
+#define PSMMA_STATS(KD) \
+  case KD: k_ex_stats<KD><<<blocks, 256, 0, stream>>>(gs, M, N, K, L.kp, A, lda, amax, asq, alsb, Ht, hmax, hsum, hsq, hlsb); break;
+      PSMMA_STATS(KIND_CAUCHY)
+      PSMMA_STATS(KIND_TOEPLITZ)
+      PSMMA_STATS(KIND_HANKEL)
+      PSMMA_STATS(KIND_CAUCHY_EIG)
+#undef PSMMA_STATS
+      default: return PSMMA_EUNSUPPORTED;
+    }
+    prof_mark(stream, "statistics");
+    const int a_blocks = ((M + 63) / 64) * (L.kp / 64), h_blocks = (N * (L.kp / 4) + 255) / 256;
+    if (M + N <= INLINE_ROWS) {
+      k_ex_residues<true><<<a_blocks + h_blocks, 256, 0, stream>>>(A, lda, M, N, K, L.kp, xs, lg, planes / 4, a_blocks, Ht, RA,
+                                                                   RH, prm);
+    } else {
+      k_ex_params<<<1, 1024, 0, stream>>>(prm, lg, planes / 4, M, N, K, xs);
+      k_ex_residues<false><<<a_blocks + h_blocks, 256, 0, stream>>>(A, lda, M, N, K, L.kp, xs, lg, planes / 4, a_blocks, Ht,
+                                                                    RA, RH, prm);
+    }
+    prof_mark(stream, "residues");
+  } else {
+    k_ex_init<<<(M + 255) / 256, 256, 0, stream>>>(prm, amax, asq, alsb, M);
+    // enough blocks for some eight waves, so that the loads of a chunk (eight in flight a thread) are
+    // not a serial chain: n = 2048 at 1024-column chunks 208 us, n = 256 at 128 27 us
+    int kchunk = 1024;
+    while (kchunk > 16 && (long)((M + 127) / 128) * ((K + kchunk - 1) / kchunk) < 8L * sms) kchunk >>= 1;
+    k_ex_row_stats<<<dim3((M + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, stream>>>(A, lda, M, K, kchunk, amax, asq,
+                                                                                       alsb);
+    prof_mark(stream, "row_scale");
+    switch (gs.kind) {
+      case KIND_CAUCHY: k_ex_h<KIND_CAUCHY><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
+      case KIND_TOEPLITZ: k_ex_h<KIND_TOEPLITZ><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
+      case KIND_HANKEL: k_ex_h<KIND_HANKEL><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
+      case KIND_CAUCHY_EIG: k_ex_h<KIND_CAUCHY_EIG><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
+      default: return PSMMA_EUNSUPPORTED;
+    }
+    prof_mark(stream, "h_generate");
+    k_ex_params<<<1, 1024, 0, stream>>>(prm, lg, planes / 4, M, N, K, xs);
+    prof_mark(stream, "params");
+    k_ex_residues_A<<<dim3((M + 63) / 64, L.kp / 64), 256, 0, stream>>>(A, lda, M, K, L.kp, alsb, prm, RA);
+    prof_mark(stream, "residues_A");
+    k_ex_residues_H<<<dim3(N, (L.kp / 4 + 127) / 128), 128, 0, stream>>>(Ht, N, L.kp, hlsb, prm, RH);
+    prof_mark(stream, "residues_H");
   }
-  prof_mark(stream, "h_generate");
-  k_ex_params<<<1, 1024, 0, stream>>>(prm, lg, planes / 4, M, N, K, amax, asq, alsb, hmax, hsum, hsq, hlsb);
-  prof_mark(stream, "params");
-  k_ex_residues_A<<<dim3((M + 63) / 64, L.kp / 64), 256, 0, stream>>>(A, lda, M, K, L.kp, alsb, prm, RA);
-  prof_mark(stream, "residues_A");
-  k_ex_residues_H<<<dim3(N, (L.kp / 4 + 127) / 128), 128, 0, stream>>>(Ht, N, L.kp, hlsb, prm, RH);
-  prof_mark(stream, "residues_H");
   const int st = launch_modular_gemm(RA, RH, R, M, N, L.kp, L.kr, planes, kExModuli, &prm->nmod, &prm->status, sms, stream);
   if (st) return st;
   prof_mark(stream, "modular_gemm");

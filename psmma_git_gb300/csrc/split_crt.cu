@@ -601,15 +601,10 @@ __global__ void k_guess_params(SplitDevParams* g, int PA, int PH) {
 }
 
 // RH[l][j][kk] = residues of H' (bf16) from Ht[j][kk]; one thread per 4 consecutive kk.
-__device__ __forceinline__ void residues_H_blk(const double* __restrict__ Ht, int ncols, int kp,
-                                               const unsigned long long* __restrict__ hmax_bits,
-                                               const SplitDevParams* prm, const CrtConsts& cc,
-                                               __nv_bfloat16* __restrict__ RH, int bx, int by, int ph = -1,
-                                               int krows = 1 << 30) {
-  const int j = by;
-  const int kk = RH_PER_THREAD * (bx * blockDim.x + threadIdx.x);
-  if (kk >= kp) return;  // kp is a multiple of 64: a thread's four entries are all inside
-  const int P = ph >= 0 ? ph : prm->PH;
+__device__ __forceinline__ void residues_H_quad(const double* __restrict__ Ht, int ncols, int kp,
+                                                const unsigned long long* __restrict__ hmax_bits, int P,
+                                                const CrtConsts& cc, __nv_bfloat16* __restrict__ RH, int j, int kk,
+                                                int krows) {
   unsigned long long hb = hmax_bits[j];
   bool ok = hb > 0 && hb < INF_BITS;
   int e = ok ? scale_exp(hb, P) : 0;
@@ -625,6 +620,107 @@ __device__ __forceinline__ void residues_H_blk(const double* __restrict__ Ht, in
   }
   const size_t plane = (size_t)ncols * kp;
   write_residue_quad(u, ng, cc, (uint2*)(RH + (size_t)j * kp + kk), plane / 4);
+}
+
+__device__ __forceinline__ void residues_H_blk(const double* __restrict__ Ht, int ncols, int kp,
+                                               const unsigned long long* __restrict__ hmax_bits,
+                                               const SplitDevParams* prm, const CrtConsts& cc,
+                                               __nv_bfloat16* __restrict__ RH, int bx, int by, int ph = -1,
+                                               int krows = 1 << 30) {
+  const int kk = RH_PER_THREAD * (bx * blockDim.x + threadIdx.x);
+  if (kk >= kp) return;  // kp is a multiple of 64: a thread's four entries are all inside
+  residues_H_quad(Ht, ncols, kp, hmax_bits, ph >= 0 ? ph : prm->PH, cc, RH, by, kk, krows);
+}
+
+// Small operands (split_passes.cuh): the statistics of both operands in one launch, the first blocks 32 rows of
+// A each (the longest), then a column of H each; the parameters (rho from the columns' sums); the residues
+// of both.
+template <int KIND>
+__global__ void __launch_bounds__(256) k_split_stats(GenSpec gs, int M, int N, int K, int kp,
+                                                     const double* __restrict__ A, long lda,
+                                                     unsigned long long* __restrict__ amax, double* __restrict__ asq,
+                                                     double* __restrict__ Ht, unsigned long long* __restrict__ hmax,
+                                                     double* __restrict__ hsum, double* __restrict__ hsq) {
+  const int rb = (M + SMALL_RB - 1) / SMALL_RB, b = blockIdx.x;
+  if (b < rb)
+    small_rows_blk<false>(A, lda, M, K, b, amax, asq, nullptr);
+  else
+    h_pass1_blk<KIND>(gs, K, kp, Ht, hmax, hsum, hsq, nullptr, b - rb);
+}
+
+// One block: PA, PH and rho into *sp, with a clear status (thread 0).
+__device__ __forceinline__ void small_params(double log2M, int M, int N, int K, const unsigned long long* __restrict__ amax,
+                                             const double* __restrict__ asq, const unsigned long long* __restrict__ hmax,
+                                             const double* __restrict__ hsum, const double* __restrict__ hsq,
+                                             SplitDevParams* sp) {
+  __shared__ int rho_bits;  // of a positive float
+  if (threadIdx.x == 0) rho_bits = 0;
+  __syncthreads();
+  float rho = 0.0f;
+  for (int j = threadIdx.x; j < N; j += blockDim.x) {
+    const unsigned long long mb = hmax[j], sb = (unsigned long long)__double_as_longlong(hsum[j]);
+    if (mb == 0 || mb >= INF_BITS || sb >= INF_BITS) continue;
+    const float m = __uint_as_float(0x3F800000u | ((unsigned)(mb >> 29) & 0x7FFFFFu));
+    const float q = __uint_as_float((0x3F800000u | ((unsigned)(sb >> 29) & 0x7FFFFFu)) + 1u);
+    const int e = (int)(sb >> 52) - (int)(mb >> 52);  // 0 .. log2 k (+ 1)
+    rho = fmaxf(rho, __fdiv_ru(q, m) * __uint_as_float((unsigned)(127 + max(-1, min(e, 60))) << 23));
+  }
+  rho = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(rho)));
+  if ((threadIdx.x & 31) == 0) atomicMax(&rho_bits, __float_as_int(rho));
+  double v[6];
+  params_partial(0, M, 0, N, (float)K, amax, asq, hmax, hsq, v);  // (synchronises)
+  if (threadIdx.x == 0) {
+    sp->status = 0u;
+    sp->done = 0u;
+    sp->hbad = 0u;
+    sp->rho_bits = (unsigned long long)__double_as_longlong((double)__int_as_float(rho_bits));
+    params_finish(sp, log2M, K, v);
+  }
+}
+
+__global__ void __launch_bounds__(512) k_split_small_params(double log2M, int M, int N, int K,
+                                                            const unsigned long long* __restrict__ amax,
+                                                            const double* __restrict__ asq,
+                                                            const unsigned long long* __restrict__ hmax,
+                                                            const double* __restrict__ hsum,
+                                                            const double* __restrict__ hsq, SplitDevParams* prm) {
+  small_params(log2M, M, N, K, amax, asq, hmax, hsum, hsq, prm);
+}
+
+// INLINE: every block evaluates the parameters, block 0 publishes them.
+template <bool INLINE>
+__global__ void __launch_bounds__(256) k_split_residues(const double* __restrict__ A, long lda, int M, int N, int K, int kp,
+                                                        const unsigned long long* __restrict__ amax,
+                                                        const double* __restrict__ asq,
+                                                        const unsigned long long* __restrict__ hmax,
+                                                        const double* __restrict__ hsum, const double* __restrict__ hsq,
+                                                        int a_blocks, const double* __restrict__ Ht, CrtConsts cc,
+                                                        __nv_bfloat16* __restrict__ RA, __nv_bfloat16* __restrict__ RH,
+                                                        SplitDevParams* out) {
+  __shared__ SplitDevParams sp;
+  if (INLINE) {
+    small_params(cc.log2M, M, N, K, amax, asq, hmax, hsum, hsq, &sp);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      out->status = 0u;
+      out->PA = sp.PA;
+      out->PH = sp.PH;
+      out->rho_bits = sp.rho_bits;
+      out->done = 0u;
+      out->hbad = 0u;
+    }
+  } else if (threadIdx.x == 0) {
+    sp.PA = out->PA;
+    sp.PH = out->PH;
+  }
+  __syncthreads();
+  const int b = blockIdx.x;
+  if (b < a_blocks) {
+    const int tk = kp / 64;
+    residues_A_blk<64>(A, lda, nullptr, 0, K, M, K, kp, amax, &sp, cc, RA, b % tk, b / tk);
+  } else {
+    const int q = (b - a_blocks) * 256 + threadIdx.x, per = kp / 4, j = q / per;
+    if (j < N) residues_H_quad(Ht, N, kp, hmax, sp.PH, cc, RH, j, 4 * (q - j * per), 1 << 30);
+  }
 }
 
 __global__ void k_residues_H(const double* __restrict__ Ht, int ncols, int kp,
@@ -1882,7 +1978,7 @@ __device__ __forceinline__ void crt_row4(const int8_t* __restrict__ rp, size_t p
 // that of hmax_bits[j].
 // TOP32 (cc.top32): the sum over the moduli of (r_l + 128) times the top 32-bit limb of C_l
 // stays below 2^32 (true for M < 2^112: every top limb is below 2^16), so it is kept in 32 bits.
-template <bool DFT_OUT, bool TOP32 = false>
+template <bool DFT_OUT, bool TOP32 = false, int TI = CRT_TI>
 __device__ __forceinline__ void crt_combine_blk(const int8_t* __restrict__ R, int n, int k, int kr,
                                                 const CrtConsts& cc, const unsigned long long* __restrict__ amax_bits,
                                                 const unsigned long long* __restrict__ hmax_bits,
@@ -1892,9 +1988,9 @@ __device__ __forceinline__ void crt_combine_blk(const int8_t* __restrict__ R, in
                                                 int gw = 1) {
   // element (jl, il) of the tile at column (il + jl/4) mod 32 of row jl: the row-wise writes
   // (4 columns per thread) and the column-wise reads both hit distinct bank pairs
-  __shared__ double tile[CRT_TJ][CRT_TI];
+  __shared__ double tile[CRT_TJ][TI];
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int i0 = by * CRT_TI, j0 = bx * CRT_TJ;
+  const int i0 = by * TI, j0 = bx * CRT_TJ;
   const int PA = prm->PA, PH = prm->PH;
   const int jb = j0 + 4 * tx;
   const int kcols = DFT_OUT ? kr : k;  // residue columns covered
@@ -1909,37 +2005,37 @@ __device__ __forceinline__ void crt_combine_blk(const int8_t* __restrict__ R, in
     fexp[c] = (hb[c] != 0 && hb[c] < INF_BITS) ? scale_exp(hb[c], PH) : 0;
   }
   const size_t plane_w = (size_t)n * kr / 4;
-  for (int a = 0; a < CRT_TI / 8; ++a) {
+  for (int a = 0; a < TI / 8; ++a) {
     const int il = ty + 8 * a, i = i0 + il;
     double val[4] = {0.0, 0.0, 0.0, 0.0};
     if (i < n && jb < kcols) crt_row4<TOP32>(R + (size_t)i * kr + jb, plane_w, cc, amax_bits[i], PA, hb, fexp, val);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) tile[4 * tx + c][(il + tx) & 31] = val[c];
+    for (int c = 0; c < 4; ++c) tile[4 * tx + c][(il + tx) & (TI - 1)] = val[c];
   }
   __syncthreads();
   const bool scale = alpha != 1.0, accumulate = beta != 0.0;  // uniform: decided once
   if (!DFT_OUT && !scale && !accumulate) {
     // Q = Z 2^-(s+f): a loop of its own, without the FP64 epilogue (instructions predicated off
     // would still be issued to GB300's narrow FP64 pipe)
-    const int i = i0 + tx;
-    for (int b = 0; b < CRT_TJ / 8; ++b) {
-      const int jl = ty + 8 * b, jj = j0 + jl;
-      if (i < n && jj < k) Q[i + (long)jj * ldq] = tile[jl][(tx + (jl >> 2)) & 31];
+    const int t = ty * 32 + tx, ir = t % TI, i = i0 + ir;
+    for (int jl = t / TI; jl < CRT_TJ; jl += 256 / TI) {
+      const int jj = j0 + jl;
+      if (i < n && jj < k) Q[i + (long)jj * ldq] = tile[jl][(ir + (jl >> 2)) & (TI - 1)];
     }
   } else if (!DFT_OUT) {
-    const int i = i0 + tx;
-    for (int b = 0; b < CRT_TJ / 8; ++b) {
-      const int jl = ty + 8 * b, jj = j0 + jl;
+    const int t = ty * 32 + tx, ir = t % TI, i = i0 + ir;
+    for (int jl = t / TI; jl < CRT_TJ; jl += 256 / TI) {
+      const int jj = j0 + jl;
       if (i < n && jj < k) {
         double* qp = Q + i + (long)jj * ldq;
-        double v = tile[jl][(tx + (jl >> 2)) & 31];
+        double v = tile[jl][(ir + (jl >> 2)) & (TI - 1)];
         if (scale) v *= alpha;
         if (accumulate) v = fma(beta, *qp, v);
         *qp = v;
       }
     }
   } else {
-    for (int a = 0; a < CRT_TI / 8; ++a) {
+    for (int a = 0; a < TI / 8; ++a) {
       const int il = ty + 8 * a, i = i0 + il;
       if (i >= n) continue;
 #pragma unroll
@@ -1947,7 +2043,7 @@ __device__ __forceinline__ void crt_combine_blk(const int8_t* __restrict__ R, in
         const int jj = jb + c, hc = dft_col(jj, k, kr);
         if (hc < 0) continue;
         double* qp = Q + (long)i * ldq + 2 * hc + (jj >= (kr >> 1) ? 1 : 0);
-        double v = tile[4 * tx + c][(il + tx) & 31];
+        double v = tile[4 * tx + c][(il + tx) & (TI - 1)];
         if (scale) v *= alpha;
         if (accumulate) v = fma(beta, *qp, v);
         *qp = v;
@@ -1966,6 +2062,16 @@ __global__ void __launch_bounds__(256, 3) k_crt_combine(const int8_t* __restrict
   if (gated_off(gate)) return;
   crt_combine_blk<DFT_OUT, TOP32>(R, n, k, kr, cc, amax_bits, hmax_bits, prm, alpha, beta, Q, ldq, blockIdx.x,
                                   by0 + blockIdx.y);
+}
+
+// The same in tiles of eight rows, for outputs of few 32-row tiles (1000 x 777: 224 blocks, 26 us).
+template <bool TOP32>
+__global__ void __launch_bounds__(256, 3) k_crt_combine8(const int8_t* __restrict__ R, int n, int k, int kr, CrtConsts cc,
+                                                      const unsigned long long* __restrict__ amax_bits,
+                                                      const unsigned long long* __restrict__ hmax_bits,
+                                                      const SplitDevParams* prm, double alpha, double beta,
+                                                      double* __restrict__ Q, long ldq) {
+  crt_combine_blk<false, TOP32, 8>(R, n, k, kr, cc, amax_bits, hmax_bits, prm, alpha, beta, Q, ldq, blockIdx.x, blockIdx.y);
 }
 
 // The recombination of the block-recursive products (group exponents unless prm->hbad).
@@ -2321,32 +2427,54 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
   const CrtConsts cc = get_consts(nmod);
 
   if (!gate) prof_begin(stream);
-  if (cudaMemsetAsync(w, 0, L.off_wtab, stream) != cudaSuccess) return PSMMA_EDEVICE;  // params, maxima, sums
-
-  // ---- A side: row maxima and norms
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return PSMMA_EDEVICE;
-  int rst = launch_row_stats(A, lda, M, K, b.amax, b.asq, sms, stream, gate);
-  if (rst) return rst;
-  prof_mark(stream, "row_scale");
-  // ---- H side: generate, column maxima / sums / norms
-  switch (gs.kind) {
-    case KIND_CAUCHY: k_h_pass1<KIND_CAUCHY><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
-    case KIND_TOEPLITZ: k_h_pass1<KIND_TOEPLITZ><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
-    case KIND_HANKEL: k_h_pass1<KIND_HANKEL><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
-    case KIND_DENSE: k_h_pass1<KIND_DENSE><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
-    case KIND_CAUCHY_EIG: k_h_pass1<KIND_CAUCHY_EIG><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
-    default: return PSMMA_EUNSUPPORTED;
+  if (!gate && small_operands(M, N, K)) {
+    const int blocks = N + (M + SMALL_RB - 1) / SMALL_RB;
+    switch (gs.kind) {
+#define PSMMA_STATS(KD) \
+  case KD: k_split_stats<KD><<<blocks, 256, 0, stream>>>(gs, M, N, K, L.kp, A, lda, b.amax, b.asq, b.Ht, b.hmax, b.hsum, b.hsq); break;
+      PSMMA_STATS(KIND_CAUCHY)
+      PSMMA_STATS(KIND_TOEPLITZ)
+      PSMMA_STATS(KIND_HANKEL)
+      PSMMA_STATS(KIND_DENSE)
+      PSMMA_STATS(KIND_CAUCHY_EIG)
+#undef PSMMA_STATS
+      default: return PSMMA_EUNSUPPORTED;
+    }
+    prof_mark(stream, "statistics");
+    const int a_blocks = (L.kp / 64) * ((M + 63) / 64), h_blocks = (N * (L.kp / 4) + 255) / 256;
+    const bool in_line = M + N <= INLINE_ROWS;
+    if (!in_line) k_split_small_params<<<1, 512, 0, stream>>>(cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsum, b.hsq, b.prm);
+    (in_line ? k_split_residues<true> : k_split_residues<false>)<<<a_blocks + h_blocks, 256, 0, stream>>>(
+        A, lda, M, N, K, L.kp, b.amax, b.asq, b.hmax, b.hsum, b.hsq, a_blocks, b.Ht, cc, b.RA, b.RH, b.prm);
+    prof_mark(stream, "residues");
+  } else {
+    if (cudaMemsetAsync(w, 0, L.off_wtab, stream) != cudaSuccess) return PSMMA_EDEVICE;  // params, maxima, sums
+
+    // ---- A side: row maxima and norms
+    int rst = launch_row_stats(A, lda, M, K, b.amax, b.asq, sms, stream, gate);
+    if (rst) return rst;
+    prof_mark(stream, "row_scale");
+    // ---- H side: generate, column maxima / sums / norms
+    switch (gs.kind) {
+      case KIND_CAUCHY: k_h_pass1<KIND_CAUCHY><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
+      case KIND_TOEPLITZ: k_h_pass1<KIND_TOEPLITZ><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
+      case KIND_HANKEL: k_h_pass1<KIND_HANKEL><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
+      case KIND_DENSE: k_h_pass1<KIND_DENSE><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
+      case KIND_CAUCHY_EIG: k_h_pass1<KIND_CAUCHY_EIG><<<N, 256, 0, stream>>>(gs, K, L.kp, b.Ht, b.hmax, b.hsum, b.hsq, b.prm, gate); break;
+      default: return PSMMA_EUNSUPPORTED;
+    }
+    prof_mark(stream, "h_generate");
+    k_split_params<<<params_blocks(M, N), 512, 0, stream>>>(b.prm, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsq, gate);
+    prof_mark(stream, "params");
+    k_residues_A<<<dim3(L.kp / 64, (M + 63) / 64), 256, 0, stream>>>(A, lda, M, K, L.kp, b.amax, b.prm, cc, b.RA, gate);
+    prof_mark(stream, "residues_A");
+    k_residues_H<<<dim3(gate ? std::min(N, 512) : N, rh_blocks_x(L.kp)), 128, 0, stream>>>(b.Ht, N, L.kp, b.hmax, b.prm, cc,
+                                                                                        b.RH, gate);
+    prof_mark(stream, "residues_H");
   }
-  prof_mark(stream, "h_generate");
-  k_split_params<<<params_blocks(M, N), 512, 0, stream>>>(b.prm, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsq, gate);
-  prof_mark(stream, "params");
-  k_residues_A<<<dim3(L.kp / 64, (M + 63) / 64), 256, 0, stream>>>(A, lda, M, K, L.kp, b.amax, b.prm, cc, b.RA, gate);
-  prof_mark(stream, "residues_A");
-  k_residues_H<<<dim3(gate ? std::min(N, 512) : N, rh_blocks_x(L.kp)), 128, 0, stream>>>(b.Ht, N, L.kp, b.hmax, b.prm, cc,
-                                                                                      b.RH, gate);
-  prof_mark(stream, "residues_H");
 
   OneGemm og;
   memset(&og, 0, sizeof(og));
@@ -2373,8 +2501,12 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
   prof_mark(stream, "modular_gemm");
 
   dim3 gc((N + CRT_TJ - 1) / CRT_TJ, (M + CRT_TI - 1) / CRT_TI);
-  (cc.top32 ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, stream>>>(
-      b.R, M, N, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq, 0, gate);
+  if (!gate && (long)gc.x * gc.y < 4L * sms)
+    (cc.top32 ? k_crt_combine8<true> : k_crt_combine8<false>)<<<dim3(gc.x, (M + 7) / 8), dim3(32, 8), 0, stream>>>(
+        b.R, M, N, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq);
+  else
+    (cc.top32 ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, stream>>>(
+        b.R, M, N, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq, 0, gate);
   prof_mark(stream, "crt_combine");
   if (cudaGetLastError() != cudaSuccess) return PSMMA_EDEVICE;
 

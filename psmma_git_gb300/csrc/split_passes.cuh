@@ -123,6 +123,78 @@ __device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, lon
   }
 }
 
+// Small operands (M + N at most SMALL_ROWS, K at most SMALL_K): the statistics of A's rows and H's columns are one
+// launch, the residues of both another; up to INLINE_ROWS the latter's blocks each evaluate the parameters for
+// themselves (at 1024 + 1024 that costs more than a launch of one block between the two).  Their passes
+// take a few microseconds each, so that the launches set the time (CauchyEig n = 256 on the split precision
+// 73 us in nine launches, 47 in five; 1000 x 777 126 and 105).
+constexpr int SMALL_ROWS = 2048, SMALL_K = 1024, INLINE_ROWS = 1024;
+inline bool small_operands(int M, int N, int K) { return M + N <= SMALL_ROWS && K <= SMALL_K; }
+constexpr int SMALL_RB = 32;  // rows of A a statistics block covers, 256 threads
+
+// Row maxima, squared norms (and lowest bits) of rows 32 b .. 32 b + 31 over all of K, not accumulated into
+// what was there: warp w takes columns w, w + 8, ...
+template <bool LSB>
+__device__ __forceinline__ void small_rows_blk(const double* __restrict__ A, long lda, int n, int k, int b,
+                                               unsigned long long* __restrict__ amax_bits, double* __restrict__ asq,
+                                               int* __restrict__ alsb) {
+  __shared__ unsigned long long sm[8][32];
+  __shared__ double sq[8][32];
+  __shared__ int sl[8][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, i = b * 32 + lane;
+  unsigned long long mb = 0;
+  float s32 = 0.0f;
+  int e = NO_SCALE, lsb = NO_LSB;
+  bool big = false;
+  for (int k0 = wid; k0 < k; k0 += 64) {
+    unsigned long long v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int kk = k0 + 8 * u;
+      v[u] = (i < n && kk < k) ? (unsigned long long)__double_as_longlong(__ldg(A + i + (long)kk * lda)) & ABS_MASK : 0ull;
+    }
+    unsigned long long gm = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) gm = v[u] > gm ? v[u] : gm;
+    mb = gm > mb ? gm : mb;
+    if constexpr (LSB) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) lsb = v[u] ? min(lsb, lsb_exp(v[u])) : lsb;
+    }
+    if (e == NO_SCALE && gm) e = (int)(gm >> 52) - 1023;
+    if (e != NO_SCALE) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float f = abs_scaled_up(v[u], e, &big);
+        s32 = __fmaf_ru(f, f, s32);
+      }
+    }
+  }
+  double q = 0.0;
+  if (big) {  // entries 2^56 times the thread's first ones (or Inf/NaN): FP64 sum
+    for (int kk = wid; kk < k; kk += 8) {
+      const double x = i < n ? __ldg(A + i + (long)kk * lda) : 0.0;
+      q = fma(x, x, q);
+    }
+  } else if (e != NO_SCALE) {
+    q = ldexp((double)s32, 2 * e);
+  }
+  sm[wid][lane] = mb;
+  sq[wid][lane] = q;
+  if constexpr (LSB) sl[wid][lane] = lsb;
+  __syncthreads();
+  if (wid == 0 && i < n) {
+    for (int w = 1; w < 8; ++w) {
+      mb = sm[w][lane] > mb ? sm[w][lane] : mb;
+      q += sq[w][lane];
+      if constexpr (LSB) lsb = min(lsb, sl[w][lane]);
+    }
+    amax_bits[i] = mb;
+    asq[i] = q;
+    if constexpr (LSB) alsb[i] = lsb;
+  }
+}
+
 // floor(log2 x) from the bits of a positive finite double, on the integer pipe (GB300's FP64
 // pipe is narrow, and the library ilogb goes through it).
 __device__ __forceinline__ int ilogb_bits(unsigned long long b) {
@@ -278,62 +350,77 @@ __device__ __forceinline__ void h_pass1_blk(const GenSpec& gs, int K, int kp, do
       s2_32 = __fmaf_ru(f, f, s2_32);
     }
   }
-  double s = 0.0, s2 = 0.0;
-  if (big) {  // entries 2^56 times the thread's first one (or Inf/NaN): FP64 sums
-    for (int kk = threadIdx.x; kk < srows; kk += blockDim.x) {
-      const double h = row[kk];
-      s += fabs(h);
-      s2 = fma(h, h, s2);
-    }
-  } else if (e != NO_SCALE) {
-    s = ldexp((double)s32, e);
-    s2 = ldexp((double)s2_32, 2 * e);
-  }
+  // Block maximum first; then every thread's sums on its exponent (round-up FP32: the FP64 pipe's two lanes
+  // made the former FP64 reductions and ldexps some 3000 cycles a column).
   __shared__ unsigned long long smax[32], smax_all[32];
-  __shared__ double ssum[32], ssq[32];
+  __shared__ float ssum[32], ssq[32];
   __shared__ int slsb[32];
+  const int wid = threadIdx.x >> 5, ln = threadIdx.x & 31, nw = blockDim.x >> 5;
   if constexpr (LSB) {
     lsb = __reduce_min_sync(0xffffffffu, lsb);
-    if ((threadIdx.x & 31) == 0) slsb[threadIdx.x >> 5] = lsb;
+    if (ln == 0) slsb[wid] = lsb;
   }
   for (int o = 16; o > 0; o >>= 1) {
-    unsigned long long ob = __shfl_xor_sync(0xffffffffu, mb, o);
+    const unsigned long long ob = __shfl_xor_sync(0xffffffffu, mb, o);
     mb = ob > mb ? ob : mb;
-    ob = __shfl_xor_sync(0xffffffffu, mb_all, o);
-    mb_all = ob > mb_all ? ob : mb_all;
-    s += __shfl_xor_sync(0xffffffffu, s, o);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
   }
-  int wid = threadIdx.x >> 5, ln = threadIdx.x & 31;
-  if (ln == 0) { smax[wid] = mb; smax_all[wid] = mb_all; ssum[wid] = s; ssq[wid] = s2; }
-  __syncthreads();
-  if (wid == 0) {
-    int nw = blockDim.x >> 5;
-    mb = ln < nw ? smax[ln] : 0ull;
-    mb_all = ln < nw ? smax_all[ln] : 0ull;
-    s = ln < nw ? ssum[ln] : 0.0;
-    s2 = ln < nw ? ssq[ln] : 0.0;
+  if (hmax_all) {
     for (int o = 16; o > 0; o >>= 1) {
-      unsigned long long ob = __shfl_xor_sync(0xffffffffu, mb, o);
-      mb = ob > mb ? ob : mb;
-      ob = __shfl_xor_sync(0xffffffffu, mb_all, o);
+      const unsigned long long ob = __shfl_xor_sync(0xffffffffu, mb_all, o);
       mb_all = ob > mb_all ? ob : mb_all;
-      s += __shfl_xor_sync(0xffffffffu, s, o);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     }
-    if (ln == 0) {
-      if (hmax_all) hmax_all[j] = mb_all;
-      hmax_bits[j] = mb;
-      hsum[j] = s;
-      hsq[j] = s2;
-      if constexpr (LSB) {
-        for (int w2 = 1; w2 < nw; ++w2) lsb = min(lsb, slsb[w2]);
-        hlsb[j] = lsb;
+  }
+  if (ln == 0) {
+    smax[wid] = mb;
+    smax_all[wid] = mb_all;
+  }
+  __syncthreads();
+  unsigned long long bm = 0;
+  for (int w2 = 0; w2 < nw; ++w2) bm = smax[w2] > bm ? smax[w2] : bm;
+  const int eb = (int)(bm >> 52) - 1023;
+  float fs = 0.0f, fq = 0.0f;  // sums of |h| 2^-eb and h^2 2^-2eb, below 2 k and 4 k
+  if (bm < INF_BITS) {
+    if (big) {  // entries 2^56 times the thread's first one: FP64 sums
+      double s = 0.0, s2 = 0.0;
+      for (int kk = threadIdx.x; kk < srows; kk += blockDim.x) {
+        const double h = ldexp(row[kk], -eb);
+        s += fabs(h);
+        s2 = fma(h, h, s2);
       }
-      if (prm != nullptr && mb > 0 && mb < INF_BITS && isfinite(s)) {
-        double rho = s / __longlong_as_double((long long)mb);
-        atomicMax(&prm->rho_bits, (unsigned long long)__double_as_longlong(rho));
-      }
+      fs = __double2float_ru(s);
+      fq = __double2float_ru(s2);
+    } else if (e != NO_SCALE) {
+      const int d = max(e - eb, -126), d2 = max(2 * (e - eb), -126);  // e <= eb
+      fs = __fmul_ru(s32, __uint_as_float((unsigned)(127 + d) << 23));
+      fq = __fmul_ru(s2_32, __uint_as_float((unsigned)(127 + d2) << 23));
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    fs = __fadd_ru(fs, __shfl_xor_sync(0xffffffffu, fs, o));
+    fq = __fadd_ru(fq, __shfl_xor_sync(0xffffffffu, fq, o));
+  }
+  if (ln == 0) {
+    ssum[wid] = fs;
+    ssq[wid] = fq;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w2 = 1; w2 < nw; ++w2) {
+      fs = __fadd_ru(fs, ssum[w2]);
+      fq = __fadd_ru(fq, ssq[w2]);
+      mb_all = smax_all[w2] > mb_all ? smax_all[w2] : mb_all;
+      if constexpr (LSB) lsb = min(lsb, slsb[w2]);
+    }
+    if (hmax_all) hmax_all[j] = mb_all;
+    hmax_bits[j] = bm;
+    const bool finite = bm < INF_BITS;
+    hsum[j] = finite ? ldexp((double)fs, eb) : __longlong_as_double((long long)bm);
+    hsq[j] = finite ? ldexp((double)fq, 2 * eb) : __longlong_as_double((long long)bm);
+    if constexpr (LSB) hlsb[j] = lsb;
+    if (prm != nullptr && bm > 0 && finite) {
+      const float m = __uint_as_float(0x3F800000u | ((unsigned)(bm >> 29) & 0x7FFFFFu));
+      const double rho = bm >> 52 ? (double)__fdiv_ru(fs, m) : (double)srows;
+      atomicMax(&prm->rho_bits, (unsigned long long)__double_as_longlong(rho));
     }
   }
 }
