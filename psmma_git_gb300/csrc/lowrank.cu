@@ -107,15 +107,122 @@ __device__ double block_sum(double x, double* sm) {
   return r;
 }
 
-// CauchyMax (Cauchylowrank.f90:166-188): max_i |u(i) / (D(i) - f)| over i in [0, len) and its
-// 1-based index.
-__device__ ArgMax cauchy_max(const double* D, double f, const double* u, int len, ArgMax* sm) {
+// ---- maxima of quotients ---------------------------------------------------------------------
+// The pivot searches compare |u / x| in FP64, and a division is some ten instructions on GB300's two-lane FP64
+// pipe, one SM per block of the merge level: that pipe bounded the compression.  qkey orders the quotients from
+// their exponents and FP32 mantissas with an error of at most two units (2^-19 each); only quotients within
+// QK_SLACK units of the largest key are divided and compared in FP64 -- one or two of thousands -- and the result
+// is the full search's, ties included.  64 blocks of 2048 x 2048: 4244 us with every quotient divided, 1608 us so.
+// QK_EXACT: zero, subnormal or not finite operands and far exponents, always divided.
+constexpr int QK_EXACT = -0x70000000, QK_SLACK = 6;
+__device__ __forceinline__ int qkey(double u, double x) {
+  const unsigned hu = (unsigned)__double2hiint(u), hx = (unsigned)__double2hiint(x);
+  const int eu = (int)(hu >> 20) & 0x7FF, ex = (int)(hx >> 20) & 0x7FF;
+  if (eu == 0 || eu == 0x7FF || ex == 0 || ex == 0x7FF || abs(eu - ex) > 900) return QK_EXACT;
+  const float mu = __uint_as_float(0x3F800000u | ((hu << 3) & 0x7FFFF8u) | ((unsigned)__double2loint(u) >> 29));
+  const float mx = __uint_as_float(0x3F800000u | ((hx << 3) & 0x7FFFF8u) | ((unsigned)__double2loint(x) >> 29));
+  return ((eu - ex) << 19) + (int)(__float_as_uint(__fdividef(mu, mx)) >> 4);
+}
+// The key of (a quotient with key k) times |w|; QK_EXACT as above, and where the product may leave the normal range.
+__device__ __forceinline__ int qkey_times(int k, double w) {
+  const unsigned h = (unsigned)__double2hiint(w);
+  const int e = (int)(h >> 20) & 0x7FF;
+  const int ep = (k >> 19) - 127 + e - 1023;
+  if (k == QK_EXACT || e == 0 || e == 0x7FF || abs(ep) > 1000) return QK_EXACT;
+  const float m = __uint_as_float(0x3F800000u | ((unsigned)(k & 0x7FFFF) << 4));
+  const float mw = __uint_as_float(0x3F800000u | ((h << 3) & 0x7FFFF8u) | ((unsigned)__double2loint(w) >> 29));
+  return (ep << 19) + (int)(__float_as_uint(m * mw) >> 4);
+}
+
+// better() on the bits: the values are -1 or |.|, and a NaN (never better) is passed on as -1.
+__device__ __forceinline__ ArgMax better_bits(ArgMax a, ArgMax b) {
+  const long long x = __double_as_longlong(a.v), y = __double_as_longlong(b.v);
+  return (y > x || (y == x && b.i < a.i)) ? b : a;
+}
+__device__ __forceinline__ ArgMax warp_argmax(ArgMax x) {
+  for (int o = 16; o > 0; o >>= 1) {
+    ArgMax y;
+    y.v = __shfl_xor_sync(0xffffffffu, x.v, o);
+    y.i = __shfl_xor_sync(0xffffffffu, x.i, o);
+    x = better_bits(x, y);
+  }
+  return x;
+}
+__device__ __forceinline__ ArgMax quotient(double u, double x, int i) {
+  const double v = fabs(u / x);
+  return ArgMax{__double_as_longlong(v) > 0x7FF0000000000000ll ? -1.0 : v, i};
+}
+
+// Shared words of a block's searches.  A search writes `key`, synchronises, reads it, writes `best`,
+// synchronises, writes best[32], synchronises: the next one's writes are behind every earlier read.
+struct SearchSm {
+  int key[32];
+  ArgMax best[33];
+};
+
+// max_i |u(i) / x(i)| over i in [0, len) and its smallest 1-based index; the whole block.
+template <class X>
+__device__ ArgMax max_quotient(const double* u, X x, int len, SearchSm& sm) {
+  const int wid = threadIdx.x >> 5, ln = threadIdx.x & 31, nw = blockDim.x >> 5;
+  int km = QK_EXACT;
   ArgMax best{-1.0, 0x7fffffff};
   for (int i = threadIdx.x; i < len; i += blockDim.x) {
-    const double v = fabs(u[i] / (D[i] - f));
-    best = better(best, ArgMax{v, i + 1});
+    const double xi = x(i);
+    const int k = qkey(u[i], xi);
+    if (k == QK_EXACT) best = better_bits(best, quotient(u[i], xi, i + 1));
+    km = max(km, k);
   }
-  return block_argmax(best, sm);
+  km = __reduce_max_sync(0xffffffffu, km);
+  if (ln == 0) sm.key[wid] = km;
+  __syncthreads();
+  km = __reduce_max_sync(0xffffffffu, ln < nw ? sm.key[ln] : QK_EXACT);
+  if (km != QK_EXACT)
+    for (int i = threadIdx.x; i < len; i += blockDim.x) {
+      const double xi = x(i);
+      const int k = qkey(u[i], xi);
+      if (k != QK_EXACT && k >= km - QK_SLACK) best = better_bits(best, quotient(u[i], xi, i + 1));
+    }
+  best = warp_argmax(best);
+  if (ln == 0) sm.best[wid] = best;
+  __syncthreads();
+  if (wid == 0) {
+    best = warp_argmax(ln < nw ? sm.best[ln] : ArgMax{-1.0, 0x7fffffff});
+    if (ln == 0) sm.best[32] = best;
+  }
+  __syncthreads();
+  return sm.best[32];
+}
+
+// The same by one warp; *key receives the largest key (QK_EXACT if some quotient has none).  Quotients are
+// divided only where the key reaches `floor_key` after the product with |w| (a column that cannot win).
+template <class X>
+__device__ __forceinline__ ArgMax warp_max_quotient(const double* u, X x, int i0, int len, double w, int floor_key, int* key) {
+  const int lane = threadIdx.x & 31;
+  int km = QK_EXACT;
+  bool special = false;
+  for (int i = i0 + lane; i < len; i += 32) {
+    const int k = qkey(u[i], x(i));
+    special |= k == QK_EXACT;
+    km = max(km, k);
+  }
+  km = __reduce_max_sync(0xffffffffu, km);
+  special = __any_sync(0xffffffffu, special);
+  const int kw = special ? QK_EXACT : qkey_times(km, w);
+  *key = kw;
+  ArgMax a{-1.0, 0x7fffffff};
+  if (kw != QK_EXACT && floor_key != QK_EXACT && kw < floor_key) return a;
+  for (int i = i0 + lane; i < len; i += 32) {
+    const double xi = x(i);
+    const int k = qkey(u[i], xi);
+    if (k == QK_EXACT || k >= km - QK_SLACK) a = better_bits(a, quotient(u[i], xi, i - i0 + 1));
+  }
+  return warp_argmax(a);
+}
+
+// CauchyMax (Cauchylowrank.f90:166-188): max_i |u(i) / (D(i) - f)| over i in [0, len) and its
+// 1-based index.
+__device__ ArgMax cauchy_max(const double* D, double f, const double* u, int len, SearchSm& sm) {
+  return max_quotient(u, [=](int i) { return D[i] - f; }, len, sm);
 }
 
 __device__ __forceinline__ void swapd(double* a, int i, int j) {
@@ -130,7 +237,7 @@ __device__ __forceinline__ void swapi(int* a, int i, int j) {
 }
 
 // CauchyPivtG (:191-243), 0-based k0 = k - 1.
-__device__ void pivt_g(RrluBlock& b, int k0, ArgMax* sm) {
+__device__ void pivt_g(RrluBlock& b, int k0, SearchSm& sm) {
   const int M = b.M, N = b.N;
   ArgMax L = cauchy_max(b.D + k0, b.F[k0], b.U + k0, M - k0, sm);
   ArgMax R = cauchy_max(b.F + k0, b.D[k0], b.V + k0, N - k0, sm);
@@ -138,6 +245,7 @@ __device__ void pivt_g(RrluBlock& b, int k0, ArgMax* sm) {
   double junkU = R.v * fabs(b.U[k0]);
   const double piv = fabs(b.U[k0] * b.V[k0] / (b.D[k0] - b.F[k0]));
   if (junkL <= piv && junkU <= piv) return;
+  __syncthreads();  // every thread has read the pivot before thread 0 swaps it away
   int flg = junkL > junkU ? 1 : 0;
   int jjL = L.i, jjU = R.i;
   for (int guard = 0; guard < 4 * (M + N); ++guard) {
@@ -187,15 +295,14 @@ __device__ Cand multi_cauchy_max(const double* D, const double* u, int len, cons
                                  int nc, Cand* smc) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   Cand wb{-1.0, 0x7fffffff, 0};
+  int floor_key = QK_EXACT;  // below it a column cannot beat one this warp has seen
   for (int j = warp; j < nc; j += nw) {
     const double pj = P[j];
-    ArgMax a{-1.0, 0x7fffffff};
-    for (int i = lane; i < len; i += 32) a = better(a, ArgMax{fabs(u[i] / (D[i] - pj)), i + 1});
-    for (int o = 16; o > 0; o >>= 1) {
-      ArgMax y;
-      y.v = __shfl_xor_sync(0xffffffffu, a.v, o);
-      y.i = __shfl_xor_sync(0xffffffffu, a.i, o);
-      a = better(a, y);
+    int key;
+    const ArgMax a = warp_max_quotient(u, [=](int i) { return D[i] - pj; }, 0, len, Wt[j], floor_key, &key);
+    if (key != QK_EXACT) {
+      if (floor_key != QK_EXACT && key < floor_key) continue;
+      floor_key = max(floor_key, key - 2 * QK_SLACK);
     }
     wb = better_c(wb, Cand{a.v * fabs(Wt[j]), j + 1, a.i});
   }
@@ -231,7 +338,7 @@ __device__ void apply_cp(RrluBlock& b, int k0, int ii, int jj) {
 // search (CauchyPivtG_CP): a step whose pivot is below tol * amax saves its state, counts
 // itself in *pending and returns; the search runs grid-wide and the next launch resumes.
 __global__ void __launch_bounds__(RRLU_THREADS) k_rrlu_cauchy(RrluBlock* blocks, double tol, int* pending) {
-  __shared__ ArgMax sm[33];
+  __shared__ SearchSm sm;
   __shared__ Cand smc[33];
   RrluBlock& gb = blocks[blockIdx.x];
   RrluBlock b = gb;
@@ -356,15 +463,14 @@ __global__ void __launch_bounds__(RRLU_THREADS) k_cp_search(const RrluBlock* blo
   const int k0 = b.k_next - 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   Cand wb{-1.0, 0x7fffffff, 0};
+  int floor_key = QK_EXACT;
   for (int j = ch.c0 + warp; j < ch.c1; j += nw) {
     const double pj = b.F[j];
-    ArgMax a{-1.0, 0x7fffffff};
-    for (int i = k0 + lane; i < b.M; i += 32) a = better(a, ArgMax{fabs(b.U[i] / (b.D[i] - pj)), i - k0 + 1});
-    for (int o = 16; o > 0; o >>= 1) {
-      ArgMax y;
-      y.v = __shfl_xor_sync(0xffffffffu, a.v, o);
-      y.i = __shfl_xor_sync(0xffffffffu, a.i, o);
-      a = better(a, y);
+    int key;
+    const ArgMax a = warp_max_quotient(b.U, [&](int i) { return b.D[i] - pj; }, k0, b.M, b.V[j], floor_key, &key);
+    if (key != QK_EXACT) {
+      if (floor_key != QK_EXACT && key < floor_key) continue;
+      floor_key = max(floor_key, key - 2 * QK_SLACK);
     }
     wb = better_c(wb, Cand{a.v * fabs(b.V[j]), j - k0 + 1, a.i});
   }
@@ -421,20 +527,14 @@ __device__ __forceinline__ double eig_dd(const RrluEigBlock& b, int pj, int pk) 
 }
 
 // CauchyMaxEigmc (:1506-1589): max_i |U(i) / (F(PL(i)) - D(PU(k0)))|, i in [k0, M), 1-based offset
-__device__ ArgMax eig_col_max(const RrluEigBlock& b, int k0, ArgMax* sm) {
-  ArgMax best{-1.0, 0x7fffffff};
+__device__ ArgMax eig_col_max(const RrluEigBlock& b, int k0, SearchSm& sm) {
   const int pu = b.PU[k0];
-  for (int i = k0 + threadIdx.x; i < b.M; i += blockDim.x)
-    best = better(best, ArgMax{fabs(b.U[i] / eig_fd(b, b.PL[i], pu)), i - k0 + 1});
-  return block_argmax(best, sm);
+  return max_quotient(b.U + k0, [&](int i) { return eig_fd(b, b.PL[k0 + i], pu); }, b.M - k0, sm);
 }
 // CauchyMaxEigm (:1418-1503): max_j |V(j) / (F(PL(k0)) - D(PU(j)))|, j in [k0, N)
-__device__ ArgMax eig_row_max(const RrluEigBlock& b, int k0, ArgMax* sm) {
-  ArgMax best{-1.0, 0x7fffffff};
+__device__ ArgMax eig_row_max(const RrluEigBlock& b, int k0, SearchSm& sm) {
   const int pl = b.PL[k0];
-  for (int j = k0 + threadIdx.x; j < b.N; j += blockDim.x)
-    best = better(best, ArgMax{fabs(b.V[j] / eig_fd(b, pl, b.PU[j])), j - k0 + 1});
-  return block_argmax(best, sm);
+  return max_quotient(b.V + k0, [&](int j) { return eig_fd(b, pl, b.PU[k0 + j]); }, b.N - k0, sm);
 }
 
 __device__ __forceinline__ void eig_swap_rows(RrluEigBlock& b, int a, int c) {
@@ -450,13 +550,14 @@ __device__ __forceinline__ void eig_swap_cols(RrluEigBlock& b, int a, int c) {
 }
 
 // CauchyPivtEig (:571-717); the pivot magnitude is |U(k)V(k) / computfd(k, k)|.
-__device__ void pivt_eig(RrluEigBlock& b, int k0, ArgMax* sm) {
+__device__ void pivt_eig(RrluEigBlock& b, int k0, SearchSm& sm) {
   ArgMax L = eig_col_max(b, k0, sm);
   ArgMax R = eig_row_max(b, k0, sm);
   const double junkL = L.v * fabs(b.V[k0]);
   const double junkU = R.v * fabs(b.U[k0]);
   const double piv = fabs(b.U[k0] * b.V[k0] / eig_fd(b, b.PL[k0], b.PU[k0]));
   if (junkL <= piv && junkU <= piv) return;
+  __syncthreads();  // every thread has read the pivot before thread 0 swaps it away
   int flg = junkL > junkU ? 1 : 0;
   int jjL = L.i, jjU = R.i;
   for (int guard = 0; guard < 4 * (b.M + b.N); ++guard) {
@@ -478,7 +579,7 @@ __device__ void pivt_eig(RrluEigBlock& b, int k0, ArgMax* sm) {
 }
 
 __global__ void __launch_bounds__(RRLU_THREADS) k_rrlu_eig(RrluEigBlock* blocks, double tol, int* pending) {
-  __shared__ ArgMax sm[33];
+  __shared__ SearchSm sm;
   __shared__ Cand smc[33];
   RrluEigBlock& gb = blocks[blockIdx.x];
   RrluEigBlock b = gb;
@@ -599,15 +700,15 @@ __global__ void __launch_bounds__(RRLU_THREADS) k_cp_search_eig(const RrluEigBlo
   const int k0 = b.k_next - 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   Cand wb{-1.0, 0x7fffffff, 0};
+  int floor_key = QK_EXACT;
   for (int j = ch.c0 + warp; j < ch.c1; j += nw) {
     const int pu = b.PU[j];
-    ArgMax a{-1.0, 0x7fffffff};
-    for (int i = k0 + lane; i < b.M; i += 32) a = better(a, ArgMax{fabs(b.U[i] / eig_fd(b, b.PL[i], pu)), i - k0 + 1});
-    for (int o = 16; o > 0; o >>= 1) {
-      ArgMax y;
-      y.v = __shfl_xor_sync(0xffffffffu, a.v, o);
-      y.i = __shfl_xor_sync(0xffffffffu, a.i, o);
-      a = better(a, y);
+    int key;
+    const ArgMax a =
+        warp_max_quotient(b.U, [&](int i) { return eig_fd(b, b.PL[i], pu); }, k0, b.M, b.V[j], floor_key, &key);
+    if (key != QK_EXACT) {
+      if (floor_key != QK_EXACT && key < floor_key) continue;
+      floor_key = max(floor_key, key - 2 * QK_SLACK);
     }
     wb = better_c(wb, Cand{a.v * fabs(b.V[j]), j - k0 + 1, a.i});
   }
