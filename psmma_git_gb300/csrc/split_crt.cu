@@ -3781,7 +3781,7 @@ int launch_split_general(int M, int N, int K, double alpha, const double* A, lon
 // (enqueue) are then plain kernel launches that a stream capture can record.
 // ------------------------------------------------------------------------------------------
 struct GProb {
-  int M, N, K, kp, kr, bn;
+  int M, N, K, kp, kr, bn, row_chunk;
   double alpha, beta;
   const double* A;
   long lda;
@@ -3812,13 +3812,16 @@ __device__ __forceinline__ int gfind(const GProb* d, int count, int blk) {
   return lo;
 }
 
-constexpr int G_ROW_KCHUNK = 1024;
+// Columns of a row-statistics block: 1024, halved down to 128 while the launch has fewer than 16 blocks per SM of
+// 152 (16 problems up to n = 2900: some 300 chains of 128 loads, 317 us; short chunks 52 us).
+constexpr int G_ROW_KCHUNK = 1024, G_ROW_BLOCKS = 16 * 152;
 
 // Each CTA of a grouped pass kernel walks a run of consecutive logical blocks (one binary
 // search per CTA, then a linear advance across product boundaries): a lookup per logical block
 // (seven dependent loads of the descriptor table before any data moves) had made the small
 // blocks of these passes latency-bound.  Runs per kernel: rows 2, H columns 2, residue and CRT
-// tiles 8, H residue strips 16.
+// tiles 8, H residue strips 16, fewer where that leaves less than 16 CTAs per SM (a batch of small
+// problems then ends in one uneven wave).
 template <int W>
 __device__ __forceinline__ int gkey(const GProb& e) {
   return W == 0 ? e.b_row : W == 1 ? e.b_h : W == 2 ? e.b_ra : W == 3 ? e.b_rh : e.b_crt;
@@ -3839,16 +3842,16 @@ struct GRun {
 };
 constexpr int G_RUN_ROW = 2, G_RUN_H = 2, G_RUN_RA = 8, G_RUN_RH = 16, G_RUN_CRT = 8;
 
-__global__ void __launch_bounds__(128) k_g_row_absmax(const GProb* d, int count, int total) {
-  for (GRun<0> r(d, count, total, G_RUN_ROW); r.b < r.end; ++r.b) {
+__global__ void __launch_bounds__(128) k_g_row_absmax(const GProb* d, int count, int total, int run) {
+  for (GRun<0> r(d, count, total, run); r.b < r.end; ++r.b) {
     const GProb& e = r.owner(d, count);
     const int local = r.b - e.b_row, gx = (e.M + 127) / 128;
-    row_absmax_blk(e.A, e.lda, e.A2, e.lda2, e.ka, e.M, e.K, G_ROW_KCHUNK, e.amax, e.asq, local % gx, local / gx);
+    row_absmax_blk(e.A, e.lda, e.A2, e.lda2, e.ka, e.M, e.K, e.row_chunk, e.amax, e.asq, local % gx, local / gx);
   }
 }
 
-__global__ void __launch_bounds__(256) k_g_h_pass1(const GProb* d, int count, int total) {
-  for (GRun<1> r(d, count, total, G_RUN_H); r.b < r.end; ++r.b) {
+__global__ void __launch_bounds__(256) k_g_h_pass1(const GProb* d, int count, int total, int run) {
+  for (GRun<1> r(d, count, total, run); r.b < r.end; ++r.b) {
     const GProb& e = r.owner(d, count);
     const int j = r.b - e.b_h;
     switch (e.gs.kind) {
@@ -3867,8 +3870,8 @@ __global__ void __launch_bounds__(1024) k_g_split_params(const GProb* d, double 
   split_params_blk(e.prm, log2M, e.M, e.N, e.K, e.amax, e.asq, e.hmax, e.hsq);
 }
 
-__global__ void __launch_bounds__(256) k_g_residues_A(const GProb* d, int count, int total, CrtConsts cc) {
-  for (GRun<2> r(d, count, total, G_RUN_RA); r.b < r.end; ++r.b) {
+__global__ void __launch_bounds__(256) k_g_residues_A(const GProb* d, int count, int total, int run, CrtConsts cc) {
+  for (GRun<2> r(d, count, total, run); r.b < r.end; ++r.b) {
     const GProb& e = r.owner(d, count);
     const int local = r.b - e.b_ra, gx = e.kp / 64;
     residues_A_blk<64>(e.A, e.lda, e.A2, e.lda2, e.ka, e.M, e.K, e.kp, e.amax, e.prm, cc, e.RA, local % gx,
@@ -3877,8 +3880,8 @@ __global__ void __launch_bounds__(256) k_g_residues_A(const GProb* d, int count,
   }
 }
 
-__global__ void __launch_bounds__(128) k_g_residues_H(const GProb* d, int count, int total, CrtConsts cc) {
-  for (GRun<3> r(d, count, total, G_RUN_RH); r.b < r.end; ++r.b) {
+__global__ void __launch_bounds__(128) k_g_residues_H(const GProb* d, int count, int total, int run, CrtConsts cc) {
+  for (GRun<3> r(d, count, total, run); r.b < r.end; ++r.b) {
     const GProb& e = r.owner(d, count);
     const int local = r.b - e.b_rh, gx = rh_blocks_x(e.kp);
     residues_H_blk(e.Ht, e.N, e.kp, e.hmax, e.prm, cc, e.RH, local % gx, local / gx);
@@ -3886,8 +3889,8 @@ __global__ void __launch_bounds__(128) k_g_residues_H(const GProb* d, int count,
 }
 
 template <bool TOP32>
-__global__ void __launch_bounds__(256, 3) k_g_crt_combine(const GProb* d, int count, int total, CrtConsts cc) {
-  for (GRun<4> r(d, count, total, G_RUN_CRT); r.b < r.end; ++r.b) {
+__global__ void __launch_bounds__(256, 3) k_g_crt_combine(const GProb* d, int count, int total, int run, CrtConsts cc) {
+  for (GRun<4> r(d, count, total, run); r.b < r.end; ++r.b) {
     const GProb& e = r.owner(d, count);
     const int local = r.b - e.b_crt, gx = (e.N + CRT_TJ - 1) / CRT_TJ;
     crt_combine_blk<false, TOP32>(e.R, e.M, e.N, e.kr, cc, e.amax, e.hmax, e.prm, e.alpha, e.beta, e.Q, e.ldq,
@@ -3941,13 +3944,20 @@ int plan_group(const SplitProblem* P, int count, int nmod, const SplitTune& tune
   }
   const uintptr_t small1 = (w.off + 1023) & ~(uintptr_t)1023;
   int b_row = 0, b_h = 0, b_ra = 0, b_rh = 0, b_crt = 0;
+  int row_chunk = G_ROW_KCHUNK;
+  for (; row_chunk > 128; row_chunk >>= 1) {
+    long blocks = 0;
+    for (const GProb& e : pr) blocks += (long)((e.M + 127) / 128) * ((e.K + row_chunk - 1) / row_chunk);
+    if (blocks >= G_ROW_BLOCKS) break;
+  }
   for (int i = 0; i < count; ++i) {
     GProb& e = pr[i];
+    e.row_chunk = row_chunk;
     e.Ht = w.take<double>((size_t)e.N * e.kp, 1024);
     e.RA = w.take<__nv_bfloat16>((size_t)nmod * e.M * e.kp, 1024);
     e.RH = w.take<__nv_bfloat16>((size_t)nmod * e.N * e.kp, 1024);
     e.R = w.take<int8_t>((size_t)nmod * e.M * e.kr, 1024);
-    e.b_row = b_row; b_row += ((e.M + 127) / 128) * ((e.K + G_ROW_KCHUNK - 1) / G_ROW_KCHUNK);
+    e.b_row = b_row; b_row += ((e.M + 127) / 128) * ((e.K + row_chunk - 1) / row_chunk);
     e.b_h = b_h;     b_h += e.N;
     e.b_ra = b_ra;   b_ra += (e.kp / 64) * ((e.M + 63) / 64);
     e.b_rh = b_rh;   b_rh += rh_blocks_x(e.kp) * e.N;
@@ -4066,15 +4076,18 @@ int split_group_enqueue(const SplitGroup& g, cudaStream_t stream, unsigned* stat
     return PSMMA_EDEVICE;
   if (cudaMemsetAsync(g.small, 0, g.small_bytes, stream) != cudaSuccess) return PSMMA_EDEVICE;
   auto runs = [](int total, int chunk) { return (unsigned)((total + chunk - 1) / chunk); };
-  if (g.blocks_row > 0) k_g_row_absmax<<<runs(g.blocks_row, G_RUN_ROW), 128, 0, stream>>>(d, g.count, g.blocks_row);
+  auto run_of = [&](int total, int longest) { return std::max(1, std::min(longest, total / (16 * sms))); };
+  const int n_row = run_of(g.blocks_row, G_RUN_ROW), n_h = run_of(g.blocks_h, G_RUN_H), n_ra = run_of(g.blocks_ra, G_RUN_RA),
+            n_rh = run_of(g.blocks_rh, G_RUN_RH), n_crt = run_of(g.blocks_crt, G_RUN_CRT);
+  if (g.blocks_row > 0) k_g_row_absmax<<<runs(g.blocks_row, n_row), 128, 0, stream>>>(d, g.count, g.blocks_row, n_row);
   prof_mark(stream, "g_row_scale");
-  if (g.blocks_h > 0) k_g_h_pass1<<<runs(g.blocks_h, G_RUN_H), 256, 0, stream>>>(d, g.count, g.blocks_h);
+  if (g.blocks_h > 0) k_g_h_pass1<<<runs(g.blocks_h, n_h), 256, 0, stream>>>(d, g.count, g.blocks_h, n_h);
   prof_mark(stream, "g_h_generate");
   k_g_split_params<<<g.count, 1024, 0, stream>>>(d, cc.log2M);
   prof_mark(stream, "g_params");
-  if (g.blocks_ra > 0) k_g_residues_A<<<runs(g.blocks_ra, G_RUN_RA), 256, 0, stream>>>(d, g.count, g.blocks_ra, cc);
+  if (g.blocks_ra > 0) k_g_residues_A<<<runs(g.blocks_ra, n_ra), 256, 0, stream>>>(d, g.count, g.blocks_ra, n_ra, cc);
   prof_mark(stream, "g_residues_A");
-  if (g.blocks_rh > 0) k_g_residues_H<<<runs(g.blocks_rh, G_RUN_RH), 128, 0, stream>>>(d, g.count, g.blocks_rh, cc);
+  if (g.blocks_rh > 0) k_g_residues_H<<<runs(g.blocks_rh, n_rh), 128, 0, stream>>>(d, g.count, g.blocks_rh, n_rh, cc);
   prof_mark(stream, "g_residues_H");
   int st = launch_group_gemm<256>(g, 0, cc, sms, stream);
   prof_mark(stream, "g_gemm_256");
@@ -4084,8 +4097,8 @@ int split_group_enqueue(const SplitGroup& g, cudaStream_t stream, unsigned* stat
   prof_mark(stream, "g_gemm_64");
   if (st) return st;
   if (g.blocks_crt > 0)
-    (cc.top32 ? k_g_crt_combine<true> : k_g_crt_combine<false>)<<<runs(g.blocks_crt, G_RUN_CRT), dim3(32, 8), 0,
-                                                                   stream>>>(d, g.count, g.blocks_crt, cc);
+    (cc.top32 ? k_g_crt_combine<true> : k_g_crt_combine<false>)<<<runs(g.blocks_crt, n_crt), dim3(32, 8), 0,
+                                                                   stream>>>(d, g.count, g.blocks_crt, n_crt, cc);
   prof_mark(stream, "g_crt_combine");
   if (cudaGetLastError() != cudaSuccess) return PSMMA_EDEVICE;
   if (status_out &&
