@@ -57,7 +57,7 @@ struct NttConsts {
   uint2 fold[NT_MAXP];
   u64 inv64[NT_MAXP];                   // floor(2^64 / p)
   // CRT: Z = sum_q X_q W_q - q M, W_q = M / p_q, limbs of 32 bits; G = floor(2^52 / p)
-  u32 W[NT_MAXP][NT_MAXP], M[NT_MAXP], G[NT_MAXP];
+  u32 W[NT_MAXP][NT_MAXP], Mneg[4], G[NT_MAXP];
 };
 
 NttConsts make_ntt(int np, int lg) {
@@ -95,7 +95,16 @@ NttConsts make_ntt(int np, int lg) {
           carry = v >> 32;
         }
       }
-      memcpy(r < 0 ? c.W[q] : c.M, limb, sizeof(limb));
+      if (r < 0) {
+        memcpy(c.W[q], limb, sizeof(limb));
+      } else {  // 2^128 - M (mod 2^128)
+        u64 carry = 1;
+        for (int l = 0; l < 4; ++l) {
+          carry += (u32)~limb[l];
+          c.Mneg[l] = (u32)carry;
+          carry >>= 32;
+        }
+      }
     }
   }
   return c;
@@ -551,14 +560,15 @@ __global__ void __launch_bounds__(512, 2) k_ntt_rows(const __grid_constant__ Ntt
 
 // ------------------------------------------------------------------------------------------
 // CRT: Z = sum_q X_q W_q - round(sum_q X_q / p_q) M in 32-bit limbs (|Z| < 2^126), scaled and rounded as in
-// split_crt.cu; 32 x 128 tiles transposed through shared memory.
+// split_crt.cu; 32 x 128 tiles transposed through shared memory.  8192^2, four primes: 443 -> 329 us with the limbs'
+// sums as the words of Z and four elements of Q in flight.
 // ------------------------------------------------------------------------------------------
 template <int NPR>
 __global__ void __launch_bounds__(256) k_ntt_crt(const __grid_constant__ NttConsts c, const u32* __restrict__ X, int n, int k,
                                                  int kr, const u64* __restrict__ amax, const SplitDevParams* prm,
                                                  const NttParams* t, int slack, double alpha, double beta,
                                                  double* __restrict__ Q, long ldq) {
-  __shared__ double tile[128][32];
+  __shared__ double tile[32][129];  // as crt_combine_blk's
   if (!ntt_ok(t, prm, slack)) return;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 128, jb = j0 + 4 * tx;
@@ -571,57 +581,57 @@ __global__ void __launch_bounds__(256) k_ntt_crt(const __grid_constant__ NttCons
       uint4 w[NPR];
 #pragma unroll
       for (int q = 0; q < NPR; ++q) w[q] = __ldg((const uint4*)(X + ((size_t)q * n + i) * kr + jb));
-      const int e = ab != 0 && ab < INF_BITS ? scale_exp(ab, PA) + ge : 0;
+      const int e = ge + (ab >= INF_BITS ? EXP_NAN : ab == 0 ? EXP_ZERO : scale_exp(ab, PA));
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        u64 acc[NPR];
-#pragma unroll
-        for (int l = 0; l < NPR; ++l) acc[l] = 0;
-        u32 qs = 0;
+        u64 acc[3] = {0, 0, 0};
+        u32 top = 0, qs = 1u << 19;
 #pragma unroll
         for (int q = 0; q < NPR; ++q) {
           const u32 x = v == 0 ? w[q].x : v == 1 ? w[q].y : v == 2 ? w[q].z : w[q].w;
           qs += __umulhi(x, c.G[q]);
 #pragma unroll
-          for (int l = 0; l < NPR; ++l) acc[l] += (u64)x * c.W[q][l];
+          for (int l = 0; l < 3; ++l) acc[l] += (u64)x * c.W[q][l];
+          if (NPR > 4) top += x * c.W[q][3];  // four primes: W_q < 2^90
+          if (NPR > 4 && q == 3) {  // four terms x W[l] stay below 2^64, the fifth would not
+            acc[1] += acc[0] >> 32;
+            acc[0] = (u32)acc[0];
+            top += (u32)(acc[2] >> 32);
+            acc[2] = (u32)acc[2];
+          }
         }
-        const u32 qq = (qs + (1u << 19)) >> 20;
-        long long carry = 0;
-        u32 d[NPR + 1];
-#pragma unroll
-        for (int l = 0; l < NPR; ++l) {
-          // acc < 5 * 2^62 may pass 2^63: split before the signed step
-          const long long z = (long long)(acc[l] & 0xFFFFFFFFull) - (long long)((u64)qq * c.M[l] & 0xFFFFFFFFull) + carry;
-          d[l] = (u32)z;
-          carry = (z >> 32) + (long long)(acc[l] >> 32) - (long long)((u64)qq * c.M[l] >> 32);
-        }
+        const u32 qq = qs >> 20;
+        const u64 z0 = acc[0] + (u64)qq * c.Mneg[0];
+        const u64 z1 = acc[1] + (u64)qq * c.Mneg[1] + (z0 >> 32);
+        const u64 z2 = acc[2] + (u64)qq * c.Mneg[2] + (z1 >> 32);
+        const u32 z3 = top + qq * c.Mneg[3] + (u32)(z2 >> 32);
         // |Z| < 2^126: the low 128 bits in two's complement are Z
-        u64 lo = ((u64)d[1] << 32) | d[0], hi = ((u64)d[3] << 32) | d[2];
-        const bool neg = (long long)hi < 0;
-        if (neg) {
-          lo = ~lo + 1;
-          hi = ~hi + (lo == 0 ? 1 : 0);
-        }
-        if (ab >= INF_BITS)
-          val[v] = __longlong_as_double(0x7FF8000000000000ll);
-        else if (ab != 0)
-          val[v] = u128w_scaled(hi, lo, neg, e);
+        const unsigned __int128 z = ((unsigned __int128)(((u64)z3 << 32) | (u32)z2) << 64) | ((z1 << 32) | (u32)z0);
+        val[v] = i128_scaled((__int128)z, e);
       }
     }
 #pragma unroll
-    for (int v = 0; v < 4; ++v) tile[4 * tx + v][(il + tx) & 31] = val[v];
+    for (int v = 0; v < 4; ++v) tile[tx][v * 32 + il] = val[v];
   }
   __syncthreads();
   const bool scale = alpha != 1.0, accumulate = beta != 0.0;
-  const int i = i0 + tx;
-  for (int b = 0; b < 16; ++b) {
-    const int jl = ty + 8 * b, jj = j0 + jl;
-    if (i < n && jj < k) {
-      double* qp = Q + i + (long)jj * ldq;
-      double v = tile[jl][(tx + (jl >> 2)) & 31];
-      if (scale) v *= alpha;
-      if (accumulate) v = fma(beta, *qp, v);
-      *qp = v;
+  const int i = i0 + tx, left = i < n ? k - j0 : 0;
+  double* qp = Q + i + (long)(j0 + ty) * ldq;
+#pragma unroll
+  for (int b0 = 0; b0 < 16; b0 += 4) {
+    double qv[4];
+    const double* ql = qp;
+#pragma unroll
+    for (int b = 0; b < 4; ++b, ql += 8 * ldq) qv[b] = accumulate && ty + 8 * (b0 + b) < left ? *ql : 0.0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b, qp += 8 * ldq) {
+      const int jl = ty + 8 * (b0 + b);
+      if (jl < left) {
+        double v = tile[jl >> 2][(jl & 3) * 32 + tx];
+        if (scale) v *= alpha;
+        if (accumulate) v = fma(beta, qv[b], v);
+        *qp = v;
+      }
     }
   }
 }

@@ -34,7 +34,7 @@
 
 namespace psmma {
 
-constexpr int SPL_MAX_MODULI = 16;
+constexpr int SPL_MAX_MODULI = 16, CRT_GROUPS = 5, CRT_SLOTS = 16;
 constexpr int SPL_DEFAULT_MODULI = 14;
 // Pairwise coprime: 2^8, 3*5*17, 11*23, 13*19 and primes.
 static const int kModuli[SPL_MAX_MODULI] = {256, 255, 253, 251, 247, 241, 239, 233,
@@ -48,16 +48,18 @@ struct CrtConsts {
   float g23[SPL_MAX_MODULI];  // 2^23 mod m, symmetric (|g| <= m/2)
   float g38[SPL_MAX_MODULI];  // 2^38 mod m, symmetric
   float g14[SPL_MAX_MODULI], g28[SPL_MAX_MODULI], g42[SPL_MAX_MODULI];  // 2^14, 2^28, 2^42 mod m, symmetric
-  unsigned long long C_lo[SPL_MAX_MODULI], C_hi[SPL_MAX_MODULI];  // CRT basis C_l < M
-  float f[SPL_MAX_MODULI];                                        // C_l / M
-  unsigned long long M_lo, M_hi;
   double log2M;
-  unsigned climb[SPL_MAX_MODULI][4];   // C_l as four 32-bit limbs
-  unsigned bias[4];                    // 128 * sum_l C_l mod 2^128 (residues enter offset by 128)
-  int ffix[SPL_MAX_MODULI];            // round(2^19 * C_l / M): fixed-point quotient estimate
-  unsigned long long biasl[4];         // sum_l 128 * climb[l][t], per limb, unreduced
-  unsigned Mlimb[4];                   // M as four 32-bit limbs
-  int top32;                           // sum_l 255 * climb[l][3] < 2^32: top limb summed in 32 bits
+  // Recombination.  The moduli in order form groups of three, the first of four or the last of two where nmod asks for
+  // it (product P).  X_g = sum r_l gc (mod P) is Z W_g^-1 mod P, W_g = M / P, and
+  // Z = sum_g X_g W_g - q M, q the nearest integer to sum_g X_g / P_g.  At most one P exceeds 2^24, so that
+  // sum_g X_g times a 32-bit limb stays below 2^64.
+  int groups, four;                                    // four: the first group has four moduli
+  unsigned gc[CRT_SLOTS], gf[CRT_SLOTS];               // by slot (four, then three a group): c, floor(2^20 c / P)
+  // the sums' starts, so that they are those of r + 128 in [0, 255] and X of their reduction; P, floor(2^47 / P)
+  unsigned gb[CRT_GROUPS], gfb[CRT_GROUPS], gP[CRT_GROUPS], gG[CRT_GROUPS];
+  unsigned gW[CRT_GROUPS][4];                          // W_g in 32-bit limbs
+  unsigned Mneg[4];                                    // 2^128 - M likewise
+  int three;                                           // every W_g below 2^96
 };
 
 // ------------------------------------------------------------------------------------------
@@ -96,36 +98,35 @@ static CrtConsts make_consts(int nmod) {
     c.g14[l] = (float)(g14 > m / 2 ? g14 - m : g14);
     c.g28[l] = (float)(g28 > m / 2 ? g28 - m : g28);
     c.g42[l] = (float)(g42 > m / 2 ? g42 - m : g42);
-    u128 Ml = M / (u128)m;
-    long long Ml_mod = (long long)(Ml % (u128)m);
-    long long y = inv_mod(Ml_mod, m);
-    u128 C = (Ml * (u128)y) % M;
-    c.C_lo[l] = (unsigned long long)C;
-    c.C_hi[l] = (unsigned long long)(C >> 64);
-    // C / M as float: C < M < 2^126, take the top bits of both
-    long double cf = (long double)C / (long double)M;
-    c.f[l] = (float)cf;
   }
-  c.M_lo = (unsigned long long)M;
-  c.M_hi = (unsigned long long)(M >> 64);
   c.log2M = l2 - 1e-9;
-  u128 bias = 0;
-  for (int l = 0; l < nmod; l++) {
-    u128 C = ((u128)c.C_hi[l] << 64) | c.C_lo[l];
-    for (int t = 0; t < 4; t++) c.climb[l][t] = (unsigned)(C >> (32 * t));
-    bias += (u128)128 * C;  // wraps modulo 2^128
-  }
-  for (int t = 0; t < 4; t++) c.bias[t] = (unsigned)(bias >> (32 * t));
-  for (int t = 0; t < 4; t++) c.Mlimb[t] = (unsigned)(M >> (32 * t));
-  for (int t = 0; t < 4; t++) {
-    c.biasl[t] = 0;
-    for (int l = 0; l < nmod; l++) c.biasl[t] += 128ull * c.climb[l][t];
-  }
-  c.top32 = 2 * c.biasl[3] < (1ull << 32);  // 255 <= 2 * 128
-  for (int l = 0; l < nmod; l++) {
-    u128 C = ((u128)c.C_hi[l] << 64) | c.C_lo[l];
-    long double cf = (long double)C / (long double)M;
-    c.ffix[l] = (int)std::llround((double)(cf * 524288.0L));  // |sum_l r_l ffix_l| < 16*128*2^19 = 2^30
+  c.groups = (nmod + 1) / 3;
+  c.four = nmod % 3 == 1;
+  c.three = 1;
+  const u128 neg = (u128)0 - M;
+  for (int t = 0; t < 4; t++) c.Mneg[t] = (unsigned)(neg >> (32 * t));
+  for (int g = 0, first = 0; g < c.groups; g++) {
+    const int size = g == 0 && c.four ? 4 : std::min(3, nmod - first), slot = g == 0 ? 0 : 3 * g + 1;
+    unsigned long long P = 1, bias = 0, fbias = 0;
+    for (int i = 0; i < size; i++) P *= (unsigned long long)kModuli[first + i];
+    const u128 W = M / P;
+    for (int i = 0; i < size; i++) {
+      const long long m = kModuli[first + i], rest = (long long)(P / (unsigned long long)m);
+      const long long y = inv_mod((long long)(W % (u128)m), m) * inv_mod(rest % m, m) % m;
+      const unsigned long long cl = (unsigned long long)(rest * y);
+      c.gc[slot + i] = (unsigned)cl;
+      c.gf[slot + i] = (unsigned)((cl << 20) / P);
+      bias += 128 * cl;
+      fbias += 128ull * c.gf[slot + i];
+    }
+    const unsigned long long b = (P - bias % P) % P;  // takes the 128s out of X again
+    c.gb[g] = (unsigned)(b + bias);
+    c.gfb[g] = (unsigned)((b << 20) / P + fbias);
+    c.gP[g] = (unsigned)P;
+    c.gG[g] = (unsigned)((1ull << 47) / P);
+    for (int t = 0; t < 4; t++) c.gW[g][t] = (unsigned)(W >> (32 * t));
+    c.three = c.three && c.gW[g][3] == 0;
+    first += size;
   }
   return c;
 }
@@ -298,8 +299,8 @@ __global__ void k_h_pass1_all(GenSpec gs, int K, int kp, double* __restrict__ Ht
 
 // Bits PA (rows of A) and PH (columns of H).  The integer product must satisfy
 // |Z_ij| < 0.497 M for the CRT, with M = prod m_l: the symmetric reconstruction needs |Z| < M/2
-// and the quotient estimate (ffix at 2^-19) errs by at most 16 * 128 * 0.5 * 2^-19 < 0.002 of M,
-// a margin of 1.01 bits.  Two rigorous bounds of |Z_ij| =
+// and the quotient estimate (CrtConsts) errs by less than 10 * 2^-15 < 0.0004 of M, a margin
+// of 1.01 bits.  Two rigorous bounds of |Z_ij| =
 // |sum_k A'_ik H'_kj| for |A'| <= 2^PA, |H'| <= 2^PH (rounding adds at most 1/2 per entry):
 //   L1: 2^(PA+PH) * (rho + k 2^-9),      rho = max_j sum_k|H_kj| / max_k|H_kj|
 //   CS: 2^(PA+PH) * (ra + sqrt(k)/512) * (rh + sqrt(k)/512),
@@ -1896,79 +1897,83 @@ __device__ __forceinline__ int dft_col(int rc, int nn, int kr) {
   return (im >= 0 && im < nn) ? im : -1;
 }
 
+// The exponent of a row or column of the recombination.
+__device__ __forceinline__ int crt_exp(unsigned long long bits, int P) {
+  return bits >= INF_BITS ? EXP_NAN : bits == 0 ? EXP_ZERO : scale_exp(bits, P);
+}
+
+// Byte c of w, sign-extended.
+template <int C>
+__device__ __forceinline__ int sbyte(uint32_t w) {
+  int r;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(w), "n"(0x8880 + 0x1111 * C));
+  return r;
+}
+
 // The CRT of four neighbouring columns of one row: the residue words of the moduli at rp (a
-// 4-byte aligned address in the first plane; planes plane_w words apart), ab the row's maximum
-// (its exponent with PA), hb / fexp the columns' maxima and exponents; val = Z 2^-(s + f), NaN
-// for a non-finite row or column, 0 for a zero one.
-template <bool TOP32>
+// 4-byte aligned address in the first plane; planes plane_w words apart), sexp / fexp the row's and the columns'
+// exponents (crt_exp); val = Z 2^-(s + f).
+//
+// Instruction issue bounds it.  Summing the CRT basis modulus by modulus took four wide multiply-adds (24 lanes an SM)
+// and a sign extension per residue; grouped, a residue takes two 32-bit multiply-adds, a group three wide
+// ones, and the limbs' sums are the words of Z in two's complement.  13 moduli, 16384^2 outputs: 3.92 -> 2.35 ms
+// (planes in, doubles out at the memory's rate: 0.83); 5000 x 3003 with alpha and beta 245 -> 158 us.
+template <bool THREE>
 __device__ __forceinline__ void crt_row4(const int8_t* __restrict__ rp, size_t plane_w, const CrtConsts& cc,
-                                         unsigned long long ab, int PA, const unsigned long long (&hb)[4],
-                                         const int (&fexp)[4], double (&val)[4]) {
-  const int sexp = (ab != 0 && ab < INF_BITS) ? scale_exp(ab, PA) : 0;
-  unsigned long long acc[4][4];
-  unsigned acc3[4];
-  int qi[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    qi[c] = 0;
-    acc3[c] = 0;
-#pragma unroll
-    for (int t = 0; t < 4; ++t) acc[c][t] = 0;
-  }
+                                         int sexp, const int (&fexp)[4], double (&val)[4]) {
   const uint32_t* src = (const uint32_t*)rp;
   // all residue words first (the loads are then in flight together), then the sums
-  uint32_t wl[SPL_MAX_MODULI];
+  uint32_t wl[CRT_SLOTS];
+  const int slots = cc.nmod + (cc.four ? 0 : 1);
 #pragma unroll
-  for (int l = 0; l < SPL_MAX_MODULI; ++l) wl[l] = (l < cc.nmod) ? __ldg(src + (size_t)l * plane_w) : 0u;
-#pragma unroll
-  for (int l = 0; l < SPL_MAX_MODULI; ++l) {
-    if (l >= cc.nmod) break;
-    const uint32_t w4 = wl[l];
-    const int ff = cc.ffix[l];
-    const unsigned c0 = cc.climb[l][0], c1 = cc.climb[l][1], c2 = cc.climb[l][2], c3 = cc.climb[l][3];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int r = (int)(int8_t)(w4 >> (8 * c));
-      qi[c] += r * ff;
-      const unsigned ur = (unsigned)(r + 128);
-      acc[c][0] += (unsigned long long)ur * c0;
-      acc[c][1] += (unsigned long long)ur * c1;
-      acc[c][2] += (unsigned long long)ur * c2;
-      if (TOP32)
-        acc3[c] += ur * c3;
-      else
-        acc[c][3] += (unsigned long long)ur * c3;
+  for (int t = 0; t < CRT_SLOTS; ++t) {
+    wl[t] = 0;
+    if (t < slots && (t != 3 || cc.four)) {
+      wl[t] = __ldg(src);
+      src += plane_w;
     }
   }
-  if (TOP32) {
+  unsigned long long acc[4][3];
+  unsigned top[4], qs[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) acc[c][3] = acc3[c];
+  for (int c = 0; c < 4; ++c) {
+    qs[c] = 1u << 14;
+    top[c] = 0;
+#pragma unroll
+    for (int t = 0; t < 3; ++t) acc[c][t] = 0;
+  }
+#pragma unroll
+  for (int g = 0; g < CRT_GROUPS; ++g) {
+    if (g >= cc.groups) break;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      unsigned t = cc.gb[g], f = cc.gfb[g];
+#pragma unroll
+      for (int i = 0; i < (g == 0 ? 4 : 3); ++i) {
+        const int slot = g == 0 ? i : 3 * g + 1 + i;
+        if (slot == 3 && !cc.four) break;
+        const uint32_t w = wl[slot];
+        const unsigned r = (unsigned)(c == 0 ? sbyte<0>(w) : c == 1 ? sbyte<1>(w) : c == 2 ? sbyte<2>(w) : sbyte<3>(w));
+        t += r * cc.gc[slot];
+        f += r * cc.gf[slot];
+      }
+      const unsigned X = t - (f >> 20) * cc.gP[g];  // in [0, 1.002 P), below 2^32
+      qs[c] += __umulhi(X, cc.gG[g]);               // 2^15 X / P, less than two too small
+#pragma unroll
+      for (int s = 0; s < 3; ++s) acc[c][s] += (unsigned long long)X * cc.gW[g][s];
+      if (!THREE) top[c] += X * cc.gW[g][3];
+    }
   }
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    if (ab >= INF_BITS || hb[c] >= INF_BITS) {
-      val[c] = __longlong_as_double(0x7FF8000000000000ll);  // NaN: non-finite input row/column
-    } else if (ab != 0 && hb[c] != 0) {
-      // Z = sum_l r_l C_l - q*M in signed 64-bit limbs (|limb terms| < 2^46), then carries
-      const long long q = (long long)((qi[c] + (1 << 18)) >> 19);
-      long long z0 = (long long)acc[c][0] - (long long)cc.biasl[0] - q * (long long)cc.Mlimb[0];
-      long long z1 = (long long)acc[c][1] - (long long)cc.biasl[1] - q * (long long)cc.Mlimb[1];
-      long long z2 = (long long)acc[c][2] - (long long)cc.biasl[2] - q * (long long)cc.Mlimb[2];
-      long long z3 = (long long)acc[c][3] - (long long)cc.biasl[3] - q * (long long)cc.Mlimb[3];
-      z1 += z0 >> 32;
-      z2 += z1 >> 32;
-      z3 += z2 >> 32;  // exact: z3 holds the sign and top bits of Z (|Z| < 2^126)
-      const unsigned long long L0 = (unsigned long long)z0 & 0xFFFFFFFFull;
-      const unsigned long long L1 = (unsigned long long)z1 & 0xFFFFFFFFull;
-      const unsigned long long L2 = (unsigned long long)z2 & 0xFFFFFFFFull;
-      unsigned long long hi = ((unsigned long long)z3 << 32) | L2, lo = (L1 << 32) | L0;
-      const bool neg = z3 < 0;
-      if (neg) {  // two's-complement negate of the 128-bit value
-        lo = ~lo + 1;
-        hi = ~hi + (lo == 0 ? 1 : 0);
-      }
-      val[c] = u128w_scaled(hi, lo, neg, sexp + fexp[c]);
-    }
+    const unsigned q = qs[c] >> 15;
+    const unsigned long long z0 = acc[c][0] + (unsigned long long)q * cc.Mneg[0];
+    const unsigned long long z1 = acc[c][1] + (unsigned long long)q * cc.Mneg[1] + (z0 >> 32);
+    const unsigned long long z2 = acc[c][2] + (unsigned long long)q * cc.Mneg[2] + (z1 >> 32);
+    const unsigned z3 = top[c] + q * cc.Mneg[3] + (unsigned)(z2 >> 32);
+    const unsigned __int128 z = ((unsigned __int128)(((unsigned long long)z3 << 32) | (unsigned)z2) << 64) |
+                                ((z1 << 32) | (unsigned)z0);
+    val[c] = i128_scaled((__int128)z, sexp + fexp[c]);
   }
 }
 
@@ -1976,9 +1981,8 @@ __device__ __forceinline__ void crt_row4(const int8_t* __restrict__ rp, size_t p
 // columns [0, n) and Im in [kr/2, kr/2 + n) (the 3M layout); Re / Im of element (i, j) go to
 // the interleaved complex C at 2j / 2j + 1 + i*ldq (ldq in doubles); column j's exponent is
 // that of hmax_bits[j].
-// TOP32 (cc.top32): the sum over the moduli of (r_l + 128) times the top 32-bit limb of C_l
-// stays below 2^32 (true for M < 2^112: every top limb is below 2^16), so it is kept in 32 bits.
-template <bool DFT_OUT, bool TOP32 = false, int TI = CRT_TI>
+// THREE: cc.three.
+template <bool DFT_OUT, bool THREE = false, int TI = CRT_TI>
 __device__ __forceinline__ void crt_combine_blk(const int8_t* __restrict__ R, int n, int k, int kr,
                                                 const CrtConsts& cc, const unsigned long long* __restrict__ amax_bits,
                                                 const unsigned long long* __restrict__ hmax_bits,
@@ -1986,31 +1990,30 @@ __device__ __forceinline__ void crt_combine_blk(const int8_t* __restrict__ R, in
                                                 double* __restrict__ Q, long ldq, int bx, int by,
                                                 const unsigned long long* __restrict__ gmax_bits = nullptr,
                                                 int gw = 1) {
-  // element (jl, il) of the tile at column (il + jl/4) mod 32 of row jl: the row-wise writes
-  // (4 columns per thread) and the column-wise reads both hit distinct bank pairs
-  __shared__ double tile[CRT_TJ][TI];
+  // four columns a row of the tile, one element of padding: the row-wise writes (4 columns per
+  // thread) and the column-wise reads both hit distinct bank pairs
+  __shared__ double tile[CRT_TJ / 4][4 * TI + 1];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i0 = by * TI, j0 = bx * CRT_TJ;
   const int PA = prm->PA, PH = prm->PH;
   const int jb = j0 + 4 * tx;
   const int kcols = DFT_OUT ? kr : k;  // residue columns covered
-  unsigned long long hb[4];
   int fexp[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const int hc = DFT_OUT ? dft_col(jb + c, k, kr) : (jb + c < k ? jb + c : -1);
-    hb[c] = hc >= 0 ? hmax_bits[hc] : 0ull;
+    unsigned long long hb = hc >= 0 ? hmax_bits[hc] : 0ull;
     // block-recursive products: finite columns scaled with their group's exponent
-    if (gmax_bits != nullptr && hc >= 0 && hb[c] < INF_BITS && !prm->hbad) hb[c] = gmax_bits[hc % gw];
-    fexp[c] = (hb[c] != 0 && hb[c] < INF_BITS) ? scale_exp(hb[c], PH) : 0;
+    if (gmax_bits != nullptr && hc >= 0 && hb < INF_BITS && !prm->hbad) hb = gmax_bits[hc % gw];
+    fexp[c] = crt_exp(hb, PH);
   }
   const size_t plane_w = (size_t)n * kr / 4;
   for (int a = 0; a < TI / 8; ++a) {
     const int il = ty + 8 * a, i = i0 + il;
     double val[4] = {0.0, 0.0, 0.0, 0.0};
-    if (i < n && jb < kcols) crt_row4<TOP32>(R + (size_t)i * kr + jb, plane_w, cc, amax_bits[i], PA, hb, fexp, val);
+    if (i < n && jb < kcols) crt_row4<THREE>(R + (size_t)i * kr + jb, plane_w, cc, crt_exp(amax_bits[i], PA), fexp, val);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) tile[4 * tx + c][(il + tx) & (TI - 1)] = val[c];
+    for (int c = 0; c < 4; ++c) tile[tx][c * TI + il] = val[c];
   }
   __syncthreads();
   const bool scale = alpha != 1.0, accumulate = beta != 0.0;  // uniform: decided once
@@ -2018,20 +2021,35 @@ __device__ __forceinline__ void crt_combine_blk(const int8_t* __restrict__ R, in
     // Q = Z 2^-(s+f): a loop of its own, without the FP64 epilogue (instructions predicated off
     // would still be issued to GB300's narrow FP64 pipe)
     const int t = ty * 32 + tx, ir = t % TI, i = i0 + ir;
-    for (int jl = t / TI; jl < CRT_TJ; jl += 256 / TI) {
-      const int jj = j0 + jl;
-      if (i < n && jj < k) Q[i + (long)jj * ldq] = tile[jl][(ir + (jl >> 2)) & (TI - 1)];
+    const int left = i < n ? k - j0 : 0;
+    double* qp = Q + i + (long)(j0 + t / TI) * ldq;
+#pragma unroll
+    for (int u = 0; u < CRT_TJ * TI / 256; ++u, qp += ldq * (256 / TI)) {
+      const int jl = t / TI + u * (256 / TI);
+      if (jl < left) *qp = tile[jl >> 2][(jl & 3) * TI + ir];
     }
   } else if (!DFT_OUT) {
     const int t = ty * 32 + tx, ir = t % TI, i = i0 + ir;
-    for (int jl = t / TI; jl < CRT_TJ; jl += 256 / TI) {
-      const int jj = j0 + jl;
-      if (i < n && jj < k) {
-        double* qp = Q + i + (long)jj * ldq;
-        double v = tile[jl][(ir + (jl >> 2)) & (TI - 1)];
-        if (scale) v *= alpha;
-        if (accumulate) v = fma(beta, *qp, v);
-        *qp = v;
+    constexpr int AHEAD = 4;  // loads of Q in flight a thread (one at a time, they were the pass's longest stall)
+    static_assert(CRT_TJ * TI / 256 % AHEAD == 0);
+    const int left = i < n ? k - j0 : 0;
+    double* qp = Q + i + (long)(j0 + t / TI) * ldq;
+#pragma unroll
+    for (int u0 = 0; u0 < CRT_TJ * TI / 256; u0 += AHEAD) {
+      double q[AHEAD];
+      const double* ql = qp;
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u, ql += ldq * (256 / TI))
+        q[u] = accumulate && t / TI + (u0 + u) * (256 / TI) < left ? *ql : 0.0;
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u, qp += ldq * (256 / TI)) {
+        const int jl = t / TI + (u0 + u) * (256 / TI);
+        if (jl < left) {
+          double v = tile[jl >> 2][(jl & 3) * TI + ir];
+          if (scale) v *= alpha;
+          if (accumulate) v = fma(beta, q[u], v);
+          *qp = v;
+        }
       }
     }
   } else {
@@ -2043,7 +2061,7 @@ __device__ __forceinline__ void crt_combine_blk(const int8_t* __restrict__ R, in
         const int jj = jb + c, hc = dft_col(jj, k, kr);
         if (hc < 0) continue;
         double* qp = Q + (long)i * ldq + 2 * hc + (jj >= (kr >> 1) ? 1 : 0);
-        double v = tile[4 * tx + c][(il + tx) & (TI - 1)];
+        double v = tile[tx][c * TI + il];
         if (scale) v *= alpha;
         if (accumulate) v = fma(beta, *qp, v);
         *qp = v;
@@ -2052,7 +2070,7 @@ __device__ __forceinline__ void crt_combine_blk(const int8_t* __restrict__ R, in
   }
 }
 
-template <bool DFT_OUT, bool TOP32>
+template <bool DFT_OUT, bool THREE>
 __global__ void __launch_bounds__(256, 3) k_crt_combine(const int8_t* __restrict__ R, int n, int k, int kr,
                                                      CrtConsts cc, const unsigned long long* __restrict__ amax_bits,
                                                      const unsigned long long* __restrict__ hmax_bits,
@@ -2060,22 +2078,22 @@ __global__ void __launch_bounds__(256, 3) k_crt_combine(const int8_t* __restrict
                                                      double* __restrict__ Q, long ldq, int by0,
                                                      const unsigned* gate = nullptr) {
   if (gated_off(gate)) return;
-  crt_combine_blk<DFT_OUT, TOP32>(R, n, k, kr, cc, amax_bits, hmax_bits, prm, alpha, beta, Q, ldq, blockIdx.x,
+  crt_combine_blk<DFT_OUT, THREE>(R, n, k, kr, cc, amax_bits, hmax_bits, prm, alpha, beta, Q, ldq, blockIdx.x,
                                   by0 + blockIdx.y);
 }
 
 // The same in tiles of eight rows, for outputs of few 32-row tiles (1000 x 777: 224 blocks, 26 us).
-template <bool TOP32>
+template <bool THREE>
 __global__ void __launch_bounds__(256, 3) k_crt_combine8(const int8_t* __restrict__ R, int n, int k, int kr, CrtConsts cc,
                                                       const unsigned long long* __restrict__ amax_bits,
                                                       const unsigned long long* __restrict__ hmax_bits,
                                                       const SplitDevParams* prm, double alpha, double beta,
                                                       double* __restrict__ Q, long ldq) {
-  crt_combine_blk<false, TOP32, 8>(R, n, k, kr, cc, amax_bits, hmax_bits, prm, alpha, beta, Q, ldq, blockIdx.x, blockIdx.y);
+  crt_combine_blk<false, THREE, 8>(R, n, k, kr, cc, amax_bits, hmax_bits, prm, alpha, beta, Q, ldq, blockIdx.x, blockIdx.y);
 }
 
 // The recombination of the block-recursive products (group exponents unless prm->hbad).
-template <bool TOP32>
+template <bool THREE>
 __global__ void __launch_bounds__(256, 3) k_crt_combine_blocks(const int8_t* __restrict__ R, int n, int k, int kr,
                                                             CrtConsts cc,
                                                             const unsigned long long* __restrict__ amax_bits,
@@ -2083,7 +2101,7 @@ __global__ void __launch_bounds__(256, 3) k_crt_combine_blocks(const int8_t* __r
                                                             const unsigned long long* __restrict__ gmax_bits, int gw,
                                                             const SplitDevParams* prm, double alpha, double beta,
                                                             double* __restrict__ Q, long ldq, int by0) {
-  crt_combine_blk<false, TOP32>(R, n, k, kr, cc, amax_bits, hmax_bits, prm, alpha, beta, Q, ldq, blockIdx.x,
+  crt_combine_blk<false, THREE>(R, n, k, kr, cc, amax_bits, hmax_bits, prm, alpha, beta, Q, ldq, blockIdx.x,
                                 by0 + blockIdx.y, gmax_bits, gw);
 }
 
@@ -2282,7 +2300,7 @@ __global__ void k_dft_radix_combine(const double2* __restrict__ P, int nq, int k
 // CRT is integer work and the butterflies FP64 work: four blocks per SM (64 registers, a few
 // spilled) overlap the two better than three at 74 registers (n = 8192: 2.23 -> 1.98 ms).
 constexpr int RDX_TJ = 64;
-template <int R, bool TOP32>
+template <int R, bool THREE>
 __global__ void __launch_bounds__(256, 4) k_crt_dft_radix(const int8_t* __restrict__ Rres, int M, int nq, int kr,
                                                        CrtConsts cc, const unsigned long long* __restrict__ amax_bits,
                                                        const unsigned long long* __restrict__ hmax_bits,
@@ -2298,13 +2316,11 @@ __global__ void __launch_bounds__(256, 4) k_crt_dft_radix(const int8_t* __restri
   const bool im = tx >= 16;
   const int jl0 = 4 * (tx & 15);
   const int rc = (im ? kr / 2 : 0) + j0 + jl0;
-  unsigned long long hb[4];
   int fexp[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     const int j = j0 + jl0 + e;
-    hb[e] = j < nq ? hmax_bits[j] : 0ull;
-    fexp[e] = (hb[e] != 0 && hb[e] < INF_BITS) ? scale_exp(hb[e], PH) : 0;
+    fexp[e] = crt_exp(j < nq ? hmax_bits[j] : 0ull, PH);
   }
   const size_t plane_w = (size_t)M * kr / 4;
   const bool scale = alpha != 1.0, accumulate = beta != 0.0;
@@ -2313,7 +2329,7 @@ __global__ void __launch_bounds__(256, 4) k_crt_dft_radix(const int8_t* __restri
       const int il = ty + 8 * a;
       const int c = cb + il % CPB, i = (il / CPB) * k + c;
       double val[4] = {0.0, 0.0, 0.0, 0.0};
-      if (c < k && j0 + jl0 < nq) crt_row4<TOP32>(Rres + (size_t)i * kr + rc, plane_w, cc, amax_bits[i], PA, hb, fexp, val);
+      if (c < k && j0 + jl0 < nq) crt_row4<THREE>(Rres + (size_t)i * kr + rc, plane_w, cc, crt_exp(amax_bits[i], PA), fexp, val);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         // rotated (selects, not a dynamic index): a warp's eight-byte stores spread over the banks
@@ -2502,10 +2518,10 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
 
   dim3 gc((N + CRT_TJ - 1) / CRT_TJ, (M + CRT_TI - 1) / CRT_TI);
   if (!gate && (long)gc.x * gc.y < 4L * sms)
-    (cc.top32 ? k_crt_combine8<true> : k_crt_combine8<false>)<<<dim3(gc.x, (M + 7) / 8), dim3(32, 8), 0, stream>>>(
+    (cc.three ? k_crt_combine8<true> : k_crt_combine8<false>)<<<dim3(gc.x, (M + 7) / 8), dim3(32, 8), 0, stream>>>(
         b.R, M, N, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq);
   else
-    (cc.top32 ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, stream>>>(
+    (cc.three ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, stream>>>(
         b.R, M, N, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq, 0, gate);
   prof_mark(stream, "crt_combine");
   if (cudaGetLastError() != cudaSuccess) return PSMMA_EDEVICE;
@@ -2893,7 +2909,7 @@ struct BlockRun {
   void crt(int r0, int rows, double alpha, double beta, double* Q, long ldq, const SplitDevParams* pk,
            cudaStream_t s) {
     const dim3 gc((N + CRT_TJ - 1) / CRT_TJ, (rows + CRT_TI - 1) / CRT_TI);
-    (cc.top32 ? k_crt_combine_blocks<true> : k_crt_combine_blocks<false>)<<<gc, dim3(32, 8), 0, s>>>(
+    (cc.three ? k_crt_combine_blocks<true> : k_crt_combine_blocks<false>)<<<gc, dim3(32, 8), 0, s>>>(
         b.R, M, N, Lo.kr, cc, b.amax, b.hmax, gmax, w, pk, alpha, beta, Q, ldq, r0 / CRT_TI);
   }
 };
@@ -3119,7 +3135,7 @@ static int split_core_s2(int M, int N, int K, double alpha, const double* A, lon
   const int rc = s2_pass(st, A, lda, b.amax, b.prm, 0, M, stream);
   if (rc != PSMMA_OK) return rc;
   dim3 gc((N + CRT_TJ - 1) / CRT_TJ, (M + CRT_TI - 1) / CRT_TI);
-  (st.cc.top32 ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, stream>>>(
+  (st.cc.three ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, stream>>>(
       b.R, M, N, Lo.kr, st.cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq, 0, nullptr);
   prof_mark(stream, "crt_combine");
   if (cudaGetLastError() != cudaSuccess) return PSMMA_EDEVICE;
@@ -3243,7 +3259,7 @@ static int split_core_host(int M, int N, int K, double alpha, const double* A_h,
     k_crt_gemm<G_BN, OneGemm><<<std::min(sms, total_tiles), G_THREADS, Shape::SMEM, s>>>(og);
     const int r0 = t0 * G_BM, r1 = std::min(M, t1 * G_BM);
     dim3 gc((N + CRT_TJ - 1) / CRT_TJ, (r1 - r0 + CRT_TI - 1) / CRT_TI);
-    (cc.top32 ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, s>>>(
+    (cc.three ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, s>>>(
         b.R, M, N, L.kr, cc, b.amax, b.hmax, pk, alpha, beta, dQ, M, r0 / CRT_TI, nullptr);
     prof_mark(s, "panel_gemm_crt");
     ok &= cudaEventRecord(ev_panel[p], s) == cudaSuccess;
@@ -3654,17 +3670,17 @@ static int dft3_enqueue(int M, int nn, double alpha, const double* B, long ldb, 
   k_crt_dft_radix<RR, T32><<<gr, dim3(32, 8), 0, stream>>>(b.R, M, nn, L.kr, cc, b.amax, b.hmax, b.prm, alpha, \
                                                           src->wn, src->beta, src->C, src->ldc, src->k)
     if (src->R == 8) {
-      if (cc.top32) PSMMA_CRT_RADIX(8, true); else PSMMA_CRT_RADIX(8, false);
+      if (cc.three) PSMMA_CRT_RADIX(8, true); else PSMMA_CRT_RADIX(8, false);
     } else if (src->R == 4) {
-      if (cc.top32) PSMMA_CRT_RADIX(4, true); else PSMMA_CRT_RADIX(4, false);
+      if (cc.three) PSMMA_CRT_RADIX(4, true); else PSMMA_CRT_RADIX(4, false);
     } else {
-      if (cc.top32) PSMMA_CRT_RADIX(2, true); else PSMMA_CRT_RADIX(2, false);
+      if (cc.three) PSMMA_CRT_RADIX(2, true); else PSMMA_CRT_RADIX(2, false);
     }
 #undef PSMMA_CRT_RADIX
     prof_mark(stream, "crt_radix_combine");
   } else {
     dim3 gc(L.kr / CRT_TJ, (M + CRT_TI - 1) / CRT_TI);
-    (cc.top32 ? k_crt_combine<true, true> : k_crt_combine<true, false>)<<<gc, dim3(32, 8), 0, stream>>>(
+    (cc.three ? k_crt_combine<true, true> : k_crt_combine<true, false>)<<<gc, dim3(32, 8), 0, stream>>>(
         b.R, M, nn, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, C, 2 * ldc, 0, nullptr);
     prof_mark(stream, "crt_combine");
   }
@@ -3888,12 +3904,12 @@ __global__ void __launch_bounds__(128) k_g_residues_H(const GProb* d, int count,
   }
 }
 
-template <bool TOP32>
-__global__ void __launch_bounds__(256, 3) k_g_crt_combine(const GProb* d, int count, int total, int run, CrtConsts cc) {
+template <bool THREE>
+__global__ void __launch_bounds__(256, 4) k_g_crt_combine(const GProb* d, int count, int total, int run, CrtConsts cc) {
   for (GRun<4> r(d, count, total, run); r.b < r.end; ++r.b) {
     const GProb& e = r.owner(d, count);
     const int local = r.b - e.b_crt, gx = (e.N + CRT_TJ - 1) / CRT_TJ;
-    crt_combine_blk<false, TOP32>(e.R, e.M, e.N, e.kr, cc, e.amax, e.hmax, e.prm, e.alpha, e.beta, e.Q, e.ldq,
+    crt_combine_blk<false, THREE>(e.R, e.M, e.N, e.kr, cc, e.amax, e.hmax, e.prm, e.alpha, e.beta, e.Q, e.ldq,
                                   local % gx, local / gx);
     __syncthreads();  // the shared transpose tile is reused by the next block
   }
@@ -4097,7 +4113,7 @@ int split_group_enqueue(const SplitGroup& g, cudaStream_t stream, unsigned* stat
   prof_mark(stream, "g_gemm_64");
   if (st) return st;
   if (g.blocks_crt > 0)
-    (cc.top32 ? k_g_crt_combine<true> : k_g_crt_combine<false>)<<<runs(g.blocks_crt, n_crt), dim3(32, 8), 0,
+    (cc.three ? k_g_crt_combine<true> : k_g_crt_combine<false>)<<<runs(g.blocks_crt, n_crt), dim3(32, 8), 0,
                                                                    stream>>>(d, g.count, g.blocks_crt, n_crt, cc);
   prof_mark(stream, "g_crt_combine");
   if (cudaGetLastError() != cudaSuccess) return PSMMA_EDEVICE;

@@ -227,48 +227,45 @@ __device__ __forceinline__ unsigned long long scaled_int(double x, int e, bool* 
   return (m + ((1ull << (k - 1)) - 1) + ((m >> k) & 1)) >> k;
 }
 
-// m * 2^x with the sign, for results outside the normal range; out of line, so that its FP64
-// instructions are not issued (predicated off) for every element.
-static __device__ __noinline__ double scaled_outside_normal(unsigned long long m, int x, bool neg) {
-  const double v = ldexp((double)m, x);
+// Exponents of a row or column that make every product with it zero, or NaN: beyond any sum of two others.
+constexpr int EXP_ZERO = 1 << 20, EXP_NAN = 1 << 24;
+
+// i128_scaled's rare results: zero, few bits, outside the normal range, EXP_ZERO and EXP_NAN.  Out of line, so that its
+// FP64 instructions are not issued (predicated off) for every element.
+static __device__ __noinline__ double i128_scaled_rare(unsigned long long hi, unsigned long long lo, bool neg, int e) {
+  if (e >= EXP_ZERO / 2) return e < EXP_NAN / 2 ? 0.0 : __longlong_as_double(0x7FF8000000000000ll);
+  if ((hi | lo) == 0) return 0.0;
+  const int s = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+  const int p = 127 - s;  // exponent of the leading bit
+  const unsigned long long top = s >= 64 ? lo << (s - 64) : s ? (hi << s) | (lo >> (64 - s)) : hi;
+  const unsigned long long rest = s >= 64 ? 0 : lo << s;
+  unsigned long long m = top >> 11;  // 53 bits
+  const bool sticky = (top & 0x3FFull) != 0 || rest != 0;
+  if ((top & 0x400ull) && (sticky || (m & 1))) ++m;
+  const double v = ldexp((double)m, p - 52 - e);
   return neg ? -v : v;
 }
 
-// (hi:lo) * 2^-e as a double, (hi:lo) a non-negative 128-bit integer in two words, rounded
-// to nearest even from the bits; results outside the normal range go through ldexp.
-__device__ __forceinline__ double u128w_scaled(unsigned long long hi, unsigned long long lo, bool neg, int e) {
-  if ((hi | lo) == 0) return 0.0;
-  // normalise so that the leading bit is bit 63 of `top`; `rest` keeps the bits below
-  int p;
-  unsigned long long top, rest;
-  if (hi) {
-    const int s = __clzll((long long)hi);
-    p = 127 - s;
-    top = s ? (hi << s) | (lo >> (64 - s)) : hi;
-    rest = s ? (lo << s) : lo;
-  } else {
-    const int s = __clzll((long long)lo);
-    p = 63 - s;
-    top = lo << s;
-    rest = 0;
+// z * 2^-e as a double, rounded to nearest even from the bits; results outside the normal range go through ldexp.
+__device__ __forceinline__ double i128_scaled(__int128 z, int e) {
+  const bool neg = z < 0;
+  const unsigned __int128 sg = neg ? ~(unsigned __int128)0 : 0, u = ((unsigned __int128)z ^ sg) - sg;
+  unsigned w3 = (unsigned)(u >> 96), w2 = (unsigned)(u >> 64), w1 = (unsigned)(u >> 32), w0 = (unsigned)u;
+  int x = 127 + 1022 - e;  // biased exponent of bit 31 of w3, less one
+  if (w3 == 0) {
+    w3 = w2; w2 = w1; w1 = w0; w0 = 0;
+    x -= 32;
   }
-  unsigned long long m = top >> 11;  // 53 bits
-  const unsigned long long low11 = top & 0x7FFull;
-  const bool sticky = (low11 & 0x3FFull) != 0 || rest != 0;
-  if ((low11 & 0x400ull) && (sticky || (m & 1))) {
-    ++m;
-    if (m == (1ull << 53)) {
-      m >>= 1;
-      ++p;
-    }
-  }
-  const int field = p - e + 1023;
-  if (field >= 1 && field <= 2046) {
-    unsigned long long bits = ((unsigned long long)field << 52) | (m & 0xFFFFFFFFFFFFFull);
-    if (neg) bits |= 1ull << 63;
-    return __longlong_as_double((long long)bits);
-  }
-  return scaled_outside_normal(m, p - 52 - e, neg);
+  const int s = __clz((int)w3);
+  x -= s;
+  if (w3 == 0 || (unsigned)x >= 2045u) return i128_scaled_rare((unsigned long long)(u >> 64), (unsigned long long)u, neg, e);
+  const unsigned t3 = __funnelshift_l(w2, w3, s), t2 = __funnelshift_l(w1, w2, s);
+  const unsigned rest = (__funnelshift_l(w0, w1, s) | (w0 << s)) != 0 ? 1u : 0u;
+  // the 11 bits below the last kept one, a sticky bit, that last bit
+  const unsigned up = (((t2 & 0x7FFu) | rest) + 0x3FFu + ((t2 >> 11) & 1u)) >> 11;
+  // the leading bit of t3 >> 11 adds one to the exponent field, a carry out of the mantissa another
+  const unsigned head = ((unsigned)x << 20) + (t3 >> 11) + (neg ? 0x80000000u : 0u);
+  return __longlong_as_double((long long)((((unsigned long long)head << 32) | ((t3 << 21) | (t2 >> 11))) + up));
 }
 
 // H pass 1: Ht[j][kk] = H(kk, j) in FP64, column max |H| and column sum |H|, and the global
