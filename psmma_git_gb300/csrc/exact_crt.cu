@@ -37,19 +37,30 @@ namespace {
 // Moduli and CRT constants (compile time)
 // ------------------------------------------------------------------------------------------
 // Pairwise coprime, at most 256: 2^8, 3*5*17, 11*23, 13*19, 7*31 and primes.
-constexpr int EX_MAX = 32, EX_GROUPS = EX_MAX / 4, EX_LIMBS = 9, EX_CHUNKS = 8;
+constexpr int EX_MAX = 32, EX_GROUPS = EX_MAX / 4, EX_WORDS = 8, EX_PARTS = 10, EX_CHUNKS = 8;
 constexpr int kExModuli[EX_MAX] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193, 191,
                                    217, 181, 179, 173, 167, 163, 157, 151, 149, 139, 137, 131, 127, 113, 109, 107};
 
-// The CRT for the first 4 G moduli.  The four moduli of a group g (product P_g < 2^32) are first
-// combined in 32-bit arithmetic: with u_i = residue + 128 in [0, 255],
-//   X_g = b_g + sum_i u_i c_i (mod P_g),  X_g = Z W_g^-1 mod P_g,  W_g = M / P_g,
-// and Z = sum_g X_g W_g - q M with q the nearest integer to sum_g X_g / P_g.
+// The CRT for the first 4 G moduli.  They form parts of three and then, where 4 G is not a multiple of three, one or two
+// of four (8 moduli: 3, 3, 2), each of a product P_g < 2^32; a part's moduli are first combined in 32-bit arithmetic:
+//   X_g = b_g + sum_i r_i c_i (mod P_g),  X_g = Z W_g^-1 mod P_g,  W_g = M / P_g,
+// and Z = sum_g X_g W_g - q M with q the nearest integer to sum_g X_g / P_g.  The parts of four have the smallest
+// moduli: sum_g X_g W_g[s] stays below 2^63 for every 32-bit word s, so that the sums are the words of Z.
+__host__ __device__ constexpr int ex_fours(int G) { return G == 2 ? 0 : 4 * G % 3; }
+__host__ __device__ constexpr int ex_parts(int G) { return G == 2 ? 3 : (4 * G - 4 * ex_fours(G)) / 3 + ex_fours(G); }
+__host__ __device__ constexpr int ex_first(int G, int g) {  // first modulus of part g
+  const int threes = G == 2 ? 3 : ex_parts(G) - ex_fours(G);
+  return g < threes ? 3 * g : 3 * threes + 4 * (g - threes);
+}
+__host__ __device__ constexpr int ex_size(int G, int g) { return (g + 1 < ex_parts(G) ? ex_first(G, g + 1) : 4 * G) - ex_first(G, g); }
+__host__ __device__ constexpr int ex_shift(int G) { return G == 2 ? 47 : 52; }  // fixed point of 1 / P_g: P_g >= 2^15.7, 2^20 above
+__host__ __device__ constexpr int ex_words(int G) { return G; }                 // log2 M = 63.6, 94.8, 125.2, 155.4, 184.6, 213.1, 240.4
 struct ExCrt {
   unsigned c[EX_MAX], f[EX_MAX];      // c_i, floor(2^20 c_i / P_g)
-  unsigned b[EX_GROUPS], fb[EX_GROUPS], P[EX_GROUPS], G[EX_GROUPS];  // ..., P_g, floor(2^52 / P_g)
-  unsigned W[EX_GROUPS][EX_LIMBS];    // W_g in 28-bit limbs
-  unsigned M[EX_LIMBS];
+  // the starts of both sums, so that they are those of r + 128 in [0, 255]; P_g, floor(2^ex_shift / P_g)
+  unsigned b[EX_PARTS], fb[EX_PARTS], P[EX_PARTS], G[EX_PARTS];
+  unsigned W[EX_PARTS][EX_WORDS];     // W_g
+  unsigned Mneg[EX_WORDS];            // 2^256 - M
 };
 struct ExTables {
   ExCrt crt[EX_GROUPS + 1];           // by group count (2..8)
@@ -77,43 +88,51 @@ constexpr ExTables make_tables() {
   }
   for (int G = 2; G <= EX_GROUPS; ++G) {
     ExCrt& C = T.crt[G];
-    for (int g = 0; g < G; ++g) {
+    for (int g = 0; g < ex_parts(G); ++g) {
+      const int first = ex_first(G, g), size = ex_size(G, g);
       unsigned long long P = 1;
-      for (int i = 0; i < 4; ++i) P *= (unsigned long long)kExModuli[4 * g + i];
+      for (int i = 0; i < size; ++i) P *= (unsigned long long)kExModuli[first + i];
       C.P[g] = (unsigned)P;
-      C.G[g] = (unsigned)((1ull << 52) / P);
+      C.G[g] = (unsigned)((1ull << ex_shift(G)) / P);
       C.W[g][0] = 1;
       for (int l = 0; l < 4 * G; ++l) {
-        if (l / 4 == g) continue;
+        if (l >= first && l < first + size) continue;
         unsigned long long carry = 0;
-        for (int t = 0; t < EX_LIMBS; ++t) {
+        for (int t = 0; t < EX_WORDS; ++t) {
           const unsigned long long v = (unsigned long long)C.W[g][t] * kExModuli[l] + carry;
-          C.W[g][t] = (unsigned)(v & 0xFFFFFFFull);
-          carry = v >> 28;
+          C.W[g][t] = (unsigned)v;
+          carry = v >> 32;
         }
       }
-      unsigned long long bias = 0;
-      for (int i = 0; i < 4; ++i) {
-        const unsigned long long m = kExModuli[4 * g + i], Q = P / m;
+      unsigned long long bias = 0, fbias = 0;
+      for (int i = 0; i < size; ++i) {
+        const unsigned long long m = kExModuli[first + i], Q = P / m;
         unsigned long long w = 0;  // W_g mod m
-        for (int t = EX_LIMBS - 1; t >= 0; --t) w = (w * (1ull << 28) + C.W[g][t]) % m;
+        for (int t = EX_WORDS - 1; t >= 0; --t) w = ((w << 32) + C.W[g][t]) % m;
         const unsigned long long y = ex_inv(w, m) * ex_inv(Q % m, m) % m;
-        C.c[4 * g + i] = (unsigned)(Q * y);
-        C.f[4 * g + i] = (unsigned)((Q * y << 20) / P);
-        bias = (bias + 128 * (Q * y)) % P;
+        C.c[first + i] = (unsigned)(Q * y);
+        C.f[first + i] = (unsigned)((Q * y << 20) / P);
+        bias += 128 * (Q * y);
+        fbias += 128ull * C.f[first + i];
       }
-      const unsigned long long b = bias ? P - bias : 0;
-      C.b[g] = (unsigned)b;
-      C.fb[g] = (unsigned)((b << 20) / P);
+      const unsigned long long b = (P - bias % P) % P;  // takes the 128s out of X again
+      C.b[g] = (unsigned)(b + bias);
+      C.fb[g] = (unsigned)((b << 20) / P + fbias);
     }
-    C.M[0] = 1;
+    unsigned M[EX_WORDS] = {1, 0, 0, 0, 0, 0, 0, 0};
     for (int l = 0; l < 4 * G; ++l) {
       unsigned long long carry = 0;
-      for (int t = 0; t < EX_LIMBS; ++t) {
-        const unsigned long long v = (unsigned long long)C.M[t] * kExModuli[l] + carry;
-        C.M[t] = (unsigned)(v & 0xFFFFFFFull);
-        carry = v >> 28;
+      for (int t = 0; t < EX_WORDS; ++t) {
+        const unsigned long long v = (unsigned long long)M[t] * kExModuli[l] + carry;
+        M[t] = (unsigned)v;
+        carry = v >> 32;
       }
+    }
+    unsigned long long carry = 1;
+    for (int t = 0; t < EX_WORDS; ++t) {
+      carry += (unsigned)~M[t];
+      C.Mneg[t] = (unsigned)carry;
+      carry >>= 32;
     }
   }
   return T;
@@ -444,114 +463,107 @@ __global__ void __launch_bounds__(256) k_ex_residues(const double* __restrict__ 
 // ------------------------------------------------------------------------------------------
 // CRT
 // ------------------------------------------------------------------------------------------
-__device__ __noinline__ double ex_outside_normal(unsigned long long m, int x, bool neg) {
-  const double v = ldexp((double)m, x);
-  return neg ? -v : v;
-}
-
-// The magnitude in four 64-bit words times 2^e as a double, rounded to nearest even.
-__device__ __forceinline__ double ex_round(const unsigned long long (&w)[4], bool neg, int e) {
-  unsigned long long h, l, rest;
-  int p;
-  if (w[3]) {
-    h = w[3]; l = w[2]; rest = w[1] | w[0]; p = 255;
-  } else if (w[2]) {
-    h = w[2]; l = w[1]; rest = w[0]; p = 191;
-  } else if (w[1]) {
-    h = w[1]; l = w[0]; rest = 0; p = 127;
-  } else {
-    h = w[0]; l = 0; rest = 0; p = 63;
+// (t3:t2) the 64 bits from the leading one, of exponent p + e, `rest` whether any bit is set below: results that are not
+// normal, one rounding at their own precision (ldexp rounds a double exactly scaled; 53 bits would be
+// rounded twice).
+__device__ __noinline__ double ex_outside_normal(unsigned t3, unsigned t2, bool rest, bool neg, int field) {
+  const unsigned long long top = ((unsigned long long)t3 << 32) | t2;
+  if (field > 2045) {
+    unsigned long long m = top >> 11;
+    m += (top & 0x400ull) && ((top & 0x3FFull) != 0 || rest || (m & 1));
+    const double v = ldexp((double)m, field - 1023 - 52);
+    return neg ? -v : v;
   }
-  if (h == 0) return 0.0;
-  const int s = __clzll((long long)h);
-  p -= s;
-  const unsigned long long top = s ? (h << s) | (l >> (64 - s)) : h;
-  rest |= s ? l << s : l;
-  unsigned long long m = top >> 11;
-  const bool sticky = (top & 0x3FFull) != 0 || rest != 0;
-  const unsigned long long up = (top & 0x400ull) && (sticky || (m & 1));
-  const int field = p + e + 1023;
-  if (field >= 1 && field <= 2045) {  // adding the carry to the bits moves the exponent with it
-    unsigned long long bits = (((unsigned long long)field << 52) | (m & 0xFFFFFFFFFFFFFull)) + up;
-    if (neg) bits |= 1ull << 63;
-    return __longlong_as_double((long long)bits);
-  }
-  // subnormal or overflowing results: one rounding at their own precision, from 63 bits and a
-  // sticky bit (ldexp rounds a double exactly scaled; the 53-bit m would be rounded twice)
-  if (field > 2045) return ex_outside_normal(m + up, p - 52 + e, neg);
   const int drop = 1 - field + 11;  // bits of `top` below the subnormal's last place
   if (drop > 64) return neg ? -0.0 : 0.0;
   const unsigned long long keep = drop < 64 ? top >> drop : 0;
   const unsigned long long half = 1ull << (drop - 1);
-  const bool st2 = (top & (half - 1)) != 0 || rest != 0;
+  const bool st2 = (top & (half - 1)) != 0 || rest;
   unsigned long long bits = keep + (((top & half) && (st2 || (keep & 1))) ? 1 : 0);
   if (neg) bits |= 1ull << 63;
   return __longlong_as_double((long long)bits);
 }
 
-// Column c's element from its 4 G residues, offset by 128 (word l holds modulus l's for four
-// columns), times 2^e.
-template <int G>
-__device__ __forceinline__ double ex_crt(const unsigned (&w)[EX_MAX], int c, int e) {
-  constexpr int NL = G + 1;  // 28-bit limbs: log2 M = 63.7, 95, 125, 156, 185, 214, 241 for G = 2..8
+// The element of the 4 G residues r(l), times 2^e, rounded to nearest even.
+// Instruction issue bounds it; sums that are the words of Z need no repacking (28-bit limbs of four-moduli parts before:
+// the Toeplitz multiply of n = 2048 392 us, now 378; 1024 132 / 129; 128 37.6 / 35.5 with one element a thread).
+template <int G, class Residue>
+__device__ __forceinline__ double ex_crt(Residue r, int e) {
+  constexpr int NW = ex_words(G);
   const ExCrt& C = kEx.crt[G];
-  unsigned long long acc[NL];
+  unsigned long long acc[NW - 1];
+  unsigned top = 0, qs = 1u << (ex_shift(G) - 33);
 #pragma unroll
-  for (int t = 0; t < NL; ++t) acc[t] = 0;
-  unsigned qs = 0;
+  for (int t = 0; t < NW - 1; ++t) acc[t] = 0;
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
+  for (int g = 0; g < ex_parts(G); ++g) {
     unsigned t = C.b[g], f = C.fb[g];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const unsigned u = __byte_perm(w[4 * g + i], 0u, 0x4440u + c);
-      t += u * C.c[4 * g + i];
-      f += u * C.f[4 * g + i];
+    for (int i = 0; i < ex_size(G, g); ++i) {
+      const unsigned u = (unsigned)r(ex_first(G, g) + i);
+      t += u * C.c[ex_first(G, g) + i];
+      f += u * C.f[ex_first(G, g) + i];
     }
-    const unsigned X = t - (f >> 20) * C.P[g];  // in [0, 1.002 P_g), below 2^32
-    qs += __umulhi(X, C.G[g]);                  // 2^20 X / P_g
+    const unsigned X = t - (f >> 20) * C.P[g];  // in [0, 1.002 P_g)
+    qs += __umulhi(X, C.G[g]);                  // X / P_g
 #pragma unroll
-    for (int s = 0; s < NL; ++s) acc[s] += (unsigned long long)X * C.W[g][s];
+    for (int s = 0; s < NW - 1; ++s) acc[s] += (unsigned long long)X * C.W[g][s];
+    if (G < 7) top += X * C.W[g][NW - 1];  // 28 and 32 moduli: W_g < 2^192, 2^224
   }
-  const unsigned q = (qs + (1u << 19)) >> 20;
-  long long carry = 0;
-  unsigned long long word[4] = {0, 0, 0, 0};
+  const unsigned q = qs >> (ex_shift(G) - 32);
+  unsigned w[NW];
+  unsigned long long carry = 0;
 #pragma unroll
-  for (int s = 0; s < NL; ++s) {
-    const long long z = (long long)acc[s] - (long long)((unsigned long long)q * C.M[s]) + carry;
-    const int off = (28 * s) & 63, wi = (28 * s) >> 6;
-    if (s < NL - 1) {
-      const unsigned long long d = (unsigned long long)z & 0xFFFFFFFull;
-      carry = z >> 28;
-      word[wi] |= d << off;
-      if (off > 36) word[wi + 1] |= d >> (64 - off);
-    } else {  // the top limb carries the sign
-      word[wi] |= (unsigned long long)z << off;
+  for (int s = 0; s < NW - 1; ++s) {
+    carry += acc[s] + (unsigned long long)q * C.Mneg[s];
+    w[s] = (unsigned)carry;
+    carry >>= 32;
+  }
+  w[NW - 1] = top + q * C.Mneg[NW - 1] + (unsigned)carry;
+  const bool neg = (int)w[NW - 1] < 0;
+  const unsigned sg = neg ? 0xFFFFFFFFu : 0u;
+  carry = sg & 1u;
 #pragma unroll
-      for (int v = wi + 1; v < 4; ++v)
-        word[v] = (unsigned long long)(v == wi + 1 && off ? z >> (64 - off) : z >> 63);
+  for (int s = 0; s < NW; ++s) {
+    carry += w[s] ^ sg;
+    w[s] = (unsigned)carry;
+    carry >>= 32;
+  }
+  // the three words from the leading nonzero one, and whether anything is below
+  unsigned below[NW];
+  below[0] = w[0];
+#pragma unroll
+  for (int s = 1; s < NW; ++s) below[s] = below[s - 1] | w[s];
+  unsigned h = w[NW - 1], m = w[NW - 2], l = NW > 2 ? w[NW > 2 ? NW - 3 : 0] : 0, rest = NW > 3 ? below[NW > 3 ? NW - 4 : 0] : 0;
+  int field = 32 * NW - 1 + e + 1023;
+#pragma unroll
+  for (int s = 1; s < NW; ++s)
+    if (h == 0) {
+      h = m;
+      m = l;
+      l = NW - 3 - s >= 0 ? w[NW - 3 - s >= 0 ? NW - 3 - s : 0] : 0;
+      rest = NW - 4 - s >= 0 ? below[NW - 4 - s >= 0 ? NW - 4 - s : 0] : 0;
+      field -= 32;
     }
-  }
-  const bool neg = (long long)word[3] < 0;
-  if (neg) {
-    unsigned long long cy = 1;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      word[v] = ~word[v] + cy;
-      cy = cy && word[v] == 0;
-    }
-  }
-  return ex_round(word, neg, e);
+  if (h == 0) return 0.0;
+  const int s = __clz((int)h);
+  field -= s;
+  const unsigned t3 = __funnelshift_l(m, h, s), t2 = __funnelshift_l(l, m, s);
+  rest = (rest | (l << s)) != 0 ? 1u : 0u;
+  if (field < 1 || field > 2045) return ex_outside_normal(t3, t2, rest != 0, neg, field);
+  const unsigned up = (((t2 & 0x7FFu) | rest) + 0x3FFu + ((t2 >> 11) & 1u)) >> 11;  // as i128_scaled
+  const unsigned head = ((unsigned)(field - 1) << 20) + (t3 >> 11) + (neg ? 0x80000000u : 0u);
+  return __longlong_as_double((long long)((((unsigned long long)head << 32) | ((t3 << 21) | (t2 >> 11))) + up));
 }
 
 // TI rows x 128 columns a block (32 x 8 threads), four neighbouring columns of a row per thread,
 // transposed through shared memory as in crt_combine_blk.  TI = 32 writes whole 256-byte runs of
-// Q's columns; small outputs take TI = 8, four times the blocks, each with a quarter of the serial
-// recombinations (n = 256: 16 blocks are a tenth of the SMs).
+// Q's columns; smaller outputs take TI = 8, four times the blocks, each with a quarter of the serial
+// recombinations.
 template <int G, int TI>
 __device__ __forceinline__ void ex_combine(const int8_t* __restrict__ R, int n, int k, int kr,
                                            const int* __restrict__ alsb, const int* __restrict__ hlsb, double alpha,
-                                           double beta, double* __restrict__ Q, long ldq, double (&tile)[128][TI]) {
+                                           double beta, double* __restrict__ Q, long ldq, double (&tile)[32][4 * TI + 1]) {
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i0 = blockIdx.y * TI, j0 = blockIdx.x * 128, jb = j0 + 4 * tx;
   const size_t plane = (size_t)n * kr;
@@ -559,42 +571,76 @@ __device__ __forceinline__ void ex_combine(const int8_t* __restrict__ R, int n, 
     const int il = ty + 8 * a, i = i0 + il;
     double val[4] = {0.0, 0.0, 0.0, 0.0};
     if (i < n && jb < k) {
-      unsigned w[EX_MAX];
+      unsigned w[4 * G];
       const int8_t* rp = R + (size_t)i * kr + jb;
 #pragma unroll
-      for (int l = 0; l < 4 * G; ++l) w[l] = __ldg((const unsigned*)(rp + (size_t)l * plane)) ^ 0x80808080u;
+      for (int l = 0; l < 4 * G; ++l) w[l] = __ldg((const unsigned*)(rp + (size_t)l * plane));
       const int ea = alsb[i];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int eh = jb + c < k ? hlsb[jb + c] : NO_LSB;
-        if (ea != NO_LSB && eh != NO_LSB) val[c] = ex_crt<G>(w, c, ea + eh);
+        if (ea != NO_LSB && eh != NO_LSB)
+          val[c] = ex_crt<G>([&](int l) { return (int)(int8_t)(w[l] >> (8 * c)); }, ea + eh);
       }
     }
 #pragma unroll
-    for (int c = 0; c < 4; ++c) tile[4 * tx + c][(il + tx) & (TI - 1)] = val[c];
+    for (int c = 0; c < 4; ++c) tile[tx][c * TI + il] = val[c];
   }
   __syncthreads();
   const bool scale = alpha != 1.0, accumulate = beta != 0.0;
-  const int t = ty * 32 + tx, ir = t % TI, i = i0 + ir;
-  for (int jl = t / TI; jl < 128; jl += 256 / TI) {
-    const int jj = j0 + jl;
-    if (i < n && jj < k) {
-      double* qp = Q + i + (long)jj * ldq;
-      double v = tile[jl][(ir + (jl >> 2)) & (TI - 1)];
-      if (scale || accumulate) {
-        v *= alpha;
-        if (accumulate) v = fma(beta, *qp, v);
+  const int t = ty * 32 + tx, ir = t % TI, i = i0 + ir, left = i < n ? k - j0 : 0;
+  double* qp = Q + i + (long)(j0 + t / TI) * ldq;
+#pragma unroll
+  for (int u0 = 0; u0 < TI / 2; u0 += 4) {
+    double q[4];
+    const double* ql = qp;
+#pragma unroll
+    for (int u = 0; u < 4; ++u, ql += ldq * (256 / TI)) q[u] = accumulate && t / TI + (u0 + u) * (256 / TI) < left ? *ql : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u, qp += ldq * (256 / TI)) {
+      const int jl = t / TI + (u0 + u) * (256 / TI);
+      if (jl < left) {
+        double v = tile[jl >> 2][(jl & 3) * TI + ir];
+        if (scale || accumulate) {
+          v *= alpha;
+          if (accumulate) v = fma(beta, q[u], v);
+        }
+        *qp = v;
       }
-      *qp = v;
     }
   }
 }
 
+// One element a thread, 8 rows x 32 columns a block, for the smallest outputs: the four serial recombinations of a
+// thread are most of the pass there.
+template <int G>
+__device__ __forceinline__ void ex_combine_one(const int8_t* __restrict__ R, int n, int k, int kr,
+                                               const int* __restrict__ alsb, const int* __restrict__ hlsb, double alpha,
+                                               double beta, double* __restrict__ Q, long ldq) {
+  const int i = blockIdx.y * 8 + threadIdx.y, j = blockIdx.x * 32 + threadIdx.x;
+  if (i >= n || j >= k) return;
+  const size_t plane = (size_t)n * kr;
+  const int8_t* rp = R + (size_t)i * kr + j;
+  int8_t b[4 * G];
+#pragma unroll
+  for (int l = 0; l < 4 * G; ++l) b[l] = __ldg(rp + (size_t)l * plane);
+  const int ea = alsb[i], eh = hlsb[j];
+  double* qp = Q + i + (long)j * ldq;
+  double v = 0.0;
+  if (ea != NO_LSB && eh != NO_LSB) v = ex_crt<G>([&](int l) { return (int)b[l]; }, ea + eh);
+  if (alpha != 1.0 || beta != 0.0) {
+    v *= alpha;
+    if (beta != 0.0) v = fma(beta, *qp, v);
+  }
+  *qp = v;
+}
+
+// TI = 1: ex_combine_one.
 template <int TI>
 __global__ void __launch_bounds__(256, 2) k_ex_combine(const int8_t* __restrict__ R, int n, int k, int kr, ExParams* prm,
                                                     const int* __restrict__ alsb, const int* __restrict__ hlsb,
                                                     double alpha, double beta, double* __restrict__ Q, long ldq) {
-  __shared__ double tile[128][TI];
+  __shared__ double tile[32][4 * TI + 1];
   const int nmod = prm->nmod;
   if (nmod == 0) return;
   if (prm->status != 0) {  // a wait of the GEMM gave up: the DMMA kernel computes the product
@@ -602,13 +648,21 @@ __global__ void __launch_bounds__(256, 2) k_ex_combine(const int8_t* __restrict_
     return;
   }
   switch (nmod / 4) {
-    case 2: ex_combine<2, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
-    case 3: ex_combine<3, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
-    case 4: ex_combine<4, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
-    case 5: ex_combine<5, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
-    case 6: ex_combine<6, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
-    case 7: ex_combine<7, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
-    default: ex_combine<8, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile); break;
+#define PSMMA_COMBINE(G)                                                       \
+  case G:                                                                      \
+    if constexpr (TI == 1)                                                     \
+      ex_combine_one<G>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq);         \
+    else                                                                       \
+      ex_combine<G, TI>(R, n, k, kr, alsb, hlsb, alpha, beta, Q, ldq, tile);   \
+    break;
+    PSMMA_COMBINE(2)
+    PSMMA_COMBINE(3)
+    PSMMA_COMBINE(4)
+    PSMMA_COMBINE(5)
+    PSMMA_COMBINE(6)
+    PSMMA_COMBINE(7)
+    PSMMA_COMBINE(8)
+#undef PSMMA_COMBINE
   }
 }
 
@@ -720,7 +774,10 @@ int launch_exact(int M, int N, int K, double alpha, const double* A, long lda, c
   if (st) return st;
   prof_mark(stream, "modular_gemm");
   const int cols = (N + 127) / 128;
-  if ((long)cols * ((M + 31) / 32) >= 4L * sms)
+  if ((long)cols * ((M + 7) / 8) < 2L * sms)
+    k_ex_combine<1><<<dim3((N + 31) / 32, (M + 7) / 8), dim3(32, 8), 0, stream>>>(R, M, N, L.kr, prm, alsb, hlsb, alpha, beta,
+                                                                                Q, ldq);
+  else if ((long)cols * ((M + 31) / 32) >= 4L * sms)
     k_ex_combine<32><<<dim3(cols, (M + 31) / 32), dim3(32, 8), 0, stream>>>(R, M, N, L.kr, prm, alsb, hlsb, alpha, beta,
                                                                             Q, ldq);
   else

@@ -15,35 +15,31 @@ MODULI = [256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 211, 199, 197, 
           217, 181, 179, 173, 167, 163, 157, 151, 149, 139, 137, 131, 127, 113, 109, 107]
 
 
-def _group_consts(G):
-    M = math.prod(MODULI[:4 * G])
-    out = []
-    for g in range(G):
-        ms = MODULI[4 * g:4 * g + 4]
-        P = math.prod(ms)
-        W = M // P
-        c = [(P // m) * (pow(W % m, -1, m) * pow(P // m % m, -1, m) % m) for m in ms]
-        b = -sum(128 * x for x in c) % P
-        out.append((ms, P, W, c, [(x << 20) // P for x in c], b, (b << 20) // P, (1 << 52) // P))
-    return M, out
+def _parts(G):
+    sizes = [3, 3, 2] if G == 2 else [3] * ((4 * G - 4 * (4 * G % 3)) // 3) + [4] * (4 * G % 3)
+    first = [sum(sizes[:i]) for i in range(len(sizes))]
+    return [MODULI[f:f + n] for f, n in zip(first, sizes)]
 
 
 @pytest.mark.parametrize("G", range(2, 9))
 def test_grouped_crt_recovers_the_integer(G):
-    # the kernel's 32-bit group step, quotient estimates and 28-bit limbs restated in Python
+    # the kernel's 32-bit part step, quotient estimates and sums of 32-bit limbs restated in Python
     # integers with its word sizes, at both ends of the range and at random Z, from any
     # representatives of the residues in [-128, 127]
-    M, groups = _group_consts(G)
+    M, shift = math.prod(MODULI[:4 * G]), 47 if G == 2 else 52
     assert all(math.gcd(a, b) == 1 for i, a in enumerate(MODULI) for b in MODULI[:i])
-    assert M < 1 << (28 * (G + 1) - 1)
+    assert sum(map(len, _parts(G))) == 4 * G and M < 1 << (32 * G)
     rng = np.random.default_rng(G)
     top = int(0.497 * M)
     cases = [0, 1, -1, top, -top, M // 3] + [int.from_bytes(rng.bytes(32), "little") % (2 * top) - top
                                              for _ in range(200)]
     for Z in cases:
-        acc = [0] * (G + 1)
-        qs = 0
-        for ms, P, W, c, f, b, fb, Gc in groups:
+        acc, qs = [0] * G, 1 << (shift - 33)
+        for ms in _parts(G):
+            P = math.prod(ms)
+            W = M // P
+            c = [(P // m) * (pow(W % m, -1, m) * pow(P // m % m, -1, m) % m) for m in ms]
+            b = -sum(128 * x for x in c) % P
             u = []
             for m in ms:
                 r = Z % m
@@ -51,16 +47,22 @@ def test_grouped_crt_recovers_the_integer(G):
                 assert -128 <= r <= 127
                 u.append(r + 128)
             t = (b + sum(x * y for x, y in zip(u, c))) % (1 << 32)
-            est = fb + sum(x * y for x, y in zip(u, f))
-            assert est < 1 << 32
+            est = (b << 20) // P + sum(x * ((y << 20) // P) for x, y in zip(u, c))
+            assert est < 1 << 32 and (1 << shift) // P < 1 << 32
             X = (t - (est >> 20) * P) % (1 << 32)
             assert X < 1.002 * P and (X - b - sum(x * y for x, y in zip(u, c))) % P == 0
-            qs += (X * Gc) >> 32
-            for s in range(G + 1):
-                acc[s] += X * ((W >> (28 * s)) & 0xFFFFFFF)
-        assert max(acc) < 1 << 63
-        q = (qs + (1 << 19)) >> 20
-        assert sum(a << (28 * s) for s, a in enumerate(acc)) - q * M == Z
+            qs += (X * ((1 << shift) // P)) >> 32
+            for s in range(G):
+                acc[s] += X * ((W >> (32 * s)) & 0xFFFFFFFF)
+            assert G < 7 or W < 1 << (32 * (G - 1))
+        assert max(acc[:G - 1]) < 1 << 63
+        q, carry, out = qs >> (shift - 32), 0, 0
+        for s in range(G):
+            v = acc[s] + q * ((((1 << 256) - M) >> (32 * s)) & 0xFFFFFFFF) + carry
+            assert s == G - 1 or v < 1 << 64
+            out |= (v & 0xFFFFFFFF) << (32 * s)
+            carry = v >> 32
+        assert out - ((1 << (32 * G)) if out >> (32 * G - 1) else 0) == Z
 
 
 def test_residue_chunks_stay_exact_in_fp32():
