@@ -185,6 +185,7 @@ ExLayout ex_layout(int M, int N, int K, int planes) {
 // Passes
 // ------------------------------------------------------------------------------------------
 __global__ void k_ex_init(ExParams* prm, unsigned long long* amax, double* asq, int* alsb, int M) {
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *prm = ExParams{0u, 0, 0, 0, 1u};
   if (i < M) {
@@ -197,12 +198,14 @@ __global__ void k_ex_init(ExParams* prm, unsigned long long* amax, double* asq, 
 __global__ void k_ex_row_stats(const double* __restrict__ A, long lda, int n, int k, int kchunk,
                                unsigned long long* __restrict__ amax, double* __restrict__ asq,
                                int* __restrict__ alsb) {
+  grid_wait();
   row_absmax_blk<true>(A, lda, nullptr, 0, k, n, k, kchunk, amax, asq, blockIdx.x, blockIdx.y, alsb);
 }
 
 template <int KIND>
 __global__ void k_ex_h(GenSpec gs, int K, int kp, double* __restrict__ Ht, unsigned long long* __restrict__ hmax,
                        double* __restrict__ hsum, double* __restrict__ hsq, int* __restrict__ hlsb) {
+  grid_wait();
   h_pass1_blk<KIND, true>(gs, K, kp, Ht, hmax, hsum, hsq, nullptr, blockIdx.x, nullptr, hlsb);
 }
 
@@ -214,6 +217,7 @@ __global__ void __launch_bounds__(256) k_ex_stats(GenSpec gs, int M, int N, int 
                                                   double* __restrict__ Ht, unsigned long long* __restrict__ hmax,
                                                   double* __restrict__ hsum, double* __restrict__ hsq,
                                                   int* __restrict__ hlsb) {
+  grid_wait();
   const int rb = (M + SMALL_RB - 1) / SMALL_RB, b = blockIdx.x;
   if (b < rb)
     small_rows_blk<true>(A, lda, M, K, b, amax, asq, alsb);
@@ -296,6 +300,7 @@ __device__ __forceinline__ ExParams ex_params(const ExStats& st, const ExLog2& l
 
 __global__ void __launch_bounds__(1024) k_ex_params(ExParams* prm, ExLog2 lg, int max_groups, int M, int N, int K,
                                                     ExStats st) {
+  grid_wait();
   const ExParams p = ex_params(st, lg, max_groups, M, N, K);
   if (threadIdx.x == 0) *prm = p;
 }
@@ -404,6 +409,7 @@ __device__ __forceinline__ void ex_residues_A_blk(const double* __restrict__ A, 
 __global__ void __launch_bounds__(256) k_ex_residues_A(const double* __restrict__ A, long lda, int n, int k, int kp,
                                                        const int* __restrict__ alsb, const ExParams* prm,
                                                        __nv_bfloat16* __restrict__ RA) {
+  grid_wait();
   const int nmod = prm->nmod;
   if (nmod == 0) return;
   ex_residues_A_blk(A, lda, n, k, kp, alsb, nmod, prm->ncA, RA, blockIdx.x, blockIdx.y);
@@ -424,6 +430,7 @@ __device__ __forceinline__ void ex_residues_H_quad(const double* __restrict__ Ht
 __global__ void __launch_bounds__(128) k_ex_residues_H(const double* __restrict__ Ht, int ncols, int kp,
                                                        const int* __restrict__ hlsb, const ExParams* prm,
                                                        __nv_bfloat16* __restrict__ RH) {
+  grid_wait();
   const int nmod = prm->nmod;
   if (nmod == 0) return;
   const int j = blockIdx.x, kk = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
@@ -439,6 +446,7 @@ __global__ void __launch_bounds__(256) k_ex_residues(const double* __restrict__ 
                                                      const double* __restrict__ Ht, __nv_bfloat16* __restrict__ RA,
                                                      __nv_bfloat16* __restrict__ RH, ExParams* prm) {
   __shared__ ExParams sp;
+  grid_wait();
   if (INLINE) {
     const ExParams p = ex_params(st, lg, max_groups, M, N, K);
     if (threadIdx.x == 0) {
@@ -641,6 +649,7 @@ __global__ void __launch_bounds__(256, 2) k_ex_combine(const int8_t* __restrict_
                                                     const int* __restrict__ alsb, const int* __restrict__ hlsb,
                                                     double alpha, double beta, double* __restrict__ Q, long ldq) {
   __shared__ double tile[32][4 * TI + 1];
+  grid_wait();
   const int nmod = prm->nmod;
   if (nmod == 0) return;
   if (prm->status != 0) {  // a wait of the GEMM gave up: the DMMA kernel computes the product
@@ -738,12 +747,12 @@ int launch_exact(int M, int N, int K, double alpha, const double* A, long lda, c
     prof_mark(stream, "statistics");
     const int a_blocks = ((M + 63) / 64) * (L.kp / 64), h_blocks = (N * (L.kp / 4) + 255) / 256;
     if (M + N <= INLINE_ROWS) {
-      k_ex_residues<true><<<a_blocks + h_blocks, 256, 0, stream>>>(A, lda, M, N, K, L.kp, xs, lg, planes / 4, a_blocks, Ht, RA,
-                                                                   RH, prm);
+      launch_behind(true, k_ex_residues<true>, a_blocks + h_blocks, 256, 0, stream, A, lda, M, N, K, L.kp, xs, lg, planes / 4,
+                    a_blocks, Ht, RA, RH, prm);
     } else {
-      k_ex_params<<<1, 1024, 0, stream>>>(prm, lg, planes / 4, M, N, K, xs);
-      k_ex_residues<false><<<a_blocks + h_blocks, 256, 0, stream>>>(A, lda, M, N, K, L.kp, xs, lg, planes / 4, a_blocks, Ht,
-                                                                    RA, RH, prm);
+      launch_behind(true, k_ex_params, 1, 1024, 0, stream, prm, lg, planes / 4, M, N, K, xs);
+      launch_behind(true, k_ex_residues<false>, a_blocks + h_blocks, 256, 0, stream, A, lda, M, N, K, L.kp, xs, lg, planes / 4,
+                    a_blocks, Ht, RA, RH, prm);
     }
     prof_mark(stream, "residues");
   } else {
@@ -752,37 +761,41 @@ int launch_exact(int M, int N, int K, double alpha, const double* A, long lda, c
     // not a serial chain: n = 2048 at 1024-column chunks 208 us, n = 256 at 128 27 us
     int kchunk = 1024;
     while (kchunk > 16 && (long)((M + 127) / 128) * ((K + kchunk - 1) / kchunk) < 8L * sms) kchunk >>= 1;
-    k_ex_row_stats<<<dim3((M + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, stream>>>(A, lda, M, K, kchunk, amax, asq,
-                                                                                       alsb);
+    launch_behind(true, k_ex_row_stats, dim3((M + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, stream, A, lda, M, K, kchunk,
+                  amax, asq, alsb);
     prof_mark(stream, "row_scale");
     switch (gs.kind) {
-      case KIND_CAUCHY: k_ex_h<KIND_CAUCHY><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
-      case KIND_TOEPLITZ: k_ex_h<KIND_TOEPLITZ><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
-      case KIND_HANKEL: k_ex_h<KIND_HANKEL><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
-      case KIND_CAUCHY_EIG: k_ex_h<KIND_CAUCHY_EIG><<<N, 256, 0, stream>>>(gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
+#define PSMMA_H(KD) \
+  case KD: launch_behind(true, k_ex_h<KD>, N, 256, 0, stream, gs, K, L.kp, Ht, hmax, hsum, hsq, hlsb); break;
+      PSMMA_H(KIND_CAUCHY)
+      PSMMA_H(KIND_TOEPLITZ)
+      PSMMA_H(KIND_HANKEL)
+      PSMMA_H(KIND_CAUCHY_EIG)
+#undef PSMMA_H
       default: return PSMMA_EUNSUPPORTED;
     }
     prof_mark(stream, "h_generate");
-    k_ex_params<<<1, 1024, 0, stream>>>(prm, lg, planes / 4, M, N, K, xs);
+    launch_behind(true, k_ex_params, 1, 1024, 0, stream, prm, lg, planes / 4, M, N, K, xs);
     prof_mark(stream, "params");
-    k_ex_residues_A<<<dim3((M + 63) / 64, L.kp / 64), 256, 0, stream>>>(A, lda, M, K, L.kp, alsb, prm, RA);
+    launch_behind(true, k_ex_residues_A, dim3((M + 63) / 64, L.kp / 64), 256, 0, stream, A, lda, M, K, L.kp, alsb, prm, RA);
     prof_mark(stream, "residues_A");
-    k_ex_residues_H<<<dim3(N, (L.kp / 4 + 127) / 128), 128, 0, stream>>>(Ht, N, L.kp, hlsb, prm, RH);
+    launch_behind(true, k_ex_residues_H, dim3(N, (L.kp / 4 + 127) / 128), 128, 0, stream, Ht, N, L.kp, hlsb, prm, RH);
     prof_mark(stream, "residues_H");
   }
+  // the whole chain overlaps its launches: the route is never captured
   const int st = launch_modular_gemm(RA, RH, R, M, N, L.kp, L.kr, planes, kExModuli, &prm->nmod, &prm->status, sms, stream);
   if (st) return st;
   prof_mark(stream, "modular_gemm");
   const int cols = (N + 127) / 128;
   if ((long)cols * ((M + 7) / 8) < 2L * sms)
-    k_ex_combine<1><<<dim3((N + 31) / 32, (M + 7) / 8), dim3(32, 8), 0, stream>>>(R, M, N, L.kr, prm, alsb, hlsb, alpha, beta,
-                                                                                Q, ldq);
+    launch_behind(true, k_ex_combine<1>, dim3((N + 31) / 32, (M + 7) / 8), dim3(32, 8), 0, stream, R, M, N, L.kr, prm, alsb, hlsb,
+                  alpha, beta, Q, ldq);
   else if ((long)cols * ((M + 31) / 32) >= 4L * sms)
-    k_ex_combine<32><<<dim3(cols, (M + 31) / 32), dim3(32, 8), 0, stream>>>(R, M, N, L.kr, prm, alsb, hlsb, alpha, beta,
-                                                                            Q, ldq);
+    launch_behind(true, k_ex_combine<32>, dim3(cols, (M + 31) / 32), dim3(32, 8), 0, stream, R, M, N, L.kr, prm, alsb, hlsb,
+                  alpha, beta, Q, ldq);
   else
-    k_ex_combine<8><<<dim3(cols, (M + 7) / 8), dim3(32, 8), 0, stream>>>(R, M, N, L.kr, prm, alsb, hlsb, alpha, beta, Q,
-                                                                         ldq);
+    launch_behind(true, k_ex_combine<8>, dim3(cols, (M + 7) / 8), dim3(32, 8), 0, stream, R, M, N, L.kr, prm, alsb, hlsb, alpha,
+                  beta, Q, ldq);
   prof_mark(stream, "crt_combine");
   return cudaGetLastError() == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
 }

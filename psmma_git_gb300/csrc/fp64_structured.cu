@@ -295,6 +295,7 @@ __device__ __forceinline__ void struct_f64_tile(const F64Args& p, int bx, int by
 
 template <int KIND>
 __global__ void __launch_bounds__(F64_THREADS, 1) k_struct_f64(F64Args p) {
+  grid_wait();
   if (p.gate && *p.gate == 0u) return;
   struct_f64_tile<KIND>(p, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -302,6 +303,7 @@ __global__ void __launch_bounds__(F64_THREADS, 1) k_struct_f64(F64Args p) {
 // C := beta * C + sum_z W_z over the S split-K partials, in split order (deterministic).
 __global__ void k_splitk_reduce(double* __restrict__ C, long ldc, const double* __restrict__ W, long ldw, int M,
                                 int N, int S, double beta, const unsigned* gate) {
+  grid_wait();
   if (gate && *gate == 0u) return;
   const long total = (long)M * N;
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
@@ -418,7 +420,7 @@ int launch_struct_f64_ws(int M, int N, int K, double alpha, const double* X, lon
         return PSMMA_EDEVICE;                                                                 \
       attr_set = true;                                                                        \
     }                                                                                         \
-    k_struct_f64<KD><<<grid, F64_THREADS, F64_SMEM_BYTES, stream>>>(p);                       \
+    launch_behind(gate != nullptr, k_struct_f64<KD>, grid, F64_THREADS, F64_SMEM_BYTES, stream, p); \
     break;                                                                                    \
   }
     PSMMA_LAUNCH_F64(KIND_CAUCHY)
@@ -434,7 +436,7 @@ int launch_struct_f64_ws(int M, int N, int K, double alpha, const double* X, lon
   if (p.W) {
     const long total = (long)M * N;
     const int blocks = (int)std::min<long>((total + 255) / 256, 152L * 16);
-    k_splitk_reduce<<<blocks, 256, 0, stream>>>(C, ldc, p.W, p.ldw, M, N, (int)grid.z, beta, gate);
+    launch_behind(gate != nullptr, k_splitk_reduce, blocks, 256, 0, stream, C, ldc, p.W, p.ldw, M, N, (int)grid.z, beta, gate);
   }
   prof_mark(stream, "struct_gemm_f64");
   return cudaGetLastError() == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;

@@ -104,6 +104,31 @@ inline cudaError_t set_smem_attr(F* fn, int bytes) {
   return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
+// kernel<<<grid, block, smem, stream>>>(args...); with `behind`, its blocks may be resident before the stream's last
+// kernel, one of this library that the same call launched, has finished (programmatic dependent launch): it has to
+// pass grid_wait() before it touches memory.  For chains of kernels of a few microseconds; a stream that is captured
+// records plain launches (behind = false).
+template <class... P, class... A>
+inline void launch_behind(bool behind, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = stream;
+  c.attrs = &at;
+  c.numAttrs = behind ? 1 : 0;
+  (void)cudaLaunchKernelEx(&c, kernel, (P)args...);  // a refused launch stays the thread's last error, as with <<<>>>
+}
+#ifdef __CUDACC__
+// The stream's earlier work is complete and visible.  No early trigger: the next kernel's blocks come in as this one's
+// leave.  With griddepcontrol.launch_dependents behind the wait they were packed onto the SMs that had room (FP64
+// Toeplitz multiply, plain launches / trigger / wait alone: n = 256 46.8 / 46.1 / 32.8 us, 1024 131.7 / 117.7 / 115.9).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 // FP64 plain path (fp64_structured.cu).  Real GEMM C(MxN) = alpha*X*G + beta*C where one
 // operand is streamed (X, column-major, ldx) and the other generated.
 int launch_struct_f64(int M, int N, int K, double alpha, const double* X, long ldx, const GenSpec& gs,

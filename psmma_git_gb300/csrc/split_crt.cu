@@ -642,6 +642,7 @@ __global__ void __launch_bounds__(256) k_split_stats(GenSpec gs, int M, int N, i
                                                      unsigned long long* __restrict__ amax, double* __restrict__ asq,
                                                      double* __restrict__ Ht, unsigned long long* __restrict__ hmax,
                                                      double* __restrict__ hsum, double* __restrict__ hsq) {
+  grid_wait();
   const int rb = (M + SMALL_RB - 1) / SMALL_RB, b = blockIdx.x;
   if (b < rb)
     small_rows_blk<false>(A, lda, M, K, b, amax, asq, nullptr);
@@ -685,6 +686,7 @@ __global__ void __launch_bounds__(512) k_split_small_params(double log2M, int M,
                                                             const unsigned long long* __restrict__ hmax,
                                                             const double* __restrict__ hsum,
                                                             const double* __restrict__ hsq, SplitDevParams* prm) {
+  grid_wait();
   small_params(log2M, M, N, K, amax, asq, hmax, hsum, hsq, prm);
 }
 
@@ -699,6 +701,7 @@ __global__ void __launch_bounds__(256) k_split_residues(const double* __restrict
                                                         __nv_bfloat16* __restrict__ RA, __nv_bfloat16* __restrict__ RH,
                                                         SplitDevParams* out) {
   __shared__ SplitDevParams sp;
+  grid_wait();
   if (INLINE) {
     small_params(cc.log2M, M, N, K, amax, asq, hmax, hsum, hsq, &sp);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1578,6 +1581,7 @@ __global__ void __launch_bounds__((TS::kEpiWarps + 2) * 32, 1) k_crt_gemm(const 
   constexpr int EPI = TS::kEpiWarps;  // warps 0 .. EPI-1 drain, EPI issues TMA, EPI + 1 the MMAs
   using S = GemmShape<BN>;
   extern __shared__ uint8_t smem_raw[];
+  grid_wait();
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sA = base;
   uint8_t* sB = base + G_STAGES * G_A_BYTES;
@@ -2089,6 +2093,7 @@ __global__ void __launch_bounds__(256, 3) k_crt_combine8(const int8_t* __restric
                                                       const unsigned long long* __restrict__ hmax_bits,
                                                       const SplitDevParams* prm, double alpha, double beta,
                                                       double* __restrict__ Q, long ldq) {
+  grid_wait();
   crt_combine_blk<false, THREE, 8>(R, n, k, kr, cc, amax_bits, hmax_bits, prm, alpha, beta, Q, ldq, blockIdx.x, blockIdx.y);
 }
 
@@ -2187,6 +2192,7 @@ int launch_split(int kind, int n, int k, double alpha, const double* A, long lda
 
 // The device status of a call ORed into the stream's status word.
 __global__ void k_status_or(unsigned* acc, const unsigned* st) {
+  grid_wait();
   const unsigned v = *st;
   if (v) atomicOr(acc, v);
 }
@@ -2389,7 +2395,7 @@ int launch_dft_radix_combine(const double2* P, int nq, int k, const double2* wn,
   return cudaGetLastError() == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
 }
 
-static int split_status(SplitDevParams* prm, cudaStream_t stream, unsigned* status_dev_out) {
+static int split_status(SplitDevParams* prm, cudaStream_t stream, unsigned* status_dev_out, bool behind = false) {
   if (status_dev_out && status_dev_out != kStatusWait) {
     if (cudaMemcpyAsync(status_dev_out, &prm->status, sizeof(unsigned), cudaMemcpyDeviceToDevice, stream) !=
         cudaSuccess)
@@ -2400,7 +2406,7 @@ static int split_status(SplitDevParams* prm, cudaStream_t stream, unsigned* stat
     // asynchronous: the status joins the stream's word, reported by psmma_stream_status
     unsigned* acc = stream_status_word(stream);
     if (acc) {
-      k_status_or<<<1, 1, 0, stream>>>(acc, &prm->status);
+      launch_behind(behind, k_status_or, 1, 1, 0, stream, acc, (const unsigned*)&prm->status);
       return cudaGetLastError() == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
     }
   }
@@ -2446,7 +2452,8 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return PSMMA_EDEVICE;
-  if (!gate && small_operands(M, N, K)) {
+  const bool small = !gate && small_operands(M, N, K), behind = small && !stream_capturing(stream);
+  if (small) {
     const int blocks = N + (M + SMALL_RB - 1) / SMALL_RB;
     switch (gs.kind) {
 #define PSMMA_STATS(KD) \
@@ -2462,9 +2469,10 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
     prof_mark(stream, "statistics");
     const int a_blocks = (L.kp / 64) * ((M + 63) / 64), h_blocks = (N * (L.kp / 4) + 255) / 256;
     const bool in_line = M + N <= INLINE_ROWS;
-    if (!in_line) k_split_small_params<<<1, 512, 0, stream>>>(cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsum, b.hsq, b.prm);
-    (in_line ? k_split_residues<true> : k_split_residues<false>)<<<a_blocks + h_blocks, 256, 0, stream>>>(
-        A, lda, M, N, K, L.kp, b.amax, b.asq, b.hmax, b.hsum, b.hsq, a_blocks, b.Ht, cc, b.RA, b.RH, b.prm);
+    if (!in_line)
+      launch_behind(behind, k_split_small_params, 1, 512, 0, stream, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsum, b.hsq, b.prm);
+    launch_behind(behind, in_line ? k_split_residues<true> : k_split_residues<false>, a_blocks + h_blocks, 256, 0, stream, A, lda,
+                  M, N, K, L.kp, b.amax, b.asq, b.hmax, b.hsum, b.hsq, a_blocks, b.Ht, cc, b.RA, b.RH, b.prm);
     prof_mark(stream, "residues");
   } else {
     if (cudaMemsetAsync(w, 0, L.off_wtab, stream) != cudaSuccess) return PSMMA_EDEVICE;  // params, maxima, sums
@@ -2513,20 +2521,20 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
   ga.gate = gate;
   ga.gate_set = 1;
   const int total_tiles = ga.tiles_m * ga.tiles_n * nmod;
-  k_crt_gemm<G_BN, OneGemm><<<std::min(sms, total_tiles), G_THREADS, Shape::SMEM, stream>>>(og);
+  launch_behind(behind, k_crt_gemm<G_BN, OneGemm>, std::min(sms, total_tiles), G_THREADS, Shape::SMEM, stream, og);
   prof_mark(stream, "modular_gemm");
 
   dim3 gc((N + CRT_TJ - 1) / CRT_TJ, (M + CRT_TI - 1) / CRT_TI);
   if (!gate && (long)gc.x * gc.y < 4L * sms)
-    (cc.three ? k_crt_combine8<true> : k_crt_combine8<false>)<<<dim3(gc.x, (M + 7) / 8), dim3(32, 8), 0, stream>>>(
-        b.R, M, N, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq);
+    launch_behind(behind, cc.three ? k_crt_combine8<true> : k_crt_combine8<false>, dim3(gc.x, (M + 7) / 8), dim3(32, 8), 0, stream,
+                  b.R, M, N, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq);
   else
     (cc.three ? k_crt_combine<false, true> : k_crt_combine<false, false>)<<<gc, dim3(32, 8), 0, stream>>>(
         b.R, M, N, L.kr, cc, b.amax, b.hmax, b.prm, alpha, beta, Q, ldq, 0, gate);
   prof_mark(stream, "crt_combine");
   if (cudaGetLastError() != cudaSuccess) return PSMMA_EDEVICE;
 
-  return split_status(b.prm, stream, status_dev_out);
+  return split_status(b.prm, stream, status_dev_out, behind);
 }
 
 // The modular products of exact_crt.cu: R[l] (M x kr bytes) = RA[l] (M x kp) RH[l]^T (N x kp) mod
@@ -2536,7 +2544,7 @@ template <int BN>
 static int modular_gemm_launch(const OneGemm& og, int tiles, int sms, cudaStream_t stream) {
   using Shape = GemmShape<BN>;
   if (set_smem_attr(k_crt_gemm<BN, OneGemm>, (int)Shape::SMEM) != cudaSuccess) return PSMMA_EDEVICE;
-  k_crt_gemm<BN, OneGemm><<<std::min(sms, tiles), G_THREADS, Shape::SMEM, stream>>>(og);
+  launch_behind(true, k_crt_gemm<BN, OneGemm>, std::min(sms, tiles), G_THREADS, Shape::SMEM, stream, og);
   return PSMMA_OK;
 }
 
