@@ -209,7 +209,7 @@ __global__ void k_ex_h(GenSpec gs, int K, int kp, double* __restrict__ Ht, unsig
   h_pass1_blk<KIND, true>(gs, K, kp, Ht, hmax, hsum, hsq, nullptr, blockIdx.x, nullptr, hlsb);
 }
 
-// Both, for small operands: the first blocks 32 rows of A each (the longest), then a column of H each.
+// Both, for small operands: the first blocks SMALL_RB rows of A each, then a column of H each.
 template <int KIND>
 __global__ void __launch_bounds__(256) k_ex_stats(GenSpec gs, int M, int N, int K, int kp, const double* __restrict__ A,
                                                   long lda, unsigned long long* __restrict__ amax,

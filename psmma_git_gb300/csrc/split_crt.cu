@@ -633,7 +633,7 @@ __device__ __forceinline__ void residues_H_blk(const double* __restrict__ Ht, in
   residues_H_quad(Ht, ncols, kp, hmax_bits, ph >= 0 ? ph : prm->PH, cc, RH, by, kk, krows);
 }
 
-// Small operands (split_passes.cuh): the statistics of both operands in one launch, the first blocks 32 rows of
+// Small operands (split_passes.cuh): the statistics of both operands in one launch, the first blocks 8 rows of
 // A each (the longest), then a column of H each; the parameters (rho from the columns' sums); the residues
 // of both.
 template <int KIND>

@@ -130,27 +130,29 @@ __device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, lon
 // 73 us in nine launches, 47 in five; 1000 x 777 126 and 105).
 constexpr int SMALL_ROWS = 2048, SMALL_K = 1024, INLINE_ROWS = 1024;
 inline bool small_operands(int M, int N, int K) { return M + N <= SMALL_ROWS && K <= SMALL_K; }
-constexpr int SMALL_RB = 32;  // rows of A a statistics block covers, 256 threads
+constexpr int SMALL_RB = 8;  // rows of A a statistics block covers, 256 threads
 
-// Row maxima, squared norms (and lowest bits) of rows 32 b .. 32 b + 31 over all of K, not accumulated into
-// what was there: warp w takes columns w, w + 8, ...
+// Row maxima, squared norms (and lowest bits) of rows 8 b .. 8 b + 7 over all of K, not accumulated into
+// what was there: a warp takes 8 rows of 4 columns (64-byte runs), the block 32 columns a step, eight steps in
+// flight.  32 rows a block (whole 256-byte runs, a quarter of the blocks) left a chain of 16 such groups of loads at
+// K = 1024, the longest of the launch (Toeplitz n = 1024: FP64 114.1 -> 93.4 us, split 96.6 -> 81.2).
 template <bool LSB>
 __device__ __forceinline__ void small_rows_blk(const double* __restrict__ A, long lda, int n, int k, int b,
                                                unsigned long long* __restrict__ amax_bits, double* __restrict__ asq,
                                                int* __restrict__ alsb) {
-  __shared__ unsigned long long sm[8][32];
-  __shared__ double sq[8][32];
-  __shared__ int sl[8][32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, i = b * 32 + lane;
+  __shared__ unsigned long long sm[8][8];
+  __shared__ double sq[8][8];
+  __shared__ int sl[8][8];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, row = lane & 7, c0 = 4 * wid + (lane >> 3), i = b * SMALL_RB + row;
   unsigned long long mb = 0;
   float s32 = 0.0f;
   int e = NO_SCALE, lsb = NO_LSB;
   bool big = false;
-  for (int k0 = wid; k0 < k; k0 += 64) {
+  for (int k0 = c0; k0 < k; k0 += 256) {
     unsigned long long v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const int kk = k0 + 8 * u;
+      const int kk = k0 + 32 * u;
       v[u] = (i < n && kk < k) ? (unsigned long long)__double_as_longlong(__ldg(A + i + (long)kk * lda)) & ABS_MASK : 0ull;
     }
     unsigned long long gm = 0;
@@ -172,22 +174,31 @@ __device__ __forceinline__ void small_rows_blk(const double* __restrict__ A, lon
   }
   double q = 0.0;
   if (big) {  // entries 2^56 times the thread's first ones (or Inf/NaN): FP64 sum
-    for (int kk = wid; kk < k; kk += 8) {
+    for (int kk = c0; kk < k; kk += 32) {
       const double x = i < n ? __ldg(A + i + (long)kk * lda) : 0.0;
       q = fma(x, x, q);
     }
   } else if (e != NO_SCALE) {
     q = ldexp((double)s32, 2 * e);
   }
-  sm[wid][lane] = mb;
-  sq[wid][lane] = q;
-  if constexpr (LSB) sl[wid][lane] = lsb;
+#pragma unroll
+  for (int o = 8; o <= 16; o <<= 1) {
+    const unsigned long long ob = __shfl_xor_sync(0xffffffffu, mb, o);
+    mb = ob > mb ? ob : mb;
+    q += __shfl_xor_sync(0xffffffffu, q, o);
+    if constexpr (LSB) lsb = min(lsb, __shfl_xor_sync(0xffffffffu, lsb, o));
+  }
+  if (lane < 8) {
+    sm[wid][row] = mb;
+    sq[wid][row] = q;
+    if constexpr (LSB) sl[wid][row] = lsb;
+  }
   __syncthreads();
-  if (wid == 0 && i < n) {
+  if (threadIdx.x < 8 && i < n) {
     for (int w = 1; w < 8; ++w) {
-      mb = sm[w][lane] > mb ? sm[w][lane] : mb;
-      q += sq[w][lane];
-      if constexpr (LSB) lsb = min(lsb, sl[w][lane]);
+      mb = sm[w][row] > mb ? sm[w][row] : mb;
+      q += sq[w][row];
+      if constexpr (LSB) lsb = min(lsb, sl[w][row]);
     }
     amax_bits[i] = mb;
     asq[i] = q;
