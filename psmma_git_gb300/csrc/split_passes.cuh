@@ -125,10 +125,11 @@ __device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, lon
 
 // Small operands (M + N at most SMALL_ROWS, K at most SMALL_K): the statistics of A's rows and H's columns are one
 // launch, the residues of both another; up to INLINE_ROWS the latter's blocks each evaluate the parameters for
-// themselves (at 1024 + 1024 that costs more than a launch of one block between the two).  Their passes
-// take a few microseconds each, so that the launches set the time (CauchyEig n = 256 on the split precision
-// 73 us in nine launches, 47 in five; 1000 x 777 126 and 105).
-constexpr int SMALL_ROWS = 2048, SMALL_K = 1024, INLINE_ROWS = 1024;
+// themselves.  Their passes take a few microseconds each, so that the launches set the time.  Toeplitz, separate
+// passes / these, split: n = 1280 150 / 120 us, 2048 328 / 304, 3072 796 / 777; FP64: 1280 143 / 136, 2048 357 / 354,
+// 3072 901 / 904.  Parameters in line / in a launch of their own, split: n = 256 32.9 / 34, 384 37.0 / 36.4, 512
+// 41.4 / 39.9, 768 63.7 / 56.5.
+constexpr int SMALL_ROWS = 4096, SMALL_K = 2048, INLINE_ROWS = 512;
 inline bool small_operands(int M, int N, int K) { return M + N <= SMALL_ROWS && K <= SMALL_K; }
 constexpr int SMALL_RB = 8;  // rows of A a statistics block covers, 256 threads
 
