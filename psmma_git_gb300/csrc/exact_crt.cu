@@ -342,15 +342,16 @@ __device__ __forceinline__ ExChunks<NC> ex_chunks(double x, int lsb) {
   return r;
 }
 
-// Four neighbouring integers: one 8-byte store per plane.
+// Four neighbouring integers, moduli l0 .. l1 - 1: one 8-byte store per plane.
 template <int NC>
-__device__ __forceinline__ void ex_write_quad(const double (&x)[4], int lsb, bool ok, int nmod, uint2* dst,
+__device__ __forceinline__ void ex_write_quad(const double (&x)[4], int lsb, bool ok, int l0, int l1, uint2* dst,
                                               size_t plane_u2) {
   ExChunks<NC> c[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) c[q] = ex_chunks<NC>(ok ? x[q] : 0.0, lsb);
+  dst += (size_t)l0 * plane_u2;
 #pragma unroll 4
-  for (int l = 0; l < nmod; ++l) {
+  for (int l = l0; l < l1; ++l) {
     const float inv = kEx.g[l][0], mf = kEx.m[l];
     unsigned f[4];
 #pragma unroll
@@ -366,43 +367,46 @@ __device__ __forceinline__ void ex_write_quad(const double (&x)[4], int lsb, boo
   }
 }
 
-__device__ __forceinline__ void ex_write_quad_nc(int nc, const double (&x)[4], int lsb, bool ok, int nmod, uint2* dst,
+__device__ __forceinline__ void ex_write_quad_nc(int nc, const double (&x)[4], int lsb, bool ok, int l0, int l1, uint2* dst,
                                                  size_t plane_u2) {
   if (nc <= 4)
-    ex_write_quad<4>(x, lsb, ok, nmod, dst, plane_u2);
+    ex_write_quad<4>(x, lsb, ok, l0, l1, dst, plane_u2);
   else if (nc <= 6)
-    ex_write_quad<6>(x, lsb, ok, nmod, dst, plane_u2);
+    ex_write_quad<6>(x, lsb, ok, l0, l1, dst, plane_u2);
   else
-    ex_write_quad<8>(x, lsb, ok, nmod, dst, plane_u2);
+    ex_write_quad<8>(x, lsb, ok, l0, l1, dst, plane_u2);
 }
 
-// RA[l][i][kk], rows i, K-major: 64 x 64 tiles of A transposed through shared memory (element
-// (k, r) at column (r + k/4) mod 64 of row k: conflict-free both ways).
+// RA[l][i][kk], rows i, K-major: tiles of TR rows x 64 columns of A transposed through shared memory (element
+// (k, r) at column (r + k/4) mod TR of row k: conflict-free both ways).  64 rows read whole 512-byte runs;
+// 16 rows leave one quad a thread instead of a chain of four.
+template <int TR>
 __device__ __forceinline__ void ex_residues_A_blk(const double* __restrict__ A, long lda, int n, int k, int kp,
-                                                  const int* __restrict__ alsb, int nmod, int nc,
+                                                  const int* __restrict__ alsb, int l0, int l1, int nc,
                                                   __nv_bfloat16* __restrict__ RA, int bx, int by) {
-  __shared__ double tile[64][64];
-  const int i0 = bx * 64, k0 = by * 64;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int kk = ty; kk < 64; kk += 8) {
+  __shared__ double tile[64][TR];
+  constexpr int TX = TR < 32 ? TR : 32;
+  const int i0 = bx * TR, k0 = by * 64;
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+  for (int kk = ty; kk < 64; kk += 256 / TX) {
     const int gk = k0 + kk;
 #pragma unroll
-    for (int rr = tx; rr < 64; rr += 32) {
+    for (int rr = tx; rr < TR; rr += TX) {
       const int gi = i0 + rr;
-      tile[kk][(rr + (kk >> 2)) & 63] = (gi < n && gk < k) ? __ldg(A + gi + (long)gk * lda) : 0.0;
+      tile[kk][(rr + (kk >> 2)) & (TR - 1)] = (gi < n && gk < k) ? __ldg(A + gi + (long)gk * lda) : 0.0;
     }
   }
   __syncthreads();
   const size_t plane = (size_t)n * kp;
   const int tq = threadIdx.x & 15, tr = threadIdx.x >> 4;
-  for (int r = tr; r < 64; r += 16) {
+  for (int r = tr; r < TR; r += 16) {
     const int gi = i0 + r;
     if (gi >= n) continue;
     const int lsb = alsb[gi], kk = 4 * tq;
     double x[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) x[q] = tile[kk + q][(r + tq) & 63];
-    ex_write_quad_nc(nc, x, lsb, lsb != NO_LSB, nmod, (uint2*)(RA + (size_t)gi * kp + k0 + kk), plane / 4);
+    for (int q = 0; q < 4; ++q) x[q] = tile[kk + q][(r + tq) & (TR - 1)];
+    ex_write_quad_nc(nc, x, lsb, lsb != NO_LSB, l0, l1, (uint2*)(RA + (size_t)gi * kp + k0 + kk), plane / 4);
   }
 }
 
@@ -412,19 +416,19 @@ __global__ void __launch_bounds__(256) k_ex_residues_A(const double* __restrict_
   grid_wait();
   const int nmod = prm->nmod;
   if (nmod == 0) return;
-  ex_residues_A_blk(A, lda, n, k, kp, alsb, nmod, prm->ncA, RA, blockIdx.x, blockIdx.y);
+  ex_residues_A_blk<64>(A, lda, n, k, kp, alsb, 0, nmod, prm->ncA, RA, blockIdx.x, blockIdx.y);
 }
 
 // Entries kk .. kk + 3 of column j.
 __device__ __forceinline__ void ex_residues_H_quad(const double* __restrict__ Ht, int ncols, int kp,
-                                                   const int* __restrict__ hlsb, int nmod, int nc,
+                                                   const int* __restrict__ hlsb, int l0, int l1, int nc,
                                                    __nv_bfloat16* __restrict__ RH, int j, int kk) {
   const int lsb = hlsb[j];
   const double2 h01 = *(const double2*)(Ht + (size_t)j * kp + kk);
   const double2 h23 = *(const double2*)(Ht + (size_t)j * kp + kk + 2);
   const double x[4] = {h01.x, h01.y, h23.x, h23.y};
   const size_t plane = (size_t)ncols * kp;
-  ex_write_quad_nc(nc, x, lsb, lsb != NO_LSB, nmod, (uint2*)(RH + (size_t)j * kp + kk), plane / 4);
+  ex_write_quad_nc(nc, x, lsb, lsb != NO_LSB, l0, l1, (uint2*)(RH + (size_t)j * kp + kk), plane / 4);
 }
 
 __global__ void __launch_bounds__(128) k_ex_residues_H(const double* __restrict__ Ht, int ncols, int kp,
@@ -435,11 +439,13 @@ __global__ void __launch_bounds__(128) k_ex_residues_H(const double* __restrict_
   if (nmod == 0) return;
   const int j = blockIdx.x, kk = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
   if (kk >= kp) return;  // kp is a multiple of 64
-  ex_residues_H_quad(Ht, ncols, kp, hlsb, nmod, prm->ncH, RH, j, kk);
+  ex_residues_H_quad(Ht, ncols, kp, hlsb, 0, nmod, prm->ncH, RH, j, kk);
 }
 
-// Both, for small operands: blocks 0 .. a_blocks - 1 are the 64 x 64 tiles of A, the others 256 quads of H each.
-// INLINE: every block evaluates the parameters, block 0 publishes them.
+// Both, for small operands: blocks 0 .. a_blocks - 1 are the tiles of A, the others 256 quads of H each.
+// INLINE: every block evaluates the parameters, block 0 publishes them.  These launches do not fill the SMs: tiles of 16
+// rows, and blockIdx.y takes half of the moduli (an integer's 28 to 32 residues are the chain that is left).
+// Cauchy n = 256: 30.0 -> 26.7 us a call; at n = 2048 16 rows cost 2 %.
 template <bool INLINE>
 __global__ void __launch_bounds__(256) k_ex_residues(const double* __restrict__ A, long lda, int M, int N, int K, int kp,
                                                      ExStats st, ExLog2 lg, int max_groups, int a_blocks,
@@ -451,20 +457,22 @@ __global__ void __launch_bounds__(256) k_ex_residues(const double* __restrict__ 
     const ExParams p = ex_params(st, lg, max_groups, M, N, K);
     if (threadIdx.x == 0) {
       sp = p;
-      if (blockIdx.x == 0) *prm = p;
+      if (blockIdx.x == 0 && blockIdx.y == 0) *prm = p;
     }
   } else if (threadIdx.x == 0) {
     sp = *prm;
   }
   __syncthreads();
   if (sp.nmod == 0) return;
-  const int b = blockIdx.x;
+  const int b = blockIdx.x, half = sp.nmod / 2;  // nmod is a multiple of four
+  const int l0 = INLINE ? blockIdx.y * half : 0, l1 = INLINE ? l0 + half : sp.nmod;
   if (b < a_blocks) {
-    const int tm = (M + 63) / 64;
-    ex_residues_A_blk(A, lda, M, K, kp, st.alsb, sp.nmod, sp.ncA, RA, b % tm, b / tm);
+    constexpr int TR = INLINE ? 16 : 64;
+    const int tm = (M + TR - 1) / TR;
+    ex_residues_A_blk<TR>(A, lda, M, K, kp, st.alsb, l0, l1, sp.ncA, RA, b % tm, b / tm);
   } else {
     const int q = (b - a_blocks) * 256 + threadIdx.x, per = kp / 4, j = q / per;
-    if (j < N) ex_residues_H_quad(Ht, N, kp, st.hlsb, sp.nmod, sp.ncH, RH, j, 4 * (q - j * per));
+    if (j < N) ex_residues_H_quad(Ht, N, kp, st.hlsb, l0, l1, sp.ncH, RH, j, 4 * (q - j * per));
   }
 }
 
@@ -745,9 +753,9 @@ int launch_exact(int M, int N, int K, double alpha, const double* A, long lda, c
       default: return PSMMA_EUNSUPPORTED;
     }
     prof_mark(stream, "statistics");
-    const int a_blocks = ((M + 63) / 64) * (L.kp / 64), h_blocks = (N * (L.kp / 4) + 255) / 256;
+    const int tr = M + N <= INLINE_ROWS ? 16 : 64, a_blocks = ((M + tr - 1) / tr) * (L.kp / 64), h_blocks = (N * (L.kp / 4) + 255) / 256;
     if (M + N <= INLINE_ROWS) {
-      launch_behind(true, k_ex_residues<true>, a_blocks + h_blocks, 256, 0, stream, A, lda, M, N, K, L.kp, xs, lg, planes / 4,
+      launch_behind(true, k_ex_residues<true>, dim3(a_blocks + h_blocks, 2), 256, 0, stream, A, lda, M, N, K, L.kp, xs, lg, planes / 4,
                     a_blocks, Ht, RA, RH, prm);
     } else {
       launch_behind(true, k_ex_params, 1, 1024, 0, stream, prm, lg, planes / 4, M, N, K, xs);

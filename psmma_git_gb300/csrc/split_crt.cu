@@ -550,11 +550,12 @@ __device__ __forceinline__ void residues_A_blk(const double* __restrict__ A, lon
                                                __nv_bfloat16* __restrict__ RA, int bx, int by) {
   __shared__ double tile[64][TR];
   const int i0 = by * TR, k0 = bx * 64;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 256 threads: 8 x 32
-  for (int kk = ty; kk < 64; kk += 8) {
+  constexpr int TX = TR < 32 ? TR : 32;
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;  // 256 threads
+  for (int kk = ty; kk < 64; kk += 256 / TX) {
     const int gk = k0 + kk;
 #pragma unroll
-    for (int rr = tx; rr < TR; rr += 32) {
+    for (int rr = tx; rr < TR; rr += TX) {
       const int gi = i0 + rr;
       tile[kk][(rr + (kk >> 2)) & (TR - 1)] = (gi < n && gk < k) ? __ldg(acol(A, lda, A2, lda2, ka, gk) + gi) : 0.0;
     }
@@ -720,7 +721,8 @@ __global__ void __launch_bounds__(256) k_split_residues(const double* __restrict
   const int b = blockIdx.x;
   if (b < a_blocks) {
     const int tk = kp / 64;
-    residues_A_blk<64>(A, lda, nullptr, 0, K, M, K, kp, amax, &sp, cc, RA, b % tk, b / tk);
+    // in line, 16 rows: one quad a thread (Toeplitz n = 256 33.0 -> 27.3 us)
+    residues_A_blk<INLINE ? 16 : 64>(A, lda, nullptr, 0, K, M, K, kp, amax, &sp, cc, RA, b % tk, b / tk);
   } else {
     const int q = (b - a_blocks) * 256 + threadIdx.x, per = kp / 4, j = q / per;
     if (j < N) residues_H_quad(Ht, N, kp, hmax, sp.PH, cc, RH, j, 4 * (q - j * per), 1 << 30);
@@ -2467,8 +2469,8 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
       default: return PSMMA_EUNSUPPORTED;
     }
     prof_mark(stream, "statistics");
-    const int a_blocks = (L.kp / 64) * ((M + 63) / 64), h_blocks = (N * (L.kp / 4) + 255) / 256;
     const bool in_line = M + N <= INLINE_ROWS;
+    const int tr = in_line ? 16 : 64, a_blocks = (L.kp / 64) * ((M + tr - 1) / tr), h_blocks = (N * (L.kp / 4) + 255) / 256;
     if (!in_line)
       launch_behind(behind, k_split_small_params, 1, 512, 0, stream, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsum, b.hsq, b.prm);
     launch_behind(behind, in_line ? k_split_residues<true> : k_split_residues<false>, a_blocks + h_blocks, 256, 0, stream, A, lda,
