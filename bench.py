@@ -64,21 +64,6 @@ def ncu_traffic(n: int, nmod: int):
     return b0 * (nmod / m0) * (n / n0) ** 3
 
 
-def profile_traffic(tag: str):
-    """DRAM bytes per launch (ncu dram__bytes_read.sum + dram__bytes_write.sum) recorded as
-    ``traffic_bytes_per_launch_<tag>: <bytes>`` in a committed profile summary under
-    profiles/, or None."""
-    d = ROOT / "profiles"
-    if not d.is_dir():
-        return None
-    pat = re.compile(r"traffic_bytes_per_launch_" + re.escape(tag) + r":\s*([0-9.eE+]+)")
-    for f in sorted(d.glob("*.md")):
-        m = pat.search(f.read_text())
-        if m:
-            return float(m.group(1))
-    return None
-
-
 class Clocks:
     """nvidia-smi clock/throttle sampling during the timed region."""
     Q = ("clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,clocks_event_reasons.hw_slowdown,"
@@ -691,7 +676,7 @@ def run_cfg1(args, ws, rank, local, compact=False):
     oracle on a 256-row (DFT: 256-column) sample -- FFT correlation for Toeplitz/Hankel, FFT for
     the DFT, the explicit CauchylikeEig matrix (FP64 BLAS) for CAUCHYEIG, whose per-column
     maximum relative error is reported too (the eigensolver normalises columns).  Per kind a
-    roofline of the modular GEMMs (BF16, sustained peak) and of the FP64 path (in-run DGEMM),
+    roofline of the modular GEMMs (BF16, sustained peak) or of the transform that took their place, one of the FP64 path,
     and a CPU baseline: the oracle's restatement (ConstToeplitz / ConstHankel / CauchylikeEig
     of an H column panel + DGEMM; the DFT: a row panel of F times B by ZGEMM) on all host
     cores.  Returns the JSON object."""
@@ -854,21 +839,26 @@ def run_cfg1(args, ws, rank, local, compact=False):
                 cpu = {"value": 2.0 * n * k * cpu_cols / tc / 1e12, "unit": "TFLOP/s", "cores": os.cpu_count(),
                        "kind": "port", "sample": f"Q[:, 0:{cpu_cols}]: the H column panel by the oracle's "
                                                  f"restatement + DGEMM, {tc:.2f} s"}
+        byts = (32.0 if kind == "dft" else 16.0) * n * k
+        transform = {"ntt_rows": "k_ntt_rows", "dft_transform": "k_fft"}.get(
+            next((nm for nm, _ in phases if nm in ("ntt_rows", "dft_transform")), None))
+        if transform:  # no modular GEMM in the call (its gated fallback did not run)
+            roof = {"bound": "hbm", "achieved": byts / t / 1e6, "peak": pk["hbm"], "unit": "GB/s",
+                    "frac": byts / t / 1e6 / pk["hbm"], "traffic": None, "kernel": transform,
+                    "algorithmic_bytes": byts,
+                    "note": "whole call, operands read and result written once; the kernel is bound by integer issue"}
+        else:
+            roof = {"bound": "tensor", "achieved": gemm_flops / (gemm_ms * 1e-3) / 1e12 if gemm_ms else None,
+                    "peak": pk["bf16_sustained"], "unit": "TFLOP/s",
+                    "frac": gemm_flops / (gemm_ms * 1e-3) / 1e12 / pk["bf16_sustained"] if gemm_ms else None,
+                    "traffic": None, "kernel": "k_crt_gemm (modular BF16 GEMMs)", "flops_per_call": gemm_flops,
+                    "peak_note": f"{pk['source']} cuBLAS bf16 sustained"}
         out[kind] = {"split_ms": t, "split_tflops": flops / t / 1e9, "fp64_ms": t64,
                      "fp64_tflops": flops / t64 / 1e9, "speedup": t64 / t,
                      "rel_err_split_vs_fp64": rel, "rel_err_split_vs_oracle_sample": err_split,
                      "rel_err_fp64_vs_oracle_sample": err_64, "oracle": oracle,
-                     "roofline": {"bound": "tensor", "achieved": gemm_flops / (gemm_ms * 1e-3) / 1e12 if gemm_ms
-                                  else None, "peak": pk["bf16_sustained"], "unit": "TFLOP/s",
-                                  "frac": gemm_flops / (gemm_ms * 1e-3) / 1e12 / pk["bf16_sustained"]
-                                  if gemm_ms else None, "traffic": None, "kernel": "k_crt_gemm (modular BF16 GEMMs)",
-                                  "flops_per_call": gemm_flops,
-                                  "peak_note": f"{pk['source']} cuBLAS bf16 sustained"},
-                     "fp64_roofline": {"bound": "tensor", "achieved": flops / R64 / t64 / 1e9, "peak": dgemm,
-                                       "unit": "TFLOP/s", "frac": flops / R64 / t64 / 1e9 / dgemm,
-                                       "kernel": "k_struct_f64",
-                                       "peak_source": "cuBLAS DGEMM in this run; executed flops (the DFT's "
-                                                      "radix step runs 1/R of the dense flops)"},
+                     "roofline": roof,
+                     "fp64_roofline": fp64_roofline(flops / t64 / 1e9, dgemm, byts, t64, pk["hbm"], R64),
                      "cpu_baseline": cpu, "split_phases_ms": phases}
         if col_err is not None:
             out[kind]["col_max_rel_err_vs_oracle_sample"] = col_err
@@ -876,11 +866,13 @@ def run_cfg1(args, ws, rank, local, compact=False):
             out[kind]["e2e"] = e2e
         if kind in ("toeplitz", "hankel"):
             out[kind]["block_levels"] = levels
-            out[kind]["executed_tflops"] = flops * 0.75 ** levels / t / 1e9
+            if not transform:
+                out[kind]["executed_tflops"] = flops * 0.75 ** levels / t / 1e9
         if kind == "dft":
             out[kind]["split_complex_mac_tflops"] = 2.0 * n ** 3 / t / 1e9
-            out[kind]["radix"] = R
-            out[kind]["executed_real_tflops"] = 8.0 * n ** 3 / R / t / 1e9
+            if not transform:
+                out[kind]["radix"] = R
+                out[kind]["executed_real_tflops"] = 8.0 * n ** 3 / R / t / 1e9
         print(json.dumps({kind: {kk: vv for kk, vv in out[kind].items() if kk != "split_phases_ms"}}),
               file=sys.stderr, flush=True)
         del Y, Y64
@@ -894,6 +886,20 @@ def run_cfg1(args, ws, rank, local, compact=False):
                        "l2": "inputs 0.5-1 GiB > L2, no flush"},
             "cublas_dgemm_tflops": dgemm, "kinds": out}
     return line
+
+
+def fp64_roofline(rate, dgemm, byts, ms, hbm, executed=1.0):
+    """The FP64 path's roofline: the DMMA kernel's executed rate against cuBLAS DGEMM, or, where the call took a route
+    whose effective rate no FP64 GEMM reaches (modular products, transforms), its algorithmic bytes against the
+    memory's rate with the effective ratio beside it."""
+    if rate <= 1.05 * dgemm * executed:
+        return {"bound": "tensor", "achieved": rate / executed, "peak": dgemm, "unit": "TFLOP/s",
+                "frac": rate / executed / dgemm, "kernel": "k_struct_f64",
+                "peak_source": "cuBLAS DGEMM in this run; executed flops (the DFT's radix step runs 1/R of the dense flops)"}
+    return {"bound": "hbm", "achieved": byts / ms / 1e6, "peak": hbm, "unit": "GB/s", "frac": byts / ms / 1e6 / hbm,
+            "kernel": "modular products or transforms instead of k_struct_f64", "effective_over_dgemm": rate / dgemm,
+            "note": "algorithmic bytes (operands read, result written); integer issue and the modular GEMMs bound the "
+                    "route, not the memory"}
 
 
 def fp64_dgemm_rate(dev, stream):
@@ -919,7 +925,7 @@ def run_cfg0(args, ws, rank, local, compact=False):
     """Cauchy multiply on the FP64 plain path at n = k = 2048 over seeds 0..4 (A ~ U[-1,1],
     d = sort(U(0,1)), w_j ~ U(d_j, d_j+1), u, v ~ N(0,1)): median of the timed calls per seed
     (CUDA events, after args.warmup), error against the oracle's FP64 A@H, the split path
-    beside it, and the FP64 roofline against cuBLAS DGEMM measured in the same run.  e2e: the
+    beside it, and the FP64 roofline (cuBLAS DGEMM measured in the same run).  e2e: the
     same multiply through the host-pointer entry point (pinned host arrays, copies inside the
     timed region).  CPU baseline: the restatement of PSCAUCHY_COMPUTE on a 2 x 2 grid, block 64
     (4 emulated ranks), and a dense A@H, on all host cores.  Returns the JSON object."""
@@ -985,7 +991,6 @@ def run_cfg0(args, ws, rank, local, compact=False):
     t_dense = time.perf_counter() - t0
     fp64 = [s_["fp64"]["tflops"] for s_ in per_seed]
     v = float(np.median(fp64))
-    traffic = profile_traffic("fp64_cauchy_n2048")
     line = {"metric": "Cauchy A·H TFLOP/s n=2048, FP64 plain path (cfg0)", "value": v, "unit": "TFLOP/s",
             "n_gpus": 1, "steps": steps, "warmup": args.warmup,
             "ms_per_step": float(np.median([s_["fp64"]["ms"] for s_ in per_seed])), "higher_is_better": True,
@@ -996,13 +1001,9 @@ def run_cfg0(args, ws, rank, local, compact=False):
             "split_tflops_median": float(np.median([s_["split"]["tflops"] for s_ in per_seed])),
             "max_rel_err_vs_oracle": {p: max(s_[p]["rel_err_vs_oracle"] for s_ in per_seed)
                                       for p in ("fp64", "split")},
-            "roofline": {"bound": "tensor", "achieved": v, "peak": dgemm, "unit": "TFLOP/s", "frac": v / dgemm,
-                         "traffic": traffic, "kernel": "k_struct_f64<KIND_CAUCHY>",
-                         "algorithmic_bytes": 16.0 * n * n + 32.0 * n,
-                         "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64 tensor-core proxy; "
-                                        "MEASURED_PEAKS.json has no FP64 figure)",
-                         "traffic_source": "ncu dram__bytes_read+write of one launch (profiles/fp64_dmma_ncu.md)"
-                         if traffic else None},
+            "roofline": {**fp64_roofline(v, dgemm, 16.0 * n * n + 32.0 * n,
+                                         float(np.median([s_["fp64"]["ms"] for s_ in per_seed])), peaks()["hbm"]),
+                         "traffic": None, "algorithmic_bytes": 16.0 * n * n + 32.0 * n, "dgemm_tflops": dgemm},
             "e2e": {"value": flops / te / 1e12, "unit": "TFLOP/s", "h2d_bytes_per_step": 8 * n * n + 32 * n,
                     "d2h_bytes_per_step": 8 * n * n, "ms_per_step": te * 1e3, "steps": steps,
                     "api": "psmma_cauchy_host (pinned host buffers), FP64 path", "rel_err_vs_oracle": e2e_err},
@@ -1010,7 +1011,7 @@ def run_cfg0(args, ws, rank, local, compact=False):
                              "kind": "port", "sample": f"whole product, ring restatement 2x2 grid nb=64: "
                                                        f"{t_ring:.2f} s; dense A@H: {t_dense:.2f} s"},
             "ring_vs_dense_rel": O.rel_fro(Qr, dense),
-            "gpu_launches": 2 * 5 * (steps + args.warmup)}
+            "gpu_launches": 7 * 5 * (steps + args.warmup)}
     return line
 
 
