@@ -161,7 +161,9 @@ int psmma_split_dft_radix(int n);
  * k columns of Q written.  This returns the automatic choice (opts->block_levels = 0): the L
  * in {1, 2} with w = k' / 2^L >= 4096 that minimises the modular GEMM work (k'/k)^2 (3/4)^L,
  * if that is at most 0.85, else 0 (smaller leaves make the modular GEMMs' per-tile epilogue
- * outweigh their MMAs).  The
+ * outweigh their MMAs).  With the automatic choice, device-pointer calls of orders whose number-theoretic
+ * transform (2^13 to 2^15 points) is the faster one compute the same integer product by it instead, when the
+ * generator's columns allow one scale; a level asked for, or -1, keeps the modular products.  The
  * device-pointer calls, the host-pointer calls (in their overlapped row panels) and the server
  * take the step.  On the device, without a synchronisation, the call takes the single product
  * instead when an entry of H is not finite (NaN then appears in exactly the columns it does

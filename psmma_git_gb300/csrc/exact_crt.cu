@@ -11,7 +11,7 @@
 //   2. Row i times 2^-lsb_i and column j times 2^-lsb_j are integers without any rounding.  A bound
 //      of |Z_ij| = |(A'H')_ij| from the norms gives the number of moduli whose product exceeds
 //      2 |Z| (8 to 32 in steps of 4, up to 241 bits), on the device.
-//   3. One BF16 GEMM per modulus, the Chinese remainder theorem in 28-bit limbs, and one rounding
+//   3. One BF16 GEMM per modulus, the Chinese remainder theorem on 32-bit words, and one rounding
 //      of Z 2^(lsb_i + lsb_j) to FP64; then alpha and beta.
 // The rounded sum of exact products is at least as accurate as any order of FP64 additions.  Where
 // a row or column spans more than 112 bits, the bound exceeds the moduli, an entry is not finite or

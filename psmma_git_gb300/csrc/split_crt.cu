@@ -1884,15 +1884,11 @@ __global__ void __launch_bounds__((TS::kEpiWarps + 2) * 32, 1) k_crt_gemm(const 
 
 // ------------------------------------------------------------------------------------------
 // CRT recombination + FP64 epilogue: Q(i,j) = alpha * Z_ij * 2^-(s_i+f_j) + beta * Q(i,j).
-// 32 x 32 output tile per block (32 x 8 threads), transposed through shared memory so that
+// The tile is transposed through shared memory so that
 // both the residue reads (row-major) and the Q writes (column-major) are coalesced.
 // ------------------------------------------------------------------------------------------
-typedef unsigned __int128 u128;
-
-// One block: 32 rows x 128 columns (32 x 8 threads); a thread recombines 4 neighbouring
-// columns of one row per pass from 32-bit loads (4 residues) of each plane, so each warp
-// request moves 128 bytes.  Per modulus and element: four 32x32->64-bit multiply-adds for
-// the limbs of sum_l (r_l + 128) C_l and one for the fixed-point quotient estimate.
+// One block: 32 rows x 128 columns (32 x 8 threads); a thread recombines 4 neighbouring columns of a row at a
+// time from 32-bit loads (4 residues) of each plane, so each warp request moves 128 bytes.
 constexpr int CRT_TI = 32, CRT_TJ = 128;
 
 // The column of C^T that residue column rc of the 3M DFT layout holds (Re: rc < nn, Im: from
