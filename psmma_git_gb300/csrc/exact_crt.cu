@@ -443,10 +443,10 @@ __global__ void __launch_bounds__(128) k_ex_residues_H(const double* __restrict_
 }
 
 // Both, for small operands: blocks 0 .. a_blocks - 1 are the tiles of A, the others 256 quads of H each.
-// INLINE: every block evaluates the parameters, block 0 publishes them.  These launches do not fill the SMs: tiles of 16
-// rows, and blockIdx.y takes half of the moduli (an integer's 28 to 32 residues are the chain that is left).
-// Cauchy n = 256: 30.0 -> 26.7 us a call; at n = 2048 16 rows cost 2 %.
-template <bool INLINE>
+// INLINE: every block evaluates the parameters, block 0 publishes them; these launches do not fill the SMs, and
+// blockIdx.y takes half of the moduli (an integer's 28 to 32 residues are a serial chain).  With that and tiles of 16 rows:
+// Cauchy n = 256 30.0 -> 26.7 us a call.
+template <bool INLINE, int TR>
 __global__ void __launch_bounds__(256) k_ex_residues(const double* __restrict__ A, long lda, int M, int N, int K, int kp,
                                                      ExStats st, ExLog2 lg, int max_groups, int a_blocks,
                                                      const double* __restrict__ Ht, __nv_bfloat16* __restrict__ RA,
@@ -467,7 +467,6 @@ __global__ void __launch_bounds__(256) k_ex_residues(const double* __restrict__ 
   const int b = blockIdx.x, half = sp.nmod / 2;  // nmod is a multiple of four
   const int l0 = INLINE ? blockIdx.y * half : 0, l1 = INLINE ? l0 + half : sp.nmod;
   if (b < a_blocks) {
-    constexpr int TR = INLINE ? 16 : 64;
     const int tm = (M + TR - 1) / TR;
     ex_residues_A_blk<TR>(A, lda, M, K, kp, st.alsb, l0, l1, sp.ncA, RA, b % tm, b / tm);
   } else {
@@ -753,13 +752,13 @@ int launch_exact(int M, int N, int K, double alpha, const double* A, long lda, c
       default: return PSMMA_EUNSUPPORTED;
     }
     prof_mark(stream, "statistics");
-    const int tr = M + N <= INLINE_ROWS ? 16 : 64, a_blocks = ((M + tr - 1) / tr) * (L.kp / 64), h_blocks = (N * (L.kp / 4) + 255) / 256;
+    const int tr = small_tile_rows(M, N), a_blocks = ((M + tr - 1) / tr) * (L.kp / 64), h_blocks = (N * (L.kp / 4) + 255) / 256;
     if (M + N <= INLINE_ROWS) {
-      launch_behind(true, k_ex_residues<true>, dim3(a_blocks + h_blocks, 2), 256, 0, stream, A, lda, M, N, K, L.kp, xs, lg, planes / 4,
+      launch_behind(true, k_ex_residues<true, 16>, dim3(a_blocks + h_blocks, 2), 256, 0, stream, A, lda, M, N, K, L.kp, xs, lg, planes / 4,
                     a_blocks, Ht, RA, RH, prm);
     } else {
       launch_behind(true, k_ex_params, 1, 1024, 0, stream, prm, lg, planes / 4, M, N, K, xs);
-      launch_behind(true, k_ex_residues<false>, a_blocks + h_blocks, 256, 0, stream, A, lda, M, N, K, L.kp, xs, lg, planes / 4,
+      launch_behind(true, tr == 16 ? k_ex_residues<false, 16> : k_ex_residues<false, 64>, a_blocks + h_blocks, 256, 0, stream, A, lda, M, N, K, L.kp, xs, lg, planes / 4,
                     a_blocks, Ht, RA, RH, prm);
     }
     prof_mark(stream, "residues");

@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(512) k_split_small_params(double log2M, int M,
 }
 
 // INLINE: every block evaluates the parameters, block 0 publishes them.
-template <bool INLINE>
+template <bool INLINE, int TR>
 __global__ void __launch_bounds__(256) k_split_residues(const double* __restrict__ A, long lda, int M, int N, int K, int kp,
                                                         const unsigned long long* __restrict__ amax,
                                                         const double* __restrict__ asq,
@@ -721,8 +721,7 @@ __global__ void __launch_bounds__(256) k_split_residues(const double* __restrict
   const int b = blockIdx.x;
   if (b < a_blocks) {
     const int tk = kp / 64;
-    // in line, 16 rows: one quad a thread (Toeplitz n = 256 33.0 -> 27.3 us)
-    residues_A_blk<INLINE ? 16 : 64>(A, lda, nullptr, 0, K, M, K, kp, amax, &sp, cc, RA, b % tk, b / tk);
+    residues_A_blk<TR>(A, lda, nullptr, 0, K, M, K, kp, amax, &sp, cc, RA, b % tk, b / tk);
   } else {
     const int q = (b - a_blocks) * 256 + threadIdx.x, per = kp / 4, j = q / per;
     if (j < N) residues_H_quad(Ht, N, kp, hmax, sp.PH, cc, RH, j, 4 * (q - j * per), 1 << 30);
@@ -2466,10 +2465,11 @@ static int split_core(int M, int N, int K, double alpha, const double* A, long l
     }
     prof_mark(stream, "statistics");
     const bool in_line = M + N <= INLINE_ROWS;
-    const int tr = in_line ? 16 : 64, a_blocks = (L.kp / 64) * ((M + tr - 1) / tr), h_blocks = (N * (L.kp / 4) + 255) / 256;
+    const int tr = small_tile_rows(M, N), a_blocks = (L.kp / 64) * ((M + tr - 1) / tr), h_blocks = (N * (L.kp / 4) + 255) / 256;
     if (!in_line)
       launch_behind(behind, k_split_small_params, 1, 512, 0, stream, cc.log2M, M, N, K, b.amax, b.asq, b.hmax, b.hsum, b.hsq, b.prm);
-    launch_behind(behind, in_line ? k_split_residues<true> : k_split_residues<false>, a_blocks + h_blocks, 256, 0, stream, A, lda,
+    launch_behind(behind, in_line ? k_split_residues<true, 16> : tr == 16 ? k_split_residues<false, 16> : k_split_residues<false, 64>,
+                  a_blocks + h_blocks, 256, 0, stream, A, lda,
                   M, N, K, L.kp, b.amax, b.asq, b.hmax, b.hsum, b.hsq, a_blocks, b.Ht, cc, b.RA, b.RH, b.prm);
     prof_mark(stream, "residues");
   } else {

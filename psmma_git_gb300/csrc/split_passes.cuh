@@ -130,6 +130,9 @@ __device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, lon
 // 3072 901 / 904.  Parameters in line / in a launch of their own, split: n = 256 32.9 / 34, 384 37.0 / 36.4, 512
 // 41.4 / 39.9, 768 63.7 / 56.5.
 constexpr int SMALL_ROWS = 4096, SMALL_K = 2048, INLINE_ROWS = 512;
+// Rows of A's residue tiles: 16 (one quad a thread) while their blocks do not fill the SMs, 64 otherwise.  FP64
+// Toeplitz, 64 / 16: n = 384 34.4 / 31.0 us, 512 42.3 / 38.4, 768 60.7 / 57.5, 2048 354 / 366.
+inline int small_tile_rows(int M, int N) { return M + N <= 1536 ? 16 : 64; }
 inline bool small_operands(int M, int N, int K) { return M + N <= SMALL_ROWS && K <= SMALL_K; }
 constexpr int SMALL_RB = 8;  // rows of A a statistics block covers, 256 threads
 
