@@ -722,7 +722,7 @@ __global__ void __launch_bounds__(RRLU_THREADS) k_cp_search_eig(const RrluEigBlo
 }
 
 // Columns of A(:, R) (n x M, lda) in RRLU pivot order for every compressed block:
-// T0(:, j) = A(:, PL(j)) for j < Rk, Ar(:, t) = A(:, PL(Rk + t)) for t < M - Rk (PL 1-based).
+// T0(:, j) = A(:, PL(j)) for j < Rk, and on the FP64 path Ar(:, t) = A(:, PL(Rk + t)) for t < M - Rk (PL 1-based).
 // One block per column of the batch (columns numbered from c0 per block).
 struct GatherDesc {
   const double* A;
@@ -1596,14 +1596,17 @@ void build_rounds_split(const Plan& P, const psmma_batch_item* items, int count,
     double* T = P.gather[b];
     if (compressor == PSMMA_COMPRESS_RRLU) {
       const LuParts lp = lu_parts(P, kind, b, items);
-      GenSpec gz;  // Z'(t, j) = Z(Rk+t) W(j) / (P(Rk+t) - P(j)): T0 += Ar * Z'
+      GenSpec gz;  // Z'(t, j) = Z(Rk+t) W(j) / (P(Rk+t) - P(j)): T0 += A(:, PL(Rk+1:)) * Z'
       gz.kind = KIND_CAUCHY;
       gz.Dr = lp.pole + Rk;
       gz.Ur = lp.z + Rk;
       gz.Fc = lp.pole;
       gz.Vc = lp.w;
       if (ob.M - Rk > 0) {
-        R.r1.push_back(SplitProblem{n, Rk, ob.M - Rk, 1.0, 1.0, T + (size_t)n * Rk, n, gz, T, n});
+        // A's columns are read through the pivots (gathered first: a copy of half of A, 363 of 11000 us at 32 problems)
+        SplitProblem q{n, Rk, ob.M - Rk, 1.0, 1.0, it.A + (long)ob.r0 * it.lda, it.lda, gz, T, n};
+        q.perm = lp.perm + Rk;
+        R.r1.push_back(q);
         R.executed += 2.0 * n * (double)(ob.M - Rk) * Rk;
       }
     } else {
@@ -2159,7 +2162,7 @@ static int batch_run(int kind, int count, const psmma_batch_item* items, double 
       g.T0 = P.gather[b];
       g.Ar = P.gather[b] + (size_t)it.n * ranks[b];
       gd.push_back(g);
-      gather_cols += ob.M;
+      gather_cols += precision == PSMMA_PREC_SPLIT ? ranks[b] : ob.M;  // the split passes read the rest in place
     }
     if (!gd.empty() && cudaMemcpyAsync(P.d_gather, gd.data(), sizeof(GatherDesc) * gd.size(),
                                        cudaMemcpyHostToDevice, st) != cudaSuccess)

@@ -243,6 +243,7 @@ struct SplitProblem {
   const double* A2 = nullptr;  // columns k >= ka of A come from A2 (ld lda2) at k - ka
   long lda2 = 0;
   int ka = 0;                  // 0: A alone
+  const int* perm = nullptr;   // column k < ka of A is column perm[k] - 1 (device; nullptr: k)
 };
 // Tunables of the grouped GEMM: output-tile width 64 for products with N <= narrow_max, 128
 // for N <= mid_max, else 256; raster group of group_m row tiles.

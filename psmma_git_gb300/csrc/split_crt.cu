@@ -547,17 +547,26 @@ __device__ __forceinline__ void residues_A_blk(const double* __restrict__ A, lon
                                                int ka, int n, int k, int kp,
                                                const unsigned long long* __restrict__ amax_bits,
                                                const SplitDevParams* prm, const CrtConsts& cc,
-                                               __nv_bfloat16* __restrict__ RA, int bx, int by) {
+                                               __nv_bfloat16* __restrict__ RA, int bx, int by,
+                                               const int* perm = nullptr) {
   __shared__ double tile[64][TR];
   const int i0 = by * TR, k0 = bx * 64;
   constexpr int TX = TR < 32 ? TR : 32;
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;  // 256 threads
-  for (int kk = ty; kk < 64; kk += 256 / TX) {
-    const int gk = k0 + kk;
+  long step;
+  const double* run = acol_run(A, lda, A2, lda2, ka, k0, min(k, k0 + 64), perm, &step);
+  if (run) {
+    for (int kk = ty; kk < 64; kk += 256 / TX) {
 #pragma unroll
-    for (int rr = tx; rr < TR; rr += TX) {
-      const int gi = i0 + rr;
-      tile[kk][(rr + (kk >> 2)) & (TR - 1)] = (gi < n && gk < k) ? __ldg(acol(A, lda, A2, lda2, ka, gk) + gi) : 0.0;
+      for (int rr = tx; rr < TR; rr += TX)
+        tile[kk][(rr + (kk >> 2)) & (TR - 1)] = (i0 + rr < n && k0 + kk < k) ? __ldg(run + kk * step + i0 + rr) : 0.0;
+    }
+  } else {
+    for (int kk = ty; kk < 64; kk += 256 / TX) {
+      const double* col = k0 + kk < k ? acol(A, lda, A2, lda2, ka, k0 + kk, perm) : A;
+#pragma unroll
+      for (int rr = tx; rr < TR; rr += TX)
+        tile[kk][(rr + (kk >> 2)) & (TR - 1)] = (i0 + rr < n && k0 + kk < k) ? __ldg(col + i0 + rr) : 0.0;
     }
   }
   __syncthreads();
@@ -3810,6 +3819,7 @@ struct GProb {
   const double* A2;
   long lda2;
   int ka;
+  const int* perm;
   GenSpec gs;
   double* Q;
   long ldq;
@@ -3868,7 +3878,8 @@ __global__ void __launch_bounds__(128) k_g_row_absmax(const GProb* d, int count,
   for (GRun<0> r(d, count, total, run); r.b < r.end; ++r.b) {
     const GProb& e = r.owner(d, count);
     const int local = r.b - e.b_row, gx = (e.M + 127) / 128;
-    row_absmax_blk(e.A, e.lda, e.A2, e.lda2, e.ka, e.M, e.K, e.row_chunk, e.amax, e.asq, local % gx, local / gx);
+    row_absmax_blk(e.A, e.lda, e.A2, e.lda2, e.ka, e.M, e.K, e.row_chunk, e.amax, e.asq, local % gx, local / gx, nullptr,
+                   e.perm);
   }
 }
 
@@ -3897,7 +3908,7 @@ __global__ void __launch_bounds__(256) k_g_residues_A(const GProb* d, int count,
     const GProb& e = r.owner(d, count);
     const int local = r.b - e.b_ra, gx = e.kp / 64;
     residues_A_blk<64>(e.A, e.lda, e.A2, e.lda2, e.ka, e.M, e.K, e.kp, e.amax, e.prm, cc, e.RA, local % gx,
-                       local / gx);
+                       local / gx, e.perm);
     __syncthreads();  // the shared tile is refilled for the next block
   }
 }
@@ -3957,6 +3968,7 @@ int plan_group(const SplitProblem* P, int count, int nmod, const SplitTune& tune
     e.A = q.A; e.lda = q.lda; e.gs = q.gs; e.Q = q.Q; e.ldq = q.ldq;
     e.A2 = q.A2; e.lda2 = q.lda2;
     e.ka = (q.ka > 0 && q.A2) ? q.ka : q.K;
+    e.perm = q.perm;
     e.prm = w.take<SplitDevParams>(1, 256);
     e.amax = w.take<unsigned long long>(q.M, 256);
     e.asq = w.take<double>(q.M, 256);

@@ -51,11 +51,24 @@ __device__ __forceinline__ int lsb_exp(unsigned long long ab) {
 
 // Row max of |A| as the bits of a non-negative double (NaN/Inf compare above all finite) and
 // row sums of squares (for the Cauchy-Schwarz bound of the integer product).
-// Columns kk >= ka of A come from A2 (ld lda2) at kk - ka (ka = k: A alone).  LSB: also the
+// Columns kk >= ka of A come from A2 (ld lda2) at kk - ka (ka = k: A alone), column kk < ka is column perm[kk] - 1 of A
+// where perm is given.  LSB: also the
 // rows' smallest lsb_exp over their nonzero entries (alsb, initialised above every exponent).
 __device__ __forceinline__ const double* acol(const double* A, long lda, const double* A2, long lda2, int ka,
-                                              int kk) {
-  return kk < ka ? A + (long)kk * lda : A2 + (long)(kk - ka) * lda2;
+                                              int kk, const int* perm) {
+  return kk < ka ? A + (long)(perm ? __ldg(perm + kk) - 1 : kk) * lda : A2 + (long)(kk - ka) * lda2;
+}
+
+// The first of columns [k0, k1) and their distance where they are one run of A or of A2, nullptr otherwise: the choice
+// per element is a good part of a pass's instructions (residues of 32 products' A: 955 -> 807 us without it).
+__device__ __forceinline__ const double* acol_run(const double* A, long lda, const double* A2, long lda2, int ka, int k0,
+                                                  int k1, const int* perm, long* step) {
+  if (k0 >= ka) {
+    *step = lda2;
+    return A2 + (long)(k0 - ka) * lda2;
+  }
+  *step = lda;
+  return k1 <= ka && !perm ? A + (long)k0 * lda : nullptr;
 }
 
 template <bool LSB = false>
@@ -63,7 +76,7 @@ __device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, lon
                                                int ka, int n, int k, int kchunk,
                                                unsigned long long* __restrict__ amax_bits,
                                                double* __restrict__ asq, int bx, int by,
-                                               int* __restrict__ alsb = nullptr) {
+                                               int* __restrict__ alsb = nullptr, const int* perm = nullptr) {
   int i = bx * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int k0 = by * kchunk, k1 = min(k, k0 + kchunk);
@@ -73,12 +86,20 @@ __device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, lon
   bool big = false;
   int lsb = NO_LSB;
   int kk = k0;
+  long step;
+  const double* run = acol_run(A, lda, A2, lda2, ka, k0, k1, perm, &step);
+  const double* p = run + i;
   // eight independent loads in flight per thread (a warp reads 32 consecutive rows)
   for (; kk + 8 <= k1; kk += 8) {
     unsigned long long b[8];
+    if (run) {
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      b[u] = (unsigned long long)__double_as_longlong(__ldg(acol(A, lda, A2, lda2, ka, kk + u) + i)) & ABS_MASK;
+      for (int u = 0; u < 8; ++u, p += step) b[u] = (unsigned long long)__double_as_longlong(__ldg(p)) & ABS_MASK;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        b[u] = (unsigned long long)__double_as_longlong(__ldg(acol(A, lda, A2, lda2, ka, kk + u, perm) + i)) & ABS_MASK;
+    }
     unsigned long long gm = 0;
 #pragma unroll
     for (int u = 0; u < 8; ++u) gm = b[u] > gm ? b[u] : gm;
@@ -98,7 +119,7 @@ __device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, lon
   }
   for (; kk < k1; ++kk) {
     const unsigned long long b =
-        (unsigned long long)__double_as_longlong(__ldg(acol(A, lda, A2, lda2, ka, kk) + i)) & ABS_MASK;
+        (unsigned long long)__double_as_longlong(__ldg(acol(A, lda, A2, lda2, ka, kk, perm) + i)) & ABS_MASK;
     mb = b > mb ? b : mb;
     if constexpr (LSB) lsb = b ? min(lsb, lsb_exp(b)) : lsb;
     if (e == NO_SCALE && b) e = (int)(b >> 52) - 1023;
@@ -110,7 +131,7 @@ __device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, lon
   double sq = 0.0;
   if (big) {  // entries 2^56 times the thread's first ones (or Inf/NaN): FP64 sum
     for (kk = k0; kk < k1; ++kk) {
-      const double a = __ldg(acol(A, lda, A2, lda2, ka, kk) + i);
+      const double a = __ldg(acol(A, lda, A2, lda2, ka, kk, perm) + i);
       sq = fma(a, a, sq);
     }
   } else if (e != NO_SCALE) {
