@@ -2068,6 +2068,7 @@ static int batch_run(int kind, int count, const psmma_batch_item* items, double 
   if (stats) *stats = psmma_batch_stats{0.0, 0.0, 0.0, 0, 0, 0, 0};
   if (count == 0) return PSMMA_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  const StreamCall call(st, !(opts && opts->work));
 
   Plan P;
   const size_t need_a = part_a_bytes(P, items, count, compressor, kind);

@@ -1,12 +1,14 @@
 // C ABI of libpsmma_gb300: argument checks with the reference's INFO numbering, dispatch
 // to the FP64 and split kernels, host-pointer wrappers, Fortran-ABI shims and the
 // library-owned workspace pools.
+#include <climits>
 #include <cstdio>
 #include <cstring>
 #include <map>
 #include <tuple>
 #include <mutex>
 #include <utility>
+#include <vector>
 
 #include "psmma_internal.h"
 #include "tcgen05_util.cuh"  // DEV_ERR_TIMEOUT
@@ -15,7 +17,9 @@ namespace psmma {
 
 // ------------------------------------------------------------------------------------
 // Workspace pools: grow-only device buffers, one per (device, stream).  A pool is only
-// reallocated after its stream has drained, so work in flight never loses its buffer.
+// reallocated after its stream has drained, so work in flight never loses its buffer, and by
+// a caller that holds the stream's StreamCall, so no other thread is between taking the buffer
+// and its last launch on it.
 // ------------------------------------------------------------------------------------
 namespace {
 struct Pool {
@@ -24,7 +28,21 @@ struct Pool {
 };
 std::mutex g_pool_mu;
 std::map<std::tuple<int, cudaStream_t, int>, Pool> g_pools;
+
+std::mutex g_call_mu;  // guards the map; a stream's mutex, once made, stays
+std::map<std::pair<int, cudaStream_t>, std::mutex> g_calls;
 }  // namespace
+
+StreamCall::StreamCall(cudaStream_t stream, bool pooled) {
+  int dev = 0;
+  if (!pooled || cudaGetDevice(&dev) != cudaSuccess) return;
+  std::mutex* mu;
+  {
+    std::lock_guard<std::mutex> lk(g_call_mu);
+    mu = &g_calls[{dev, stream}];
+  }
+  lock_ = std::unique_lock<std::mutex>(*mu);
+}
 
 void* pool_get(size_t bytes, cudaStream_t stream, int* status, int slot) {
   *status = PSMMA_OK;
@@ -227,6 +245,7 @@ int run_real(int kind, int n, int k, double alpha, const double* A, int lda, con
   if (st == 1) return PSMMA_OK;
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
+  const StreamCall call(s, o->work == nullptr);
   if (o->precision == PSMMA_PREC_SPLIT && alpha != 0.0) {
     size_t need = split_workspace_bytes(kind, n, k, o->n_moduli, o->block_levels);
     void* work = o->work;
@@ -251,6 +270,7 @@ int run_dft(int n, int k, double alpha, const psmma_complex* B, int ldb, double 
   if (st == 1) return PSMMA_OK;
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
+  const StreamCall call(s, o->work == nullptr);
   if (o->precision == PSMMA_PREC_SPLIT && alpha != 0.0) {
     size_t need = split_workspace_bytes(KIND_DFT, n, k, o->n_moduli);
     void* work = o->work;
@@ -385,6 +405,7 @@ int host_real(int kind, int n, int k, double alpha, const double* A, int lda, co
     cudaEvent_t* ev;
     st = host_copy_stream(&cs, &ev);
     if (st) return st;
+    const StreamCall call(s, o->work == nullptr);
     const size_t need = split_workspace_bytes(kind, n, k, o->n_moduli, o->block_levels);
     void* work = host_split_work(need, o, s, &st);
     if (st) return st;
@@ -450,6 +471,7 @@ int run_eig(int n, int k, double alpha, const double* A, int lda, const double* 
   if (st == 1) return PSMMA_OK;
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
+  const StreamCall call(s, o->work == nullptr);
   const GenSpec gs = eig_gens(F, U, V, difl, difr, k);
   if (o->precision == PSMMA_PREC_SPLIT && alpha != 0.0) {
     size_t need = split_workspace_general(n, k, k, o->n_moduli, o->block_levels);
@@ -500,6 +522,7 @@ int host_eig(int n, int k, double alpha, const double* A, int lda, const double*
     cudaEvent_t* ev;
     st = host_copy_stream(&cs, &ev);
     if (st) return st;
+    const StreamCall call(s, o->work == nullptr);
     const size_t need = split_workspace_general(n, k, k, o->n_moduli);
     void* work = host_split_work(need, o, s, &st);
     if (st) return st;
@@ -711,17 +734,21 @@ int psmma_stream_release(void* stream) {
 void psmma_release_workspace(void) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return;
+  std::vector<cudaStream_t> streams;
   {
     std::lock_guard<std::mutex> lk(g_pool_mu);
-    for (auto it = g_pools.begin(); it != g_pools.end();) {
-      if (std::get<0>(it->first) == dev) {
-        cudaStreamSynchronize(std::get<1>(it->first));
-        cudaFree(it->second.ptr);
-        it = g_pools.erase(it);
-      } else {
-        ++it;
-      }
-    }
+    for (const auto& e : g_pools)
+      if (std::get<0>(e.first) == dev && (streams.empty() || streams.back() != std::get<1>(e.first)))
+        streams.push_back(std::get<1>(e.first));
+  }
+  for (cudaStream_t s : streams) {
+    const StreamCall call(s, true);  // before g_pool_mu, as in a call
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    cudaStreamSynchronize(s);
+    const auto first = g_pools.lower_bound(std::make_tuple(dev, s, INT_MIN));
+    auto it = first;
+    for (; it != g_pools.end() && std::get<0>(it->first) == dev && std::get<1>(it->first) == s; ++it) cudaFree(it->second.ptr);
+    g_pools.erase(first, it);
   }
   std::lock_guard<std::mutex> lk(g_host_mu);
   auto it = g_host.find(dev);

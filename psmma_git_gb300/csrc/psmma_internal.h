@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 
 #include "../../include/psmma.h"
 
@@ -285,6 +286,16 @@ size_t f64_group_bytes(int count);
 int f64_group_prepare(const F64Prob* P, int count, void* dev, cudaStream_t stream, F64Group* g);
 int f64_group_enqueue(const F64Group& g, cudaStream_t stream);
 
+// Held by a call that works in its stream's pools from taking them to its last launch: the launches of two host
+// threads on one stream would otherwise interleave over the same buffer, and one thread's growth free it under the
+// other's.  Nothing with pooled = false (the caller's workspace).  Order: StreamCall, then the pools' own mutex.
+class StreamCall {
+ public:
+  StreamCall(cudaStream_t stream, bool pooled);
+
+ private:
+  std::unique_lock<std::mutex> lock_;
+};
 // Library-owned device workspace (psmma_capi.cu): grow-only, one pool per (device, stream,
 // slot); a call that needs two independent regions takes them from two slots.
 void* pool_get(size_t bytes, cudaStream_t stream, int* status, int slot = 0);
