@@ -440,13 +440,14 @@ int psmma_server_destroy(psmma_server* s);
 
 /* ---- workspace and housekeeping ----------------------------------------------------- */
 
-/* Bytes of device workspace a call with these sizes and options needs.  The FP64 path needs
- * none, except for products with too few 128 x 128 output tiles to fill the SMs, which it
- * splits along K into partial sums when workspace is available (0 otherwise).  Pass a buffer
- * at least this large in opts->work to avoid library allocation.  An FP64 call with opts->work
- * runs the FP64 tensor-core kernel; one without it takes the exact modular product, whose
- * planes (up to 40 GiB: n = k = 4096 2.9 GB) come from the stream's pool, or the kernel where
- * that allocation fails. */
+/* Bytes of device workspace a call with these sizes and options takes in opts->work; with a buffer
+ * at least this large the call allocates nothing.  FP64 real kinds: 0, except for products with too
+ * few 128 x 128 output tiles to fill the SMs, which the FP64 tensor-core kernel splits along K into
+ * partial sums when workspace is available.  An FP64 call with opts->work runs that kernel.  One
+ * without it takes the exact modular product: its planes (n = k = 4096 2.9 GB, at most 40 GiB) are a
+ * buffer of the stream of their own, which grows within half of the device's free memory, is given
+ * back when another allocation of the library needs the room, and is freed by psmma_stream_release
+ * and psmma_release_workspace; where it does not fit, the call runs the kernel. */
 size_t psmma_workspace_size(int kind, int n, int k, const psmma_opts* opts);
 
 /* Frees the library-owned workspace pools of the current device. */
@@ -460,9 +461,10 @@ void psmma_release_workspace(void);
  * status, or call psmma_stream_release, before destroying a stream. */
 int psmma_stream_status(void* stream);
 
-/* Waits for `stream`, frees the status record of (current device, stream) and returns what
- * psmma_stream_status would have returned.  Call it before cudaStreamDestroy on streams that
- * ran split-path calls; a later call on the stream creates a fresh record. */
+/* Waits for `stream`, frees the status record of (current device, stream) and its FP64 planes
+ * (psmma_workspace_size), and returns what psmma_stream_status would have returned.  Call it before
+ * cudaStreamDestroy on streams that ran split-path or FP64 calls; a later call on the stream creates
+ * what it needs afresh. */
 int psmma_stream_release(void* stream);
 
 /* Per-phase tracing.  While enabled, each call records a CUDA event on its stream after

@@ -44,6 +44,57 @@ StreamCall::StreamCall(cudaStream_t stream, bool pooled) {
   lock_ = std::unique_lock<std::mutex>(*mu);
 }
 
+namespace {
+// Work that needs no memory of its own may use what the device has left, not what another caller needs: slot
+// POOL_EXACT alone.  A call without it takes the DMMA kernel.
+constexpr int POOL_EXACT = 3;
+
+size_t pool_round(size_t bytes) { return (bytes + (1u << 20) - 1) & ~((size_t)(1u << 20) - 1); }
+
+// Allocations that a capture on another stream or thread must not be disturbed by.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Frees the POOL_EXACT buffers of device `dev` but those of streams with a call under way in another thread.  g_pool_mu
+// is held, and the StreamCall of *mine where the caller is a call that has not taken its POOL_EXACT buffer.
+bool give_back_exact(int dev, const cudaStream_t* mine) {
+  bool any = false;
+  for (auto& e : g_pools) {
+    if (std::get<0>(e.first) != dev || std::get<2>(e.first) != POOL_EXACT || !e.second.ptr) continue;
+    const cudaStream_t s = std::get<1>(e.first);
+    std::unique_lock<std::mutex> lk;
+    if (!mine || s != *mine) {
+      std::unique_lock<std::mutex> mk(g_call_mu);
+      std::mutex& mu = g_calls[{dev, s}];
+      mk.unlock();
+      lk = std::unique_lock<std::mutex>(mu, std::try_to_lock);
+      if (!lk.owns_lock()) continue;
+    }
+    if (cudaDeviceSynchronize() != cudaSuccess) {  // the stream itself may be gone
+      cudaGetLastError();
+      return any;
+    }
+    cudaFree(e.second.ptr);
+    e.second = Pool{};
+    any = true;
+  }
+  return any;
+}
+}  // namespace
+
+// cudaMalloc, and once more with the exact route's buffers given back where memory is short.
+cudaError_t device_alloc(void** p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  int dev = 0;
+  if (e != cudaErrorMemoryAllocation || cudaGetDevice(&dev) != cudaSuccess) return e;
+  cudaGetLastError();
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  return give_back_exact(dev, nullptr) ? cudaMalloc(p, bytes) : e;
+}
+
 void* pool_get(size_t bytes, cudaStream_t stream, int* status, int slot) {
   *status = PSMMA_OK;
   if (bytes == 0) return nullptr;
@@ -58,8 +109,13 @@ void* pool_get(size_t bytes, cudaStream_t stream, int* status, int slot) {
     pl.ptr = nullptr;
     pl.bytes = 0;
   }
-  size_t want = (bytes + (1u << 20) - 1) & ~((size_t)(1u << 20) - 1);
-  if (cudaMalloc(&pl.ptr, want) != cudaSuccess) {
+  const size_t want = pool_round(bytes);
+  cudaError_t e = cudaMalloc(&pl.ptr, want);
+  if (e == cudaErrorMemoryAllocation && !stream_capturing(stream)) {
+    cudaGetLastError();
+    if (give_back_exact(dev, &stream)) e = cudaMalloc(&pl.ptr, want);
+  }
+  if (e != cudaSuccess) {
     cudaGetLastError();
     pl.ptr = nullptr;
     *status = PSMMA_ENOMEM;
@@ -67,6 +123,34 @@ void* pool_get(size_t bytes, cudaStream_t stream, int* status, int slot) {
   }
   pl.bytes = want;
   return pl.ptr;
+}
+
+// The stream's POOL_EXACT buffer, or nullptr: it grows only within half of the free memory, and the buffer there is
+// kept where growth fails.
+void* pool_exact(size_t bytes, cudaStream_t stream) {
+  int dev = 0;
+  if (bytes == 0 || cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  Pool& pl = g_pools[std::make_tuple(dev, stream, POOL_EXACT)];
+  if (pl.bytes >= bytes) return pl.ptr;
+  const RelaxedCapture relaxed;
+  const size_t want = pool_round(bytes);
+  size_t left = 0, total = 0;
+  void* p = nullptr;
+  if (cudaMemGetInfo(&left, &total) != cudaSuccess || want > left / 2 || cudaMalloc(&p, want) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (pl.ptr) {
+    if (cudaStreamSynchronize(stream) != cudaSuccess) {
+      cudaFree(p);
+      return nullptr;
+    }
+    cudaFree(pl.ptr);
+  }
+  pl.ptr = p;
+  pl.bytes = want;
+  return p;
 }
 
 bool stream_capturing(cudaStream_t stream) {
@@ -226,8 +310,7 @@ int run_f64(int n, int k, double alpha, const double* A, int lda, const GenSpec&
   const unsigned* gate = nullptr;
   if (alpha != 0.0 && !o->work && exact_route(n, k, k) && !stream_capturing(s)) {
     const size_t need = exact_workspace(n, k, k);
-    int pst = PSMMA_OK;
-    void* xw = need ? pool_get(need, s, &pst) : nullptr;
+    void* xw = pool_exact(need, s);
     if (xw) {
       st = launch_exact(n, k, k, alpha, A, lda, gs, beta, Q, ldq, xw, need, s, &gate);
       if (st) return st;
@@ -332,7 +415,7 @@ void* host_arena(size_t bytes, cudaStream_t* stream, int* status) {
     a.ptr = nullptr;
     a.bytes = 0;
     size_t want = (bytes + (1u << 20) - 1) & ~((size_t)(1u << 20) - 1);
-    if (cudaMalloc(&a.ptr, want) != cudaSuccess) {
+    if (device_alloc(&a.ptr, want) != cudaSuccess) {
       cudaGetLastError();
       *status = PSMMA_ENOMEM;
       return nullptr;
@@ -715,9 +798,18 @@ int psmma_stream_status(void* stream) {
 }
 
 int psmma_stream_release(void* stream) {
+  const StreamCall call((cudaStream_t)stream, true);
   const int st = psmma_stream_status(stream);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return PSMMA_EDEVICE;
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    const auto it = g_pools.find(std::make_tuple(dev, (cudaStream_t)stream, POOL_EXACT));
+    if (it != g_pools.end()) {
+      cudaFree(it->second.ptr);
+      g_pools.erase(it);
+    }
+  }
   unsigned* w = nullptr;
   {
     std::lock_guard<std::mutex> lk(g_stw_mu);

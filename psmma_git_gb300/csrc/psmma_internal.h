@@ -299,6 +299,8 @@ class StreamCall {
 // Library-owned device workspace (psmma_capi.cu): grow-only, one pool per (device, stream,
 // slot); a call that needs two independent regions takes them from two slots.
 void* pool_get(size_t bytes, cudaStream_t stream, int* status, int slot = 0);
+// cudaMalloc for the library's other long-lived buffers: the pools' optional ones make room.
+cudaError_t device_alloc(void** p, size_t bytes);
 // Whether work enqueued on `stream` is being captured into a graph.
 bool stream_capturing(cudaStream_t stream);
 

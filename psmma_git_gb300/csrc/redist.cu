@@ -200,7 +200,7 @@ int upload(psmma_redist_plan* p, cudaStream_t stream) {
   size_t total = 0;
   for (const Part& q : parts) total += align16(std::max<size_t>(q.bytes, 16));
   void* mem = nullptr;
-  if (cudaMalloc(&mem, total) != cudaSuccess) {
+  if (device_alloc(&mem, total) != cudaSuccess) {
     cudaGetLastError();
     return PSMMA_ENOMEM;
   }

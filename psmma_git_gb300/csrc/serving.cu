@@ -291,7 +291,7 @@ int psmma_server_create(size_t hbm_budget_bytes, int max_inflight, psmma_server*
   if (cudaGetDevice(&s->device) != cudaSuccess) { delete s; return PSMMA_EDEVICE; }
   s->max_inflight = max_inflight;
   if (hbm_budget_bytes) {
-    if (cudaMalloc(&s->arena_base, hbm_budget_bytes) != cudaSuccess) {
+    if (device_alloc(&s->arena_base, hbm_budget_bytes) != cudaSuccess) {
       cudaGetLastError();
       delete s;
       return PSMMA_ENOMEM;
