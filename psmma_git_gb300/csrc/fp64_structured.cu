@@ -300,19 +300,32 @@ __global__ void __launch_bounds__(F64_THREADS, 1) k_struct_f64(F64Args p) {
   struct_f64_tile<KIND>(p, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// C := beta * C + sum_z W_z over the S split-K partials, in split order (deterministic).
+// C := beta * C + sum_z W_z over the S split-K partials, in split order (deterministic).  U elements a thread at a time: 1 on a
+// full grid, 4 on the few blocks of a gated launch (see there), which else have too few loads in flight.
+template <int U>
 __global__ void k_splitk_reduce(double* __restrict__ C, long ldc, const double* __restrict__ W, long ldw, int M,
                                 int N, int S, double beta, const unsigned* gate) {
   grid_wait();
   if (gate && *gate == 0u) return;
-  const long total = (long)M * N;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-    const long i = e % M, j = e / M;
-    double v = W[i + j * ldw];
-    for (int z = 1; z < S; ++z) v += W[(long)z * ldw * N + i + j * ldw];
-    double* cp = C + i + j * ldc;
-    if (beta != 0.0) v = fma(beta, *cp, v);
-    *cp = v;
+  const long total = (long)M * N, step = (long)gridDim.x * blockDim.x, part = ldw * N;
+  for (long e0 = blockIdx.x * (long)blockDim.x + threadIdx.x; e0 < total; e0 += U * step) {
+    const double* w[U];
+    double* c[U];
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long e = min(e0 + u * step, total - 1), j = e / M, i = e - j * M;
+      w[u] = W + i + j * ldw;
+      c[u] = C + i + j * ldc;
+      v[u] = *w[u];
+    }
+#pragma unroll 4
+    for (int z = 1; z < S; ++z)
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] += *(w[u] += part);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (e0 + u * step < total) *c[u] = beta != 0.0 ? fma(beta, *c[u], v[u]) : v[u];
   }
 }
 
@@ -398,8 +411,9 @@ int launch_struct_f64_ws(int M, int N, int K, double alpha, const double* X, lon
   p.gate = gate;
   dim3 grid((M + F64_BM - 1) / F64_BM, (N + F64_BN - 1) / F64_BN);
   if (grid.y > 65535) return PSMMA_EUNSUPPORTED;
+  int sms = 0;
   if (work) {
-    int dev = 0, sms = 0;
+    int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return PSMMA_EDEVICE;
     const int S = f64_splitk_count(M, N, K, sms);
@@ -435,9 +449,12 @@ int launch_struct_f64_ws(int M, int N, int K, double alpha, const double* X, lon
   }
   if (p.W) {
     const long total = (long)M * N;
-    // a gated launch mostly returns at once: a block an SM instead of 16 (n = 1024: 3.5 us of a call of 94)
-    const int blocks = (int)std::min<long>((total + 255) / 256, gate ? 152L : 152L * 16);
-    launch_behind(gate != nullptr, k_splitk_reduce, blocks, 256, 0, stream, C, ldc, p.W, p.ldw, M, N, (int)grid.z, beta, gate);
+    // a gated launch mostly returns at once: a block an SM instead of 16 (n = 1024: 3.5 us of a call of 94), four
+    // elements a thread for the products handed over (n = 1024, 2048: 2276, 16121 us with one, 2266, 16067 with four;
+    // the full grid with four instead of one: 2235 -> 2256)
+    const int blocks = (int)std::min<long>((total + 255) / 256, gate ? sms : 16L * sms);
+    launch_behind(gate != nullptr, gate ? k_splitk_reduce<4> : k_splitk_reduce<1>, blocks, 256, 0, stream, C, ldc, p.W, p.ldw, M, N,
+                  (int)grid.z, beta, gate);
   }
   prof_mark(stream, "struct_gemm_f64");
   return cudaGetLastError() == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
