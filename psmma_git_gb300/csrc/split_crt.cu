@@ -3844,9 +3844,9 @@ __device__ __forceinline__ int gfind(const GProb* d, int count, int blk) {
   return lo;
 }
 
-// Columns of a row-statistics block: 1024, halved down to 128 while the launch has fewer than 16 blocks per SM of
-// 152 (16 problems up to n = 2900: some 300 chains of 128 loads, 317 us; short chunks 52 us).
-constexpr int G_ROW_KCHUNK = 1024, G_ROW_BLOCKS = 16 * 152;
+// Columns of a row-statistics block: 1024, halved down to 128 while the launch has fewer than 16 blocks per SM
+// (16 problems up to n = 2900: some 300 chains of 128 loads, 317 us; short chunks 52 us).
+constexpr int G_ROW_KCHUNK = 1024, G_ROW_BLOCKS_SM = 16;
 
 // Each CTA of a grouped pass kernel walks a run of consecutive logical blocks (one binary
 // search per CTA, then a linear advance across product boundaries): a lookup per logical block
@@ -3978,11 +3978,13 @@ int plan_group(const SplitProblem* P, int count, int nmod, const SplitTune& tune
   }
   const uintptr_t small1 = (w.off + 1023) & ~(uintptr_t)1023;
   int b_row = 0, b_h = 0, b_ra = 0, b_rh = 0, b_crt = 0;
-  int row_chunk = G_ROW_KCHUNK;
+  int row_chunk = G_ROW_KCHUNK, dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    sms = 1;  // the sizes alone are asked for
   for (; row_chunk > 128; row_chunk >>= 1) {
     long blocks = 0;
     for (const GProb& e : pr) blocks += (long)((e.M + 127) / 128) * ((e.K + row_chunk - 1) / row_chunk);
-    if (blocks >= G_ROW_BLOCKS) break;
+    if (blocks >= (long)G_ROW_BLOCKS_SM * sms) break;
   }
   for (int i = 0; i < count; ++i) {
     GProb& e = pr[i];
