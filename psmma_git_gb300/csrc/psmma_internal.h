@@ -174,8 +174,8 @@ int launch_split_params(SplitDevParams* prm, double log2M, int M, int N, int K, 
 size_t fft_workspace(int n, int k);
 int launch_fft(int n, int k, double alpha, const double* B, long ldb, double beta, double* C, long ldc, bool ieee,
                void* work, size_t lwork, cudaStream_t stream);
-// Bytes a DFT call needs from the library's own pool or a server's arena: the transform's where it
-// covers n, else the dense product's.
+// Bytes a DFT call needs from the library's own pool: the transform's where it covers n, else the
+// dense product's.
 size_t dft_pool_bytes(int precision, int n, int k, int n_moduli);
 // The DFT's radix step (split_crt.cu): the radix for size n (1, 2, 4 or 8); B' (n/R x R k
 // complex) = [B(0::R,:) | ... | B(R-1::R,:)]; C(j + (n/R) s, c) = sum_r w_R^(s r) w_n^(j r)

@@ -122,7 +122,9 @@ struct psmma_server {
 namespace psmma {
 namespace {
 
-size_t request_workspace(const psmma_request& r) {
+// Bytes of the arena a request takes, `total` the whole of it.  FP64 DFT: room for the transform, whose tables are up to
+// 0.6 MB more than the dense product's (n = 7200); in an arena without that room it is the dense product.
+size_t request_workspace(const psmma_request& r, size_t total) {
   psmma_opts o;
   memset(&o, 0, sizeof(o));
   o.precision = r.precision;
@@ -130,7 +132,10 @@ size_t request_workspace(const psmma_request& r) {
   if (r.kind == KIND_CAUCHY_EIG)
     return r.precision == PSMMA_PREC_SPLIT ? split_workspace_general(r.n, r.k, r.k, r.n_moduli) : 0;
   if (r.precision == PSMMA_PREC_SPLIT) return split_workspace_bytes(r.kind, r.n, r.k, r.n_moduli);
-  if (r.kind == KIND_DFT) return std::max(dft_f64_workspace(r.n, r.k), fft_workspace(r.n, r.k));
+  if (r.kind == KIND_DFT) {
+    const size_t dense = dft_f64_workspace(r.n, r.k), both = std::max(dense, fft_workspace(r.n, r.k));
+    return round_up(both, kArenaAlign) <= total ? both : dense;
+  }
   return 0;
 }
 
@@ -331,7 +336,7 @@ int psmma_server_submit(psmma_server* s, const psmma_request* r, unsigned long l
   if (!s || !r || !ticket) return PSMMA_ENULL;
   int st = check_request(*r);
   if (st) return st;
-  const size_t need = request_workspace(*r);
+  const size_t need = request_workspace(*r, s->arena.total());
   if (need > s->arena.total()) return PSMMA_ENOMEM;  // can never be admitted
   std::lock_guard<std::mutex> lk(s->mu);
   Job j;
