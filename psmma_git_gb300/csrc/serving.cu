@@ -35,14 +35,15 @@ double now_s() {
 constexpr size_t kArenaAlign = 4096;
 size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// First-fit allocator over [0, size) with coalescing of free neighbours.
+// First-fit allocator over [0, size) with coalescing of free neighbours, in whole pages but for the last one.
 class Arena {
  public:
   void init(size_t size) { free_[0] = size; total_ = size; }
   bool alloc(size_t bytes, size_t* off) {
-    bytes = round_up(std::max<size_t>(bytes, 1), kArenaAlign);
+    const size_t pages = round_up(std::max<size_t>(bytes, 1), kArenaAlign);
     for (auto it = free_.begin(); it != free_.end(); ++it) {
-      if (it->second >= bytes) {
+      if (it->second >= pages || (it->second >= bytes && it->first + it->second == total_)) {
+        bytes = std::min(pages, it->second);
         *off = it->first;
         size_t rest = it->second - bytes, start = it->first + bytes;
         free_.erase(it);
@@ -134,7 +135,7 @@ size_t request_workspace(const psmma_request& r, size_t total) {
   if (r.precision == PSMMA_PREC_SPLIT) return split_workspace_bytes(r.kind, r.n, r.k, r.n_moduli);
   if (r.kind == KIND_DFT) {
     const size_t dense = dft_f64_workspace(r.n, r.k), both = std::max(dense, fft_workspace(r.n, r.k));
-    return round_up(both, kArenaAlign) <= total ? both : dense;
+    return both <= total ? both : dense;
   }
   return 0;
 }
