@@ -60,9 +60,11 @@ extern "C" {
 #define PSMMA_ESCRATCH      -117  /* request exceeds the fixed scratch of psmma_cauchy_split_noalloc */
 
 /* ---- options ------------------------------------------------------------------------ */
-#define PSMMA_PREC_FP64   0   /* FP64 results: real kinds by the exact modular product rounded once
-                                 (or FP64 tensor-core MMA where the operands span too many
-                                 bits, the caller brings a workspace, or the call is captured)  */
+#define PSMMA_PREC_FP64   0   /* FP64 results: real kinds by the exact modular product rounded once,
+                                 or by FP64 tensor-core MMA where the operands span too many bits or
+                                 are not finite, where its planes do not fit the device, and for calls
+                                 with opts->work, under capture or through a server (the two differ
+                                 by the roundings of the FP64 sums)                             */
 #define PSMMA_PREC_SPLIT  1   /* split path: exact modular slices on BF16 tensor cores (tcgen05),
                                  FP64 scaling and recombination (all four kinds)              */
 
