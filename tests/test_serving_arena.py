@@ -1,4 +1,5 @@
 """Requests at the limits of a server's memory budget, and FP64 requests of the real kinds alone and in the mix."""
+import numpy as np
 import pytest
 
 from oracle import psmma_oracle as O
