@@ -442,8 +442,43 @@ def run_gpu(args, ws, rank, local):
             result["clocks"] = cl
         if not args.no_extra:
             result["extra"] = run_extras(args, ws, rank, local)
-        print(json.dumps(result), flush=True)
+        print(json.dumps({"detail": result}), file=sys.stderr, flush=True)
+        print(json.dumps(compact_line(result)), flush=True)
     return 0
+
+
+LINE_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+             "vs_baseline", "dtype", "data", "config", "gpu_launches", "latency_ms", "rel_err", "phases_ms", "clocks")
+PART_KEYS = ("value", "unit", "ms_per_step", "steps", "h2d_bytes_per_step", "d2h_bytes_per_step", "median_call_tflops",
+             "stalled_calls", "redone_calls", "bound", "achieved", "peak", "frac", "traffic", "kernel", "cores", "kind",
+             "sample", "cublas_dgemm_tflops", "speedup_split_vs_fp64", "error", "wall_s")
+
+
+def _rounded(x):
+    if isinstance(x, float):
+        return float(f"{x:.5g}")
+    if isinstance(x, dict):
+        return {k: _rounded(v) for k, v in x.items()}
+    return [_rounded(v) for v in x] if isinstance(x, list) else x
+
+
+def compact_line(result: dict) -> dict:
+    """The result line: the headline whole, of each part and of each other workload its value, time and roofline
+    fraction, in some 3 KB (a reader that keeps the end of the output keeps all of it).  The phases, timelines and the
+    other workloads' entries in full are on stderr."""
+    line = {k: result[k] if k in ("value", "ms_per_step") else _rounded(result[k]) for k in LINE_KEYS if k in result}
+    for part in ("roofline", "e2e", "fp64_plain", "cpu_baseline"):
+        if part in result:
+            line[part] = {k: v if k == "value" else _rounded(v) for k, v in result[part].items() if k in PART_KEYS}
+    extra = {}
+    for name, entry in result.get("extra", {}).items():
+        extra[name] = {k: _rounded(entry[k]) for k in ("value", "unit", "ms_per_step", "saturation_tflops",
+                                                       "largest_rate_within_bound_req_s", "error", "wall_s") if k in entry}
+        if entry.get("roofline"):
+            extra[name]["frac"] = _rounded(entry["roofline"].get("frac"))
+    if extra:
+        line["extra"] = extra
+    return line
 
 
 def run_case(args, ws, rank, local):
@@ -1011,6 +1046,8 @@ def run_cfg0(args, ws, rank, local, compact=False):
                              "kind": "port", "sample": f"whole product, ring restatement 2x2 grid nb=64: "
                                                        f"{t_ring:.2f} s; dense A@H: {t_dense:.2f} s"},
             "ring_vs_dense_rel": O.rel_fro(Qr, dense),
+            # an FP64 call: statistics, parameters, residues, GEMM, recombination, and behind its gate the kernel
+            # and its reduction
             "gpu_launches": 7 * 5 * (steps + args.warmup)}
     return line
 
