@@ -444,8 +444,8 @@ __global__ void __launch_bounds__(128) k_ex_residues_H(const double* __restrict_
 
 // Both, for small operands: blocks 0 .. a_blocks - 1 are the tiles of A, the others 256 quads of H each.
 // INLINE: every block evaluates the parameters, block 0 publishes them; these launches do not fill the SMs, and
-// blockIdx.y takes half of the moduli (an integer's 28 to 32 residues are a serial chain).  With that and tiles of 16 rows:
-// Cauchy n = 256 30.0 -> 26.7 us a call.
+// blockIdx.y takes half of the moduli (an integer's 28 to 32 residues are a serial chain): with that and tiles of 16 rows
+// a call of n = 256 is some 3 us of 24 shorter.
 template <bool INLINE, int TR>
 __global__ void __launch_bounds__(256) k_ex_residues(const double* __restrict__ A, long lda, int M, int N, int K, int kp,
                                                      ExStats st, ExLog2 lg, int max_groups, int a_blocks,
@@ -500,8 +500,8 @@ __device__ __noinline__ double ex_outside_normal(unsigned t3, unsigned t2, bool 
 }
 
 // The element of the 4 G residues r(l), times 2^e, rounded to nearest even.
-// Instruction issue bounds it; sums that are the words of Z need no repacking (28-bit limbs of four-moduli parts before:
-// the Toeplitz multiply of n = 2048 392 us, now 378; 1024 132 / 129; 128 37.6 / 35.5 with one element a thread).
+// Instruction issue bounds it; sums that are the words of Z need no repacking (28-bit limbs of four-moduli parts: the
+// Toeplitz multiply of n = 2048 14 us longer, 1024 3 us).
 template <int G, class Residue>
 __device__ __forceinline__ double ex_crt(Residue r, int e) {
   constexpr int NW = ex_words(G);
@@ -711,7 +711,7 @@ size_t exact_workspace(int M, int N, int K) {
 
 // Every size the passes' grids cover: the DMMA kernel's time is that of whole 128 x 128 x 16 tile
 // steps, about 75 us each (2 FP64 FMAs per SM and cycle), so that it is slower from one step on
-// (n = 32: 166 us against 61-68; n = 256: 609 / 92; n = 2048: 16.4 ms / 0.75; n = 4096: 129 / 3.0).
+// (Toeplitz n = 32: 166 us against 22; n = 256: 610 / 24; n = 2048: 16.0 ms / 0.354; n = 4096: 129 / 1.83).
 bool exact_route(int M, int N, int K) { return K < (1 << 21) && M <= 8 * 65535 && N <= 8 * 65535; }
 
 // Enqueues the exact route of Q (M x N) = alpha A (M x K) H (K x N) + beta Q; *gate receives the
@@ -765,7 +765,7 @@ int launch_exact(int M, int N, int K, double alpha, const double* A, long lda, c
   } else {
     k_ex_init<<<(M + 255) / 256, 256, 0, stream>>>(prm, amax, asq, alsb, M);
     // enough blocks for some eight waves, so that the loads of a chunk (eight in flight a thread) are
-    // not a serial chain: n = 2048 at 1024-column chunks 208 us, n = 256 at 128 27 us
+    // not a serial chain: the Toeplitz multiply of n = 3072 at 1024-column chunks 1052 us, so 900
     int kchunk = 1024;
     while (kchunk > 16 && (long)((M + 127) / 128) * ((K + kchunk - 1) / kchunk) < 8L * sms) kchunk >>= 1;
     launch_behind(true, k_ex_row_stats, dim3((M + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, stream, A, lda, M, K, kchunk,

@@ -20,8 +20,8 @@
 //               one of the two forms.
 // Sizes none of the three covers keep the dense products (split_crt.cu, fp64_structured.cu).
 //
-// Measured (n = k, against the dense products it replaces): split precision n = 4096 0.30 ms (2.64),
-// 8192 1.42 (7.17), 16384 8.9 (43.0); FP64 n = 4800 0.71 ms (209).  ncu at n = 8192, before the first pass
+// Measured (n = k, against the dense products it replaces): split precision n = 4096 0.29 ms (2.64),
+// 8192 1.37 (7.17), 16384 8.9 (43.0); FP64 n = 4800 0.69 ms (209).  ncu at n = 8192, before the first pass
 // took its entries from registers (1.73 ms): 510 instructions a point with the conversions, the integer
 // pipe 51 % and the wide multiply-adds 37 % busy, issue 45 %, DRAM 12 %: bound by the passes' instructions
 // and by the latencies that 16 warps (128 registers each thread) leave uncovered.

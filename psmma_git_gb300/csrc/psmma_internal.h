@@ -125,8 +125,9 @@ inline void launch_behind(bool behind, void (*kernel)(P...), dim3 grid, dim3 blo
 }
 #ifdef __CUDACC__
 // The stream's earlier work is complete and visible.  No early trigger: the next kernel's blocks come in as this one's
-// leave.  With griddepcontrol.launch_dependents behind the wait they were packed onto the SMs that had room (FP64
-// Toeplitz multiply, plain launches / trigger / wait alone: n = 256 46.8 / 46.1 / 32.8 us, 1024 131.7 / 117.7 / 115.9).
+// leave.  With griddepcontrol.launch_dependents behind the wait they were packed onto the SMs that had room (Toeplitz
+// multiply, plain launches / trigger / wait alone: FP64 n = 256 35.2 / 30.2 / 24.2 us, 1024 107.0 / 93.8 / 92.7; split n = 256
+// 37.2 / 47.1 / 28.1, 1024 94.5 / 83.1 / 81.6).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif
 

@@ -2297,7 +2297,7 @@ static int split_status(SplitDevParams* prm, cudaStream_t stream, unsigned* stat
 // Core of the split path: Q (M x N) = alpha * A (M x K, column-major, lda) * H (K x N) + beta * Q
 // (column-major, ldq), H generated from gs (any kind but the DFT: split_core_dft3).
 // Row maxima and norms of A (cleared before): chunks of columns short enough for some eight waves of
-// blocks (a chunk is a chain of loads, eight in flight a thread: 1000 x 777 in one chunk 55 us).
+// blocks (a chunk is a chain of loads, eight in flight a thread: split Toeplitz n = 3072 at 1024-column chunks 957 us, so 858).
 int launch_row_stats(const double* A, long lda, int M, int K, unsigned long long* amax, double* asq, int sms,
                      cudaStream_t stream, const unsigned* gate) {
   int kchunk = 1024;
@@ -3065,8 +3065,8 @@ static int split_core_host(int M, int N, int K, double alpha, const double* A_h,
   const SplitBuffers b = split_buffers(w, L);
   const CrtConsts cc = get_consts(nmod);
   // Small operands are not worth a guess: their upload takes little longer than the H passes it
-  // hides behind, and a wrong guess repeats every product (n = 4096, new operands each call: 4.3 ms
-  // guessing, 2.5 ms not; 16384: the upload is 10.7 of 78 ms).
+  // hides behind, and a wrong guess repeats every product (n = 4096: 2.9 ms guessing, 5.0 where the guess
+  // is wrong, 2.46 not; 16384: the upload is 10.7 of 78 ms).
   const bool small = (size_t)M * K * 8 <= ((size_t)256 << 20);
   const bool spec = pa_guess >= 8 && ph_guess >= 8 && beta == 0.0 && !small;
   cudaEvent_t* ev_up = ev;               // NP: column chunks or row panels of A landed
@@ -3592,8 +3592,8 @@ static int split_core_dft3(int k, int n, double alpha, const double* B, long ldb
 // the terms in which the two differ, in microseconds.  Transforms: 2 lg levels of L points per row and
 // prime at 2.16e-7 us (8192 x 8192: 3.25 ms), 1.3 times that at L = 2^15 (tables past L1), and 60 us of
 // launches.  GEMMs: 2 k^2 flops per row and modulus at 1.5e9 a microsecond, three quarters of them per level of
-// the block step, and H's generation and residues, 1.1e-5 us an entry.  Measured (transforms / GEMMs):
-// n = k = 2048 0.35 / 0.37 ms, 3003 0.87 / 0.85, 4096 1.24 / 1.62, 8192 4.3 / 8.7, 16384 19.6 / 51.
+// the block step, and H's generation and residues, 1.1e-5 us an entry.  Measured (transforms / GEMMs, n = k,
+// 14 moduli): 3300 0.93 / 0.96 ms, 4096 1.20 / 1.60, 5000 2.38 / 2.86, 8192 4.1 / 9.2, 16384 18.8 / 54.9.
 // More than 15 moduli leave the primes no bits for unequal columns.
 static bool ntt_route(int kind, int n, int k, int nmod) {
   const int lg = ntt_log(k);

@@ -147,20 +147,22 @@ __device__ __forceinline__ void row_absmax_blk(const double* __restrict__ A, lon
 // Small operands (M + N at most SMALL_ROWS, K at most SMALL_K): the statistics of A's rows and H's columns are one
 // launch, the residues of both another; up to INLINE_ROWS the latter's blocks each evaluate the parameters for
 // themselves.  Their passes take a few microseconds each, so that the launches set the time.  Toeplitz, separate
-// passes / these, split: n = 1280 150 / 120 us, 2048 328 / 304, 3072 796 / 777; FP64: 1280 143 / 136, 2048 357 / 354,
-// 3072 901 / 904.  Parameters in line / in a launch of their own, split: n = 256 32.9 / 34, 384 37.0 / 36.4, 512
-// 41.4 / 39.9, 768 63.7 / 56.5.
+// passes / these, split: n = 256 58.7 / 28.1 us, 1024 108.7 / 81.6, 2048 331 / 305, 3072 the same; FP64: 256 35.8 / 24.2,
+// 1024 97.5 / 92.7, 2048 357 / 354, 3072 the same.  Parameters in line / in a launch of their own, split: n = 256
+// 28.1 / 29.4, 384 33.0 / 32.3, 512 41.3 / 36.5; FP64: 256 24.2 / 27.7, 384 33.4 / 29.9, 512 47.6 / 38.1.
 constexpr int SMALL_ROWS = 4096, SMALL_K = 2048, INLINE_ROWS = 512;
 // Rows of A's residue tiles: 16 (one quad a thread) while their blocks do not fill the SMs, 64 otherwise.  FP64
-// Toeplitz, 64 / 16: n = 384 34.4 / 31.0 us, 512 42.3 / 38.4, 768 60.7 / 57.5, 2048 354 / 366.
-inline int small_tile_rows(int M, int N) { return M + N <= 1536 ? 16 : 64; }
+// Toeplitz, 64 / 16: n = 384 34.2 / 29.9 us, 512 40.4 / 38.1, 768 58.9 / 56.7, 1024 92.7 / 92.4, 2048 354 / 366.
+constexpr int SMALL_TILE16 = 1536;
+inline int small_tile_rows(int M, int N) { return M + N <= SMALL_TILE16 ? 16 : 64; }
+static_assert(INLINE_ROWS <= SMALL_TILE16, "the launches with parameters in line have tiles of 16 rows");
 inline bool small_operands(int M, int N, int K) { return M + N <= SMALL_ROWS && K <= SMALL_K; }
 constexpr int SMALL_RB = 8;  // rows of A a statistics block covers, 256 threads
 
 // Row maxima, squared norms (and lowest bits) of rows 8 b .. 8 b + 7 over all of K, not accumulated into
 // what was there: a warp takes 8 rows of 4 columns (64-byte runs), the block 32 columns a step, eight steps in
 // flight.  32 rows a block (whole 256-byte runs, a quarter of the blocks) left a chain of 16 such groups of loads at
-// K = 1024, the longest of the launch (Toeplitz n = 1024: FP64 114.1 -> 93.4 us, split 96.6 -> 81.2).
+// K = 1024, the longest of the launch (Toeplitz n = 1024 with 32 rows: FP64 some 20 us more of 93, split 15 of 82).
 template <bool LSB>
 __device__ __forceinline__ void small_rows_blk(const double* __restrict__ A, long lda, int n, int k, int b,
                                                unsigned long long* __restrict__ amax_bits, double* __restrict__ asq,
