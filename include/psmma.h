@@ -133,7 +133,9 @@ int psmma_cauchyeig(int n, int k, double alpha, const double* A, int lda, const 
 
 /* Replaces PZMDFTL(N,K,NB,KB,ALPHA,B,LDB,BETA,C,LDC,IMROW,IMCOL,WORK,RWORK)
  * (pzmdftL.f90:1-2): C := alpha*F*B + beta*C with F the N-by-N DFT matrix on the left.
- * The reference's ALPHA and BETA are real (DOUBLE PRECISION); so are these. */
+ * The reference's ALPHA and BETA are real (DOUBLE PRECISION); so are these.  B and C are aligned
+ * like cuDoubleComplex (16 bytes): with one on an odd multiple of 8 bytes, orders that the
+ * fixed-point transform does not cover return PSMMA_EUNSUPPORTED (split, or FP64 with a radix step). */
 int pzmdftl(int n, int k, double alpha, const psmma_complex* B, int ldb,
             double beta, psmma_complex* C, int ldc, const psmma_opts* opts, void* stream);
 

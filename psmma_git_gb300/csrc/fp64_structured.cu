@@ -503,6 +503,7 @@ int launch_dft_f64(int n, int k, double alpha, const double* B, long ldb, double
     // real view: C'(2n x k) = F'(2n x 2n) * B'(2n x k), leading dimensions doubled
     return launch_struct_f64(2 * n, k, 2 * n, alpha, B, 2 * ldb, gs, beta, C, 2 * ldc, stream);
   }
+  if (!aligned16(B, C)) return PSMMA_EUNSUPPORTED;
   const int nq = n / R;
   if ((long)R * k > 65535L * F64_BN) return PSMMA_EUNSUPPORTED;  // the kernel's grid y covers R k columns
   double2* Bp = (double2*)w;

@@ -178,6 +178,8 @@ int launch_fft(int n, int k, double alpha, const double* B, long ldb, double bet
 // Bytes a DFT call needs from the library's own pool: the transform's where it covers n, else the
 // dense product's.
 size_t dft_pool_bytes(int precision, int n, int k, int n_moduli);
+// The dense DFT products' passes read B and write C 16 bytes at a time.
+inline bool aligned16(const void* a, const void* b) { return (((uintptr_t)a | (uintptr_t)b) & 15) == 0; }
 // The DFT's radix step (split_crt.cu): the radix for size n (1, 2, 4 or 8); B' (n/R x R k
 // complex) = [B(0::R,:) | ... | B(R-1::R,:)]; C(j + (n/R) s, c) = sum_r w_R^(s r) w_n^(j r)
 // P(j, r k + c) + beta C.

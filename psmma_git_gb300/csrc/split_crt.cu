@@ -3567,6 +3567,7 @@ static int split_core_dft3(int k, int n, double alpha, const double* B, long ldb
     if (status_dev_out == kStatusWait) return cudaStreamSynchronize(stream) == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
     return cudaMemsetAsync(status_dev_out, 0, sizeof(unsigned), stream) == cudaSuccess ? PSMMA_OK : PSMMA_EDEVICE;
   }
+  if (!aligned16(B, C)) return PSMMA_EUNSUPPORTED;
   if (R == 1) {
     st = dft3_enqueue(k, n, alpha, B, ldb, beta, C, ldc, nmod, work, lwork, stream, &prm);
   } else {

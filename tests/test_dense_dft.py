@@ -50,3 +50,15 @@ def test_dense_columns_that_are_not_finite(n, prec, cuda):
     got = dC.cpu().numpy()
     assert np.isnan(got[:, 1].real).all() and np.isnan(got[:, 1].imag).all()
     assert O.rel_fro(got[:, [0, 2]], np.fft.fft(B[:, [0, 2]], axis=0)) < 1e-12
+
+
+@pytest.mark.parametrize("n,prec", [(7207, "split"), (14414, "split"), (14414, "fp64")])
+@pytest.mark.parametrize("off", [(8, 0), (0, 8)])
+def test_bases_off_16_bytes_are_refused_before_any_launch(n, prec, off, lib):
+    # the dense products' passes would fault on them; the addresses are never read
+    import ctypes as C
+    import psmma_git_gb300 as P
+    opts = P.make_opts(prec)
+    opts.work, opts.lwork = C.c_void_p(1 << 40), P.workspace_size(P.KIND_DFT, n, 2, prec)
+    st = lib.pzmdftl(n, 2, 1.0, C.c_void_p((1 << 41) + off[0]), n, 0.0, C.c_void_p((1 << 42) + off[1]), n, C.byref(opts), None)
+    assert st == -114
