@@ -709,10 +709,18 @@ size_t exact_workspace(int M, int N, int K) {
   return planes >= 16 ? ex_layout(M, N, K, planes).total : 0;
 }
 
-// Every size the passes' grids cover: the DMMA kernel's time is that of whole 128 x 128 x 16 tile
-// steps, about 75 us each (2 FP64 FMAs per SM and cycle), so that it is slower from one step on
-// (Toeplitz n = 32: 166 us against 22; n = 256: 610 / 24; n = 2048: 16.0 ms / 0.354; n = 4096: 129 / 1.83).
-bool exact_route(int M, int N, int K) { return K < (1 << 21) && M <= 8 * 65535 && N <= 8 * 65535; }
+// Whether the route is faster than the DMMA kernel, whose time is that of whole 128 x 128 x 16 tile steps, some 75 us each
+// (2 FP64 FMAs per SM and cycle): one wave of them costs more than the route's passes at every size (Toeplitz n = 32: 166
+// us against 22; n = 256: 610 / 24; n = 2048: 16.0 ms / 0.354; n = 4096: 129 / 1.83) but where H has two steps of rows and A
+// so many rows that its passes, whose planes hold 64 columns of A and 256 of Q whatever K and N are, take longer
+// (500000 x 5: 3.9 ms against 2.0; 50000 x 5 0.42 / 0.24, 5000 x 5 0.069 / 0.083; 19456 x 32 0.180 / 0.156, 150000 x 32
+// 1.20 / 1.22).  Sizes are those the passes' grids cover.
+bool exact_route(int M, int N, int K, int sms) {
+  if (K >= (1 << 21) || M > 8 * 65535 || N > 8 * 65535) return false;
+  if (K > 32 || N > 128) return true;
+  const int waves = ((M + 127) / 128 + sms - 1) / sms;
+  return 30.0 + 0.0078 * M < waves * (6.0 + 72.0 * ((K + 15) / 16));
+}
 
 // Enqueues the exact route of Q (M x N) = alpha A (M x K) H (K x N) + beta Q; *gate receives the
 // device word that tells the DMMA kernel behind it to run.

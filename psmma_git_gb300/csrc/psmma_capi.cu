@@ -308,7 +308,7 @@ int run_f64(int n, int k, double alpha, const double* A, int lda, const GenSpec&
   void* w = f64_work(n, k, k, o, s, &wb, &st);
   if (st) return st;
   const unsigned* gate = nullptr;
-  if (alpha != 0.0 && !o->work && exact_route(n, k, k) && !stream_capturing(s)) {
+  if (alpha != 0.0 && !o->work && exact_route(n, k, k, std::max(1, device_sms())) && !stream_capturing(s)) {
     const size_t need = exact_workspace(n, k, k);
     void* xw = pool_exact(need, s);
     if (xw) {

@@ -143,7 +143,7 @@ int launch_struct_f64_ws(int M, int N, int K, double alpha, const double* X, lon
 // The FP64 precision's exact modular route (exact_crt.cu): whether it is the faster one for a
 // product of these sizes, the bytes it needs (0: none fits its workspace cap), and its launches.
 // *gate receives the device word that makes the DMMA kernel enqueued behind it run.
-bool exact_route(int M, int N, int K);
+bool exact_route(int M, int N, int K, int sms);
 size_t exact_workspace(int M, int N, int K);
 int launch_exact(int M, int N, int K, double alpha, const double* A, long lda, const GenSpec& gs, double beta,
                  double* Q, long ldq, void* work, size_t lwork, cudaStream_t stream, const unsigned** gate);
