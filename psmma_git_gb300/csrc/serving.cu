@@ -209,49 +209,52 @@ void CUDART_CB on_stream_done(void* p) {
   delete c;
 }
 
+// Admits every request at the head of the queue that finds a slot and arena space, then enqueues them in that order: the
+// requests of a burst are in flight together, not each after the launches of the one before.
 void dispatcher_main(psmma_server* s) {
   cudaSetDevice(s->device);
   std::unique_lock<std::mutex> lk(s->mu);
-  for (;;) {
-    int slot = -1;
-    size_t off = 0;
-    s->cv_dispatch.wait(lk, [&] {
-      if (s->stop) return true;
-      if (s->pending.empty()) return false;
-      slot = -1;
-      for (int i = 0; i < s->max_inflight; ++i)
-        if (!s->slot_busy[i]) { slot = i; break; }
-      if (slot < 0) return false;
-      Job& head = s->jobs[s->pending.front()];
-      return head.work_bytes == 0 || s->arena.alloc(head.work_bytes, &off);
-    });
-    if (s->stop) return;
-    int busy = 0;
-    for (int i = 0; i < s->max_inflight; ++i) busy += s->slot_busy[i] ? 1 : 0;
-    s->slot_stream[slot] = s->streams[slot][std::min(busy, s->levels - 1)];
-    const unsigned long long t = s->pending.front();
+  std::vector<Job> admitted;
+  auto admit = [&] {
+    int slot = 0, busy = 0;
+    for (int i = s->max_inflight - 1; i >= 0; --i) {
+      if (s->slot_busy[i]) ++busy; else slot = i;
+    }
+    if (s->pending.empty() || busy == s->max_inflight) return false;
+    Job& j = s->jobs[s->pending.front()];
+    if (j.work_bytes != 0 && !s->arena.alloc(j.work_bytes, &j.work_off)) return false;
     s->pending.pop_front();
-    Job& j = s->jobs[t];
-    j.slot = slot;
-    j.work_off = off;
-    j.start_s = now_s();
+    s->slot_stream[slot] = s->streams[slot][std::min(busy, s->levels - 1)];
     s->slot_busy[slot] = true;
-    s->slot_ticket[slot] = t;
-    Job copy = j;
+    s->slot_ticket[slot] = j.ticket;
+    j.slot = slot;
+    j.start_s = now_s();
+    admitted.push_back(j);
+    return true;
+  };
+  for (;;) {
+    s->cv_dispatch.wait(lk, [&] { return s->stop || admit(); });
+    if (s->stop) return;
+    while (admit()) {
+    }
     lk.unlock();
     // enqueue outside the lock; only this thread launches work
-    cudaStream_t st = s->slot_stream[slot];
-    int e = (cudaEventRecord(s->ev_start[slot], st) == cudaSuccess) ? PSMMA_OK : PSMMA_EDEVICE;
-    if (!e) e = launch_job(s, copy);
-    if (cudaEventRecord(s->ev_end[slot], st) != cudaSuccess && !e) e = PSMMA_EDEVICE;
-    cudaMemcpyAsync(s->host_status + slot, s->dev_status + slot, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-    bool cb_ok = cudaLaunchHostFunc(st, on_stream_done, new HostCbCtx{s, slot}) == cudaSuccess;
-    lk.lock();
-    s->jobs[t].status = e;
-    if (!cb_ok) {  // no callback will come: complete it here
-      s->completed_slots.push_back(slot);
-      s->cv_complete.notify_one();
+    for (Job& j : admitted) {
+      cudaStream_t st = s->slot_stream[j.slot];
+      int e = (cudaEventRecord(s->ev_start[j.slot], st) == cudaSuccess) ? PSMMA_OK : PSMMA_EDEVICE;
+      if (!e) e = launch_job(s, j);
+      if (cudaEventRecord(s->ev_end[j.slot], st) != cudaSuccess && !e) e = PSMMA_EDEVICE;
+      cudaMemcpyAsync(s->host_status + j.slot, s->dev_status + j.slot, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+      if (e) {  // before the completion can be seen
+        lk.lock();
+        s->jobs[j.ticket].status = e;
+        lk.unlock();
+      }
+      HostCbCtx* ctx = new HostCbCtx{s, j.slot};
+      if (cudaLaunchHostFunc(st, on_stream_done, ctx) != cudaSuccess) on_stream_done(ctx);  // no callback will come
     }
+    admitted.clear();
+    lk.lock();
   }
 }
 

@@ -75,3 +75,24 @@ def test_fp64_requests_alone_and_in_the_mix(cuda):
         assert torch.equal(a, Q), (kind, n)
         getattr(P, "psmma_" + kind)(n, n, 1.0, dA, dg, 0.0, Q)
         assert (np.abs(Q.cpu().numpy() - a.cpu().numpy()) <= bound).all(), (kind, n)
+
+
+def test_burst_overlaps_on_the_device(cuda):
+    # by the requests' own times: those submitted behind a product of some milliseconds start before it ends, all in one
+    # admission (none waits for the launches, let alone the end, of the one before)
+    import torch
+    import psmma_git_gb300 as P
+    from psmma_git_gb300.server import Server
+    big, reqs = 5000, []
+    for i, n in enumerate([big, 300, 257, 400]):
+        dA, dg = P.fortran_empty(n, n), torch.from_numpy(O.cfg_vector(2 * n - 1, seed=i)).to(cuda)
+        dA.copy_(torch.rand(n, n, dtype=torch.float64, device=cuda))
+        reqs.append((n, dA, dg, P.fortran_empty(n, n)))
+    need = sum(P.workspace_size(P.KIND_TOEPLITZ, n, n, "split") for n, *_ in reqs)
+    torch.cuda.synchronize()
+    with Server(need + (1 << 20), max_inflight=4) as srv:
+        for _ in range(2):  # the first burst pays for the first use of every kernel and stream
+            infos = [srv.wait(t) for t in [srv.submit("toeplitz", n, n, 1.0, A, g, 0.0, Q) for n, A, g, Q in reqs]]
+    starts = [i["submit_s"] + i["queue_s"] for i in infos]
+    assert all(i["status"] == 0 for i in infos)
+    assert max(starts) < infos[0]["end_s"]
