@@ -78,12 +78,12 @@ def test_fp64_requests_alone_and_in_the_mix(cuda):
 
 
 def test_burst_overlaps_on_the_device(cuda):
-    # by the requests' own times: those submitted behind a product of some milliseconds start before it ends, all in one
+    # by the requests' own times: those submitted behind a product of some ten milliseconds start before it ends, all in one
     # admission (none waits for the launches, let alone the end, of the one before)
     import torch
     import psmma_git_gb300 as P
     from psmma_git_gb300.server import Server
-    big, reqs = 5000, []
+    big, reqs = 12000, []
     for i, n in enumerate([big, 300, 257, 400]):
         dA, dg = P.fortran_empty(n, n), torch.from_numpy(O.cfg_vector(2 * n - 1, seed=i)).to(cuda)
         dA.copy_(torch.rand(n, n, dtype=torch.float64, device=cuda))
