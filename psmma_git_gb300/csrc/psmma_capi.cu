@@ -280,10 +280,9 @@ int device_sms() {
 // Split-K partials of the FP64 path for a product with too few output tiles to fill the SMs:
 // the caller's opts->work when it is large enough, else (no caller workspace) the stream's
 // pool, slot 2.  NULL (no split) when the product fills the SMs or the caller's buffer is short.
-void* f64_work(int M, int N, int K, const psmma_opts* o, cudaStream_t s, size_t* bytes, int* st) {
+void* f64_work(int M, int N, int K, const psmma_opts* o, cudaStream_t s, int sms, size_t* bytes, int* st) {
   *st = PSMMA_OK;
   *bytes = 0;
-  const int sms = device_sms();
   const size_t need = sms ? f64_splitk_bytes(M, N, K, sms) : 0;
   if (!need) return nullptr;
   if (o->work) {
@@ -305,10 +304,11 @@ int run_f64(int n, int k, double alpha, const double* A, int lda, const GenSpec&
             const psmma_opts* o, cudaStream_t s) {
   int st = PSMMA_OK;
   size_t wb = 0;
-  void* w = f64_work(n, k, k, o, s, &wb, &st);
+  const int sms = device_sms();
+  void* w = f64_work(n, k, k, o, s, sms, &wb, &st);
   if (st) return st;
   const unsigned* gate = nullptr;
-  if (alpha != 0.0 && !o->work && exact_route(n, k, k, std::max(1, device_sms())) && !stream_capturing(s)) {
+  if (alpha != 0.0 && !o->work && exact_route(n, k, k, std::max(1, sms)) && !stream_capturing(s)) {
     const size_t need = exact_workspace(n, k, k);
     void* xw = pool_exact(need, s);
     if (xw) {
